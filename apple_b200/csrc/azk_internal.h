@@ -59,6 +59,10 @@ struct TreeJob {
   Transcript* transcript;
   uint32_t* challenge_out;  // 4 limbs
   uint64_t* root_out;       // 4 lanes
+  // First round only (null otherwise): the transcript starts from *base, into which
+  // the public digest `pub` (4 lanes) is absorbed first.
+  const Transcript* base;
+  const uint64_t* pub;
 };
 
 // Number of counters a job needs (upper bound).

@@ -15,6 +15,7 @@
 #include "azk_field.cuh"
 #include "azk_internal.h"
 #include "azk_message.cuh"
+#include "azk_transcript_warp.cuh"
 
 namespace azk {
 
@@ -53,49 +54,6 @@ __device__ __forceinline__ void leaf_digest(const TreeJob& job, uint64_t leaf, c
   } else {
     hash_message(job.raw + leaf * job.stride, job.len, job.suffix, job.aligned8 != 0, d);
   }
-}
-
-// Reduce `count` digests in buffer a (scratch b holds count/2) level by level,
-// storing each level into the job's inner nodes.  Returns the buffer holding the
-// single remaining digest.  `level`/`idx0`: level and first node index of the
-// input digests.
-__device__ __noinline__ uint64_t* reduce_levels(uint64_t* a, uint64_t* b, uint32_t count, const TreeJob& job, uint32_t level, uint64_t idx0) {
-  uint64_t* src = a;
-  uint64_t* dst = b;
-  while (count > 1) {
-    count >>= 1;
-    idx0 >>= 1;
-    level++;
-    uint64_t* lv = job.inner + 4 * (inner_offset(job.logn, level) + idx0);
-    for (uint32_t i = threadIdx.x; i < count; i += blockDim.x) {
-      uint64_t l[4], r[4], d[4];
-      ld_dig(src + 8 * i, l);
-      ld_dig(src + 8 * i + 4, r);
-      sha3_pair(l, r, d);
-      st_dig(dst + 4 * i, d);
-      st_dig(lv + 4 * i, d);
-    }
-    __syncthreads();
-    uint64_t* t = src;
-    src = dst;
-    dst = t;
-  }
-  return src;
-}
-
-__device__ __noinline__ void root_action(const TreeJob& job, const uint64_t* rootp) {
-  uint64_t root[4];
-  ld_dig(rootp, root);
-  if (job.root_out) st_dig(job.root_out, root);
-  if (job.root_action == kRootNone) return;
-  Transcript t = *job.transcript;
-  uint32_t ch[4];
-  if (job.root_action == kRootCircleRound)
-    circle_round(t, job.round, root, ch);
-  else
-    qm31_round(t, job.round, job.frame_in_count, root, ch);
-  *job.transcript = t;
-  for (int k = 0; k < 4; k++) job.challenge_out[k] = ch[k];
 }
 
 // Sets up the sponge input of one leaf (message lanes, suffix and end padding)
@@ -150,22 +108,57 @@ __device__ __forceinline__ uint32_t leaf_setup(const TreeJob& job, uint64_t leaf
   }
 }
 
-// Subtrees of height h = min(2, log2(items)), one per thread.  Items are the
-// tile's leaves, or (from_nodes) digests already in the tree at level `base`.  The
-// subtree's inner nodes are stored (levels base+1 .. base+h, first node idx0 >> l)
-// and its root written to `out` in shared memory.  A 4-item subtree runs as a
-// 7-step loop around ONE permutation site (leaf, leaf, pair, leaf, leaf, pair,
-// pair), which keeps the kernel's code small enough for the instruction cache.
+// ---------------------------------------------------------------------------
+// Shared digest buffers.  A buffer of more than kStdDigests digests holds them
+// split into even and odd bits (two 16-byte words each, the form a pair of lanes
+// hashes); smaller ones hold them as they are (four u64 lanes), for the levels that
+// take a warp per node.
+// ---------------------------------------------------------------------------
+static constexpr uint32_t kStdLog = 3, kStdDigests = 1u << kStdLog;
+// Digests that the leaf phase of a 2^tl-leaf treelet leaves in shared memory, and
+// the height of the subtree each thread hashed: with fewer than THREADS leaves a
+// pair of lanes takes each leaf (latency is all there is), with fewer than
+// 4 x THREADS each thread hashes one or two leaves, else a 4-leaf subtree.  A small
+// tree is a chain of dependent permutations, so what bounds it is their latency
+// (4.5 us by a thread, 2.75 us by a pair, 2.2 us by a warp, at 1.965 GHz); a large
+// one is bound by integer issue, where a thread per subtree is 2 to 7 % better than
+// pairs.  With every level by threads, the 2^10-leaf commit took 116 us a call, a
+// 2^16-value commit-and-fold chain of 10 rounds 1263 us and a 2^22 proof 8090 us;
+// with this split 70, 745 and 7310 us.
+__host__ __device__ constexpr uint32_t tree_subtree_height(uint32_t leaves, uint32_t threads) {
+  return leaves >= 4 * threads ? 2u : leaves >= 2 * threads ? 1u : 0u;
+}
+__host__ __device__ constexpr uint32_t tree_phase_digests(uint32_t leaves, uint32_t threads) {
+  const uint32_t m = leaves >> tree_subtree_height(leaves, threads);
+  return m < kStdDigests ? kStdDigests : m;
+}
+// The last levels' digests: up to kStdDigests of them, then each level behind the
+// one below it.
+static constexpr uint32_t kTopWords = 4 * (2 * kStdDigests);
+// Dynamic shared memory of a launch whose deepest treelet has 2^tl leaves: the
+// leaf phase's digests and half as many for the level above.  Shallower treelets of
+// the same launch need no more than max(12 bytes per leaf, 48 x threads).
+static size_t tree_smem_bytes(uint32_t max_tile_log, uint32_t threads) {
+  const uint32_t leaves = 1u << max_tile_log;
+  size_t m = tree_phase_digests(leaves, threads);
+  if (leaves > threads && m < threads) m = threads;
+  return 48 * m;
+}
+
+// Leaf phase by threads: subtrees of height h = 0, 1 or 2, one per thread.  Items
+// are the tile's leaves.  The subtree's inner nodes are stored (levels 1 .. h,
+// first node idx0 >> l) and its root written to `out` in shared memory.  A 4-leaf
+// subtree runs as a 7-step loop around ONE permutation site (leaf, leaf, pair,
+// leaf, leaf, pair, pair), which keeps the kernel's code small enough for the
+// instruction cache.
 template <uint32_t KIND, int THREADS>
-__device__ __noinline__ uint32_t subtree_phase(const TreeJob& job, uint32_t items, uint32_t base, uint64_t idx0, const uint64_t* nodes, bool from_nodes,
-                                               uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3, uint64_t* out) {
+__device__ __noinline__ void subtree_phase(const TreeJob& job, uint32_t items, uint32_t h, uint64_t idx0, uint32_t c0, uint32_t c1, uint32_t c2,
+                                           uint32_t c3, uint64_t* out) {
   const uint32_t ch[4] = {c0, c1, c2, c3};
-  const uint32_t h = items >= 4 ? 2u : (items >= 2 ? 1u : 0u);
   const uint32_t groups = items >> h;
-  const bool item_is_digest = from_nodes || KIND == kLeafDigest;
-  const uint64_t* digests = from_nodes ? nodes : reinterpret_cast<const uint64_t*>(job.raw) + 4 * idx0;
-  uint64_t* l1 = job.inner + 4 * (inner_offset(job.logn, base + 1) + (idx0 >> 1));
-  uint64_t* l2 = job.inner + 4 * (inner_offset(job.logn, base + 2) + (idx0 >> 2));
+  const uint64_t* digests = reinterpret_cast<const uint64_t*>(job.raw) + 4 * idx0;
+  uint64_t* l1 = job.inner + 4 * (inner_offset(job.logn, 1) + (idx0 >> 1));
+  uint64_t* l2 = job.inner + 4 * (inner_offset(job.logn, 2) + (idx0 >> 2));
   // step k: item index within the subtree (leaf steps) and the step's kind
   //   k:     0  1  2  3  4  5  6        (h == 2)
   //   item:  0  1  -  2  3  -  -
@@ -178,7 +171,7 @@ __device__ __noinline__ uint32_t subtree_phase(const TreeJob& job, uint32_t item
       const uint32_t item = k < 2 ? k : k - 1;  // leaf steps only (h == 2: k = 0, 1, 3, 4)
       const uint64_t leaf = idx0 + (uint64_t)j * (1u << h) + item;
       uint64_t d[4];
-      if (!pair && item_is_digest) {
+      if (!pair && KIND == kLeafDigest) {
         ld_dig_cg(digests + 4 * ((uint64_t)j * (1u << h) + item), d);
       } else {
         uint64_t a[25];
@@ -223,25 +216,279 @@ __device__ __noinline__ uint32_t subtree_phase(const TreeJob& job, uint32_t item
       if (h == 2 && k == 5) st_dig(l1 + 8 * j + 4, d);
       if (h == 2 && k == 6) st_dig(l2 + 4 * j, d);
       if (h == 1 && k == 2) st_dig(l1 + 4 * j, d);
-      if (k + 1 == steps) st_dig(out + 4 * j, d);
+      if (k + 1 == steps) {
+        // at least THREADS digests, more than kStdDigests: split form
+        uint4 e, o;
+        split64(d[0], e.x, o.x);
+        split64(d[1], e.y, o.y);
+        split64(d[2], e.z, o.z);
+        split64(d[3], e.w, o.w);
+        reinterpret_cast<uint4*>(out)[2 * j] = e;
+        reinterpret_cast<uint4*>(out)[2 * j + 1] = o;
+      }
     }
   }
   __syncthreads();
-  return h;
+}
+
+__device__ __forceinline__ ulonglong2 pack_qm31(uint4 v) {
+  return make_ulonglong2((uint64_t)v.x | ((uint64_t)v.y << 32), (uint64_t)v.z | ((uint64_t)v.w << 32));
+}
+// Value e of the layer that a fold kind produces.
+__device__ __forceinline__ uint4 folded_value(const TreeJob& job, uint64_t e, const uint32_t (&ch)[4]) {
+  const uint4 p = __ldg(job.layer + 2 * e), q = __ldg(job.layer + 2 * e + 1);
+  const qm31 r = fri_fold_pair(qm31{p.x, p.y, p.z, p.w}, qm31{q.x, q.y, q.z, q.w}, __ldg(job.inv + e), qm31{ch[0], ch[1], ch[2], ch[3]});
+  return make_uint4(r.a, r.b, r.c, r.d);
+}
+// Word i (< 17) of a raw message of `len` bytes with its suffix (none at len 136).
+__device__ __forceinline__ uint64_t raw_message_word(const TreeJob& job, const uint8_t* p, uint32_t i) {
+  const uint32_t full = job.len >> 3, rem = job.len & 7;
+  if (i > full || i > 16) return 0;
+  if (i < full && job.aligned8) return __ldg(reinterpret_cast<const uint64_t*>(p) + i);
+  uint64_t v = i < full ? 0 : (uint64_t)job.suffix << (8 * rem);
+  const uint32_t n = i < full ? 8 : rem;
+  for (uint32_t k = 0; k < n; k++) v |= (uint64_t)__ldg(p + 8 * i + k) << (8 * k);
+  return v;
+}
+
+// Digest of one leaf by a pair of lanes, in split form.  `ok`: the pair's leaf is
+// inside the tile (its stores happen).
+template <uint32_t KIND>
+__device__ __forceinline__ uint4 pair_leaf(const TreeJob& job, uint64_t leaf, bool ok, const uint32_t (&ch)[4], uint32_t q) {
+  if constexpr (KIND == kLeafDigest) {
+    return pair_split_digest(__ldcg(reinterpret_cast<const ulonglong2*>(job.raw) + 2 * leaf + q), q);
+  } else {
+    uint32_t a[25];
+#pragma unroll
+    for (int i = 0; i < 25; i++) a[i] = 0;
+    if constexpr (KIND == kLeafQM31 || KIND == kLeafFold) {
+      uint4 v;
+      if constexpr (KIND == kLeafQM31) {
+        v = __ldg(job.layer + leaf);
+      } else {
+        v = folded_value(job, leaf, ch);
+        if (ok && q == 0) job.out_layer[leaf] = v;
+      }
+      const ulonglong2 w = pack_qm31(v);
+      pair_split2(q ? w.y : w.x, q, a[0], a[1]);
+      a[2] = pair_suffix(0x06, q);
+    } else if constexpr (KIND == kLeafQM31x4 || KIND == kLeafFoldx4) {
+      // thread q takes values 2q and 2q + 1 (lanes 4q .. 4q + 3)
+#pragma unroll
+      for (uint32_t m = 0; m < 2; m++) {
+        const uint64_t e = 4 * leaf + 2 * q + m;
+        uint4 v;
+        if constexpr (KIND == kLeafQM31x4) {
+          v = __ldg(job.layer + e);
+        } else {
+          v = folded_value(job, e, ch);
+          if (ok) job.out_layer[e] = v;
+        }
+        const ulonglong2 w = pack_qm31(v);
+        pair_split2(w.x, q, a[2 * m], a[4 + 2 * m]);
+        pair_split2(w.y, q, a[2 * m + 1], a[5 + 2 * m]);
+      }
+      a[8] = pair_suffix(0x06, q);
+    } else {
+      // words 2m by thread 0, 2m + 1 by thread 1
+      const uint8_t* p = job.raw + leaf * job.stride;
+      const uint32_t last = job.len >> 3;
+#pragma unroll
+      for (uint32_t m = 0; m < 9; m++) {
+        if (2 * m > last) continue;  // the same for the whole launch
+        uint32_t w1;
+        pair_split2(raw_message_word(job, p, 2 * m + q), q, a[2 * m], w1);
+        if (m < 8) a[2 * m + 1] = w1;
+      }
+    }
+    const bool two = KIND == kLeafRaw && job.len == 136;  // a full block, then the padding's own
+    if (!two) a[16] ^= pair_pad_end(q);
+#pragma unroll 1
+    for (uint32_t b = 0; b < (two ? 2u : 1u); b++) {
+      if (b == 1) {
+        a[0] ^= pair_suffix(job.suffix, q);
+        a[16] ^= pair_pad_end(q);
+      }
+      pair_f1600(a, q);
+    }
+    return make_uint4(a[0], a[1], a[2], a[3]);
+  }
+}
+
+// Digest i of `count` into shared memory (`buf` in split form, or `top` as it is)
+// and, joined, to global memory (`node`, null for none).
+__device__ __forceinline__ void put_digest(uint64_t* buf, uint64_t* top, uint32_t count, uint32_t i, uint4 d, uint64_t* node, bool ok, uint32_t q) {
+  const bool std_form = count <= kStdDigests;
+  if (node != nullptr || std_form) {  // the same for the whole warp
+    const ulonglong2 j = pair_join_digest(d, q);
+    if (ok && node != nullptr) reinterpret_cast<ulonglong2*>(node)[q] = j;
+    if (ok && std_form) reinterpret_cast<ulonglong2*>(top)[2 * i + q] = j;
+  }
+  if (ok && !std_form) reinterpret_cast<uint4*>(buf)[2 * i + q] = d;
+}
+
+// Leaf phase by pairs of lanes (fewer leaves than threads).
+template <uint32_t KIND, int THREADS>
+__device__ __noinline__ void pair_leaf_phase(const TreeJob& job, uint32_t items, uint64_t idx0, uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3,
+                                             uint64_t* out, uint64_t* top) {
+  const uint32_t ch[4] = {c0, c1, c2, c3};
+  const uint32_t lane = threadIdx.x & 31, q = lane & 1;
+  for (uint32_t base = threadIdx.x / 32 * 16; base < items; base += THREADS / 2) {
+    const uint32_t i = base + (lane >> 1);
+    const bool ok = i < items;
+    const uint64_t leaf = idx0 + (ok ? i : items - 1);
+    const uint4 d = pair_leaf<KIND>(job, leaf, ok, ch, q);
+    put_digest(out, top, items, i, d, job.leaf_digests ? job.leaf_digests + 4 * leaf : nullptr, ok, q);
+  }
+  __syncthreads();
+}
+
+// Levels of at least kStdDigests nodes, a pair of lanes per node, until kStdDigests
+// digests are left (in `top`): from `count` digests in buffer `a` (scratch `b`), or
+// (nodes != null) from the `count` tree nodes at `nodes`, written by other CTAs.
+// `level`, `idx0`: level and first node index of the digests; both advance.
+template <int THREADS>
+__device__ __noinline__ void pair_levels(uint64_t* a, uint64_t* b, uint64_t* top, const uint64_t* nodes, uint32_t n, const TreeJob& job, uint32_t level,
+                                         uint64_t idx0) {
+  const uint32_t lane = threadIdx.x & 31, q = lane & 1;
+  uint64_t* src = a;
+  uint64_t* dst = b;
+  if (nodes != nullptr) dst = a;
+  while (n > kStdDigests) {
+    n >>= 1;
+    idx0 >>= 1;
+    level++;
+    uint64_t* lv = job.inner + 4 * (inner_offset(job.logn, level) + idx0);
+    for (uint32_t base = threadIdx.x / 32 * 16; base < n; base += THREADS / 2) {
+      const uint32_t i = base + (lane >> 1);
+      const bool ok = i < n;
+      const uint32_t j = ok ? i : n - 1;
+      uint4 l, r;
+      if (nodes != nullptr) {
+        const ulonglong2* p = reinterpret_cast<const ulonglong2*>(nodes) + 4 * j + q;
+        l = pair_split_digest(__ldcg(p), q);
+        r = pair_split_digest(__ldcg(p + 2), q);
+      } else {
+        const uint4* p = reinterpret_cast<const uint4*>(src) + 4 * j + q;
+        l = p[0];
+        r = p[2];
+      }
+      put_digest(dst, top, n, i, pair_hash_parent(l, r, q), lv + 4 * j, ok, q);
+    }
+    __syncthreads();
+    if (nodes != nullptr) {
+      nodes = nullptr;
+      src = dst;
+      dst = b;
+    } else {
+      uint64_t* t = src;
+      src = dst;
+      dst = t;
+    }
+  }
+}
+
+// A parent node by one warp: children at src (8 lanes), the digest to dst (shared)
+// and node (global).
+__device__ __forceinline__ void warp_parent(const WarpKeccak& kf, const uint64_t* src, uint64_t* dst, uint64_t* node) {
+  const uint32_t lane = threadIdx.x & 31;
+  uint64_t a = lane < 8 ? src[lane] : lane == 8 ? 0x06ull : lane == 16 ? kPadEnd : 0ull;
+  kf.permute_small(a);
+  if (lane < 4) {
+    dst[lane] = a;
+    node[lane] = a;
+  }
+}
+
+// The last levels (at most kStdDigests digests in `top`) with a warp per node, and
+// in the CTA that reaches the root the root's transcript round.  The transcript's
+// first absorptions (the public digest before round 0, the commitment frame) need
+// no root, so the fourth warp takes them while the first two hash the top nodes.
+template <int THREADS>
+__device__ __noinline__ void top_levels(uint64_t* top, uint32_t count, const TreeJob& job, uint32_t level, uint64_t idx0, bool root, uint64_t* warp_smem) {
+  static_assert(THREADS >= 128, "four warps");
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t act = root ? job.root_action : (uint32_t)kRootNone;
+  if (warp >= 4) return;
+  if (warp == 3 && act != kRootNone) {
+    // one permutation site for all of this warp's steps
+    enum { kPublic, kNode, kCommit, kRoot, kChallenge };
+    WarpSponge sp(warp_smem + kWarpKeccakWords * 3);
+    const RoundFrames f = act == kRootCircleRound ? circle_round_frames(lane, job.round) : qm31_round_frames(lane, job.round, job.frame_in_count);
+    sp.load(job.base ? job.base : job.transcript);
+    uint64_t* const node = top + 8 * 4 + 4 * 3;  // the fourth node above eight digests
+#pragma unroll 1
+    for (uint32_t step = job.base ? kPublic : kNode; step <= kChallenge; step++) {
+      uint64_t word = 0, keep = 0;
+      if (step == kPublic) {
+        word = sp.digest_word(job.pub);
+      } else if (step == kNode) {
+        if (count != 8) continue;
+        keep = sp.a;
+        sp.a = lane < 8 ? top[24 + lane] : lane == 8 ? 0x06ull : lane == 16 ? kPadEnd : 0ull;
+      } else if (step == kCommit) {
+        word = f.commit;
+      } else if (step == kRoot) {
+        asm volatile("bar.sync 2, 128;" ::: "memory");
+        word = sp.digest_word(top + (count == 8 ? 56 : count == 4 ? 24 : count == 2 ? 8 : 0));
+      } else {
+        word = f.challenge;
+      }
+      sp.absorb(word);
+      if (step == kNode) {
+        uint64_t* const out = job.inner + 4 * (inner_offset(job.logn, level + 1) + (idx0 >> 1) + 3);
+        if (lane < 4) node[lane] = out[lane] = sp.a;
+        sp.a = keep;
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+      }
+    }
+    uint32_t ch[4];
+    sp.squeeze4_m31(ch);
+    sp.store(job.transcript);
+    if (lane == 0)
+      for (int k = 0; k < 4; k++) job.challenge_out[k] = ch[k];
+    return;
+  }
+  const WarpKeccak kf(lane, warp_smem + kWarpKeccakWords * warp);
+  uint64_t* src = top;
+  uint32_t n = count;
+  while (n > 1) {
+    n >>= 1;
+    idx0 >>= 1;
+    level++;
+    uint64_t* const dst = src + 8 * n;
+    if (warp < n) {
+      uint64_t* const node = job.inner + 4 * (inner_offset(job.logn, level) + idx0 + warp);
+      uint64_t a = lane < 8 ? src[8 * warp + lane] : lane == 8 ? 0x06ull : lane == 16 ? kPadEnd : 0ull;
+      kf.permute_small(a);
+      if (lane < 4) dst[4 * warp + lane] = node[lane] = a;
+    }
+    // four nodes take all four warps; below that only the first two go on
+    if (n == 4) {
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+    } else if (n == 2) {
+      if (warp >= 2) break;
+      asm volatile("bar.sync 3, 64;" ::: "memory");
+    }
+    src = dst;
+  }
+  if (root && warp == 0 && lane < 4 && job.root_out) job.root_out[lane] = src[lane];
+  if (act != kRootNone) asm volatile("bar.sync 2, 128;" ::: "memory");
 }
 
 // One tile of one job: leaf digests, treelet, then the last-arriver climb.
-// Shared memory: 2^(tl-2) digests + half as many for the ping-pong (12 bytes per leaf).
 template <uint32_t KIND, int THREADS>
 __device__ __forceinline__ void tree_tile_body(const TreeJob& job, const uint64_t tile) {
   extern __shared__ __align__(16) uint64_t sm[];
+  __shared__ __align__(16) uint64_t warp_smem[4 * kWarpKeccakWords];
+  __shared__ __align__(16) uint64_t top[kTopWords];
   __shared__ uint32_t s_last;
   __shared__ uint32_t s_ch[4];
   const uint32_t tl = job.tile_log < job.logn ? job.tile_log : job.logn;
   const uint32_t T = 1u << tl;
-  const uint32_t Q = T >= 4 ? T / 4 : 1;
-  uint64_t* bufA = sm;           // Q digests
-  uint64_t* bufB = sm + 4 * Q;   // Q/2 digests
+  const uint32_t M = tree_phase_digests(T, THREADS);  // capacity of bufA; bufB holds half
+  uint64_t* bufA = sm;
+  uint64_t* bufB = sm + 4 * M;
 
   uint32_t ch[4] = {0, 0, 0, 0};
   if constexpr (KIND == kLeafFold || KIND == kLeafFoldx4) {
@@ -251,11 +498,19 @@ __device__ __forceinline__ void tree_tile_body(const TreeJob& job, const uint64_
     for (int k = 0; k < 4; k++) ch[k] = s_ch[k];
   }
 
-  // 1) leaf digests and the two lowest levels of this tile, per thread
+  // 1) leaf digests (and the lowest levels of this tile, per thread)
   const uint64_t first = tile * T;
-  uint32_t h = subtree_phase<KIND, THREADS>(job, T, 0, first, nullptr, false, ch[0], ch[1], ch[2], ch[3], bufA);
-  // 2) treelet
-  uint64_t* res = reduce_levels(bufA, bufB, T >> h, job, h, first >> h);
+  uint32_t h = 0;
+  if (T < THREADS) {
+    pair_leaf_phase<KIND, THREADS>(job, T, first, ch[0], ch[1], ch[2], ch[3], bufA, top);
+  } else {
+    h = tree_subtree_height(T, THREADS);
+    subtree_phase<KIND, THREADS>(job, T, h, first, ch[0], ch[1], ch[2], ch[3], bufA);
+  }
+  // 2) treelet: the levels above, to kStdDigests digests and then to the root
+  uint32_t top_log = tl < kStdLog ? tl : kStdLog;
+  pair_levels<THREADS>(bufA, bufB, top, nullptr, T >> h, job, h, first >> h);
+  top_levels<THREADS>(top, 1u << top_log, job, tl - top_log, first >> (tl - top_log), tl == job.logn, warp_smem);
   // 3) climb: last arriver of each group continues
   uint32_t level = tl;
   uint64_t idx = tile;
@@ -263,7 +518,7 @@ __device__ __forceinline__ void tree_tile_body(const TreeJob& job, const uint64_
   while (level < job.logn) {
     uint32_t glog = job.group_log;
     if (glog > job.logn - level) glog = job.logn - level;
-    if (glog > tl) glog = tl;  // the group must fit the shared buffers (host keeps tl >= 1)
+    while (glog > 1 && (1u << glog) > 2 * M) glog--;  // the group's first level must fit bufA
     const uint32_t G = 1u << glog;
     const uint64_t gidx = idx >> glog;
     __syncthreads();
@@ -277,13 +532,19 @@ __device__ __forceinline__ void tree_tile_body(const TreeJob& job, const uint64_
     if (!s_last) return;
     __threadfence();
     const uint64_t* lv = job.inner + 4 * (inner_offset(job.logn, level) + gidx * G);
-    uint32_t hg = subtree_phase<KIND, THREADS>(job, G, level, gidx * G, lv, true, 0, 0, 0, 0, bufA);
-    res = reduce_levels(bufA, bufB, G >> hg, job, level + hg, (gidx * G) >> hg);
+    top_log = glog < kStdLog ? glog : kStdLog;
+    if (G > kStdDigests) {
+      pair_levels<THREADS>(bufA, bufB, top, lv, G, job, level, gidx * G);
+    } else {
+      if (threadIdx.x < 4 * G) top[threadIdx.x] = __ldcg(lv + threadIdx.x);
+      __syncthreads();
+    }
+    const uint32_t up = level + glog - top_log;
+    top_levels<THREADS>(top, 1u << top_log, job, up, (gidx * G) >> (glog - top_log), level + glog == job.logn, warp_smem);
     cnt_off += (1ull << (job.logn - level)) >> glog;
     level += glog;
     idx = gidx;
   }
-  if (threadIdx.x == 0) root_action(job, res);
 }
 
 template <uint32_t KIND, int THREADS>
@@ -325,7 +586,7 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) tree_direct_kernel(con
 }
 
 static constexpr int kMaxTreeLog = 13;
-static constexpr int kMaxTreeSmem = 12 << kMaxTreeLog;  // 2^11 digests + 2^10 digests
+static constexpr int kMaxTreeSmem = 12 << kMaxTreeLog;  // 2^11 digests + 2^10 digests (48 x 512 threads is less)
 
 template <uint32_t KIND>
 static cudaError_t prepare_kind() {
@@ -371,7 +632,7 @@ static uint32_t resident_grid(K kernel, int threads, size_t smem, uint32_t nwork
 template <uint32_t KIND>
 static cudaError_t launch_kind(const TreeJob* d_jobs, const uint2* d_work, uint32_t nwork, uint32_t max_tile_log, uint32_t threads, uint32_t* queue,
                                cudaStream_t s) {
-  size_t smem = max_tile_log >= 2 ? ((size_t)12 << max_tile_log) : 48;  // T/4 digests + T/8 digests
+  const size_t smem = tree_smem_bytes(max_tile_log, threads == 128 || threads == 512 ? threads : 256);
   if (queue) {
     if (threads == 128)
       tree_queue_kernel<KIND, 128><<<resident_grid(tree_queue_kernel<KIND, 128>, 128, smem, nwork), 128, smem, s>>>(d_jobs, d_work, nwork, queue);
@@ -411,7 +672,7 @@ cudaError_t launch_tree_direct_raw(const TreeJob& job, cudaStream_t s) {
   if (job.tile_log > 9 || (job.logn > 0 && job.tile_log == 0)) return cudaErrorInvalidValue;
   uint32_t tl = job.tile_log < job.logn ? job.tile_log : job.logn;
   unsigned tiles = 1u << (job.logn - tl);
-  tree_direct_kernel<kLeafRaw, 256><<<tiles, 256, tl >= 2 ? ((size_t)12 << tl) : 48, s>>>(job);
+  tree_direct_kernel<kLeafRaw, 256><<<tiles, 256, tree_smem_bytes(tl, 256), s>>>(job);
   return cudaGetLastError();
 }
 

@@ -11,6 +11,7 @@
 // batched kernel packs four tables into one CTA (sumcheck_packed_kernel).
 #include "azk_field.cuh"
 #include "azk_internal.h"
+#include "azk_keccak_coop.cuh"
 
 namespace azk {
 
@@ -22,85 +23,6 @@ __device__ void sc_frame(FrameBuf& f, uint8_t type) {
   fb_u32(f, 1);
   fb_u8(f, type);
 }
-
-// ---------------------------------------------------------------------------
-// Keccak-f[1600] spread over one warp, for the statement digest: one sponge over
-// the whole table is a chain of ~30,000 dependent permutations, so what counts is
-// the latency of one permutation, not throughput.  Lane x + 5y (< 25) holds state
-// lane (x, y); lanes 25..31 follow lane 0's indices and store nothing.  A round
-// is two exchanges, and its cost follows the number of exchange instructions
-// more than the number of dependent stages (measured on B200: three shuffle
-// stages 2.43 us per permutation, two shuffle stages 2.30 us, this form 1.98 us):
-//   1. every lane stores its lane into a column-major shared array (columns
-//      padded to 6 words so a column is two 16-byte loads and one 8-byte load)
-//      and reads columns x - 1 and x + 1: theta's D[x], then rho's rotation of
-//      its own lane, e = rotl(a ^ D[x], rho[x, y]), at the source.  Rounds
-//      alternate between two arrays, so the one __syncwarp after the stores also
-//      orders the previous round's loads of the other array before its next stores;
-//   2. pi and chi in one gather: lane (x, y) shuffles e from the pi sources of
-//      (x, y), (x + 1, y) and (x + 2, y); iota enters as chi(b0 ^ rc, b1, b2)
-//      (= chi(b0, b1, b2) ^ rc) through a mask that is zero except on lane 0, so
-//      its XOR overlaps the wait for the later shuffles.
-// ---------------------------------------------------------------------------
-__constant__ static const uint8_t kRhoOffsets[25] = {0,  1,  62, 28, 27, 36, 44, 6,  55, 20, 3,  10, 43,
-                                                     25, 39, 41, 45, 15, 21, 8,  18, 2,  61, 56, 14};
-
-struct WarpKeccak {
-  uint64_t* col;        // two arrays of 5 columns x 6 words, column-major (16-byte aligned)
-  uint32_t own;         // this lane's word in col
-  uint32_t cm, cp;      // first words of columns x - 1 and x + 1
-  uint32_t s0, s1, s2;  // pi sources of (x, y), (x + 1, y), (x + 2, y)
-  uint32_t swap, rot;   // rho[x, y] as a half swap (bit 5) and a funnel shift
-  uint64_t rc_mask;     // all ones on lane 0
-  bool stores;
-
-  __device__ WarpKeccak(uint32_t lane, uint64_t* smem) : col(smem) {
-    const uint32_t t = lane < 25 ? lane : 0;
-    const uint32_t x = t % 5, y = t / 5;
-    own = 6 * x + y;
-    cm = 6 * ((x + 4) % 5);
-    cp = 6 * ((x + 1) % 5);
-    // B[X, Y] = rotl(A'[xs, ys]) with X = ys, Y = 2 xs + 3 ys (mod 5); 2^-1 = 3 (mod 5)
-    auto src = [](uint32_t X, uint32_t Y) { return (((Y + 15 - 3 * X) % 5) * 3) % 5 + 5 * X; };
-    s0 = src(x, y);
-    s1 = src((x + 1) % 5, y);
-    s2 = src((x + 2) % 5, y);
-    const uint32_t r = kRhoOffsets[t];
-    swap = r & 32u;
-    rot = r & 31u;
-    rc_mask = lane == 0 ? ~0ull : 0ull;
-    stores = lane < 25;
-  }
-
-  __device__ __forceinline__ void permute(uint64_t& a) const {
-    // all 24 rounds unrolled: the round constants are immediates
-#pragma unroll
-    for (int r = 0; r < 24; r += 8) {
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-        uint64_t* const c = col + 32 * (k & 1);
-        if (stores) c[own] = a;
-        __syncwarp();
-        const ulonglong2 m01 = *reinterpret_cast<const ulonglong2*>(c + cm);
-        const ulonglong2 m23 = *reinterpret_cast<const ulonglong2*>(c + cm + 2);
-        const uint64_t m4 = c[cm + 4];
-        const ulonglong2 p01 = *reinterpret_cast<const ulonglong2*>(c + cp);
-        const ulonglong2 p23 = *reinterpret_cast<const ulonglong2*>(c + cp + 2);
-        const uint64_t p4 = c[cp + 4];
-        const uint64_t c_m = xor3_64(xor3_64(m01.x, m01.y, m23.x), m23.y, m4);
-        const uint64_t c_p = xor3_64(xor3_64(p01.x, p01.y, p23.x), p23.y, p4);
-        const uint64_t t = xor3_64(a, c_m, rotl<1>(c_p));
-        const uint32_t lo = (uint32_t)t, hi = (uint32_t)(t >> 32);
-        const uint32_t l2 = swap ? hi : lo, h2 = swap ? lo : hi;
-        const uint64_t e = ((uint64_t)__funnelshift_l(l2, h2, rot) << 32) | __funnelshift_l(h2, l2, rot);
-        const uint64_t b0 = __shfl_sync(0xffffffffu, e, s0) ^ (kKeccakRC[r + k] & rc_mask);
-        const uint64_t b1 = __shfl_sync(0xffffffffu, e, s1);
-        const uint64_t b2 = __shfl_sync(0xffffffffu, e, s2);
-        a = chi_64(b0, b1, b2);
-      }
-    }
-  }
-};
 
 // Byte k of the framed word-digest input: u32 len || "AppleZKProver.M31Sumcheck.Words.V1"
 // || u32 1 || u64 count || words (little-endian) (SumcheckOracle.swift:1288-1299).
