@@ -95,6 +95,11 @@ __host__ __device__ __forceinline__ qm31 fri_fold_pair(qm31 pos, qm31 neg, uint3
   return q_half(q_add(even, q_mul(ch, odd)));
 }
 
+// The same with a QM31 inverse-domain value.
+__host__ __device__ __forceinline__ qm31 fri_fold_pair_q(qm31 pos, qm31 neg, qm31 t, qm31 ch) {
+  return q_half(q_add(q_add(pos, neg), q_mul(ch, q_mul(q_sub(pos, neg), t))));
+}
+
 // ---- circle group over M31 (CircleDomain.swift:3-101) ----
 struct cpoint {
   uint32_t x, y;

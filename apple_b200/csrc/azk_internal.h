@@ -24,6 +24,7 @@ enum LeafKind : uint32_t {
   kLeafDigest = 3,  // prehashed 32-byte digests
   kLeafQM31x4 = 4,  // 64-byte leaves of 4 consecutive QM31 values
   kLeafFoldx4 = 5,  // fold of a previous layer into 4 values per 64-byte leaf, then hashed
+  kLeafFoldQ = 6,   // as kLeafFold with QM31 inverse-domain values (the QM31 fold plans')
 };
 
 enum RootAction : uint32_t {
@@ -45,7 +46,7 @@ struct TreeJob {
   uint32_t aligned8;   // raw base and stride are multiples of 8
   uint32_t pad0;
   const uint4* layer;  // kLeafQM31 values / kLeafFold previous layer (2n values)
-  const uint32_t* inv;     // kLeafFold inverse-domain values (n)
+  const uint32_t* inv;     // kLeafFold inverse-domain values (n; kLeafFoldQ: n QM31 values)
   const uint32_t* fold_ch; // kLeafFold challenge (4 limbs)
   uint4* out_layer;        // kLeafFold output layer (n values)
   // tree storage
@@ -60,7 +61,7 @@ struct TreeJob {
   uint32_t* challenge_out;  // 4 limbs
   uint64_t* root_out;       // 4 lanes
   // First round only (null otherwise): the transcript starts from *base, into which
-  // the public digest `pub` (4 lanes) is absorbed first.
+  // the public digest `pub` (4 lanes, null for none) is absorbed first.
   const Transcript* base;
   const uint64_t* pub;
 };
@@ -152,6 +153,7 @@ struct PcsInstance {
   uint64_t* trees;        // inner nodes of tree k at tree_offset(k)
   const uint32_t* tw;
   const uint32_t* inv;
+  Transcript* base;       // transcript up to the public digest (a function of the parameters)
   Transcript* transcript;
   uint32_t* challenges;   // 4 * rounds
   uint64_t* commitments;  // 4 * rounds
@@ -260,10 +262,13 @@ struct ScanJob {
 cudaError_t launch_scan_inputs(const ScanJob* d_jobs, uint32_t njobs, uint64_t max_n, uint32_t* d_bad, cudaStream_t s);
 cudaError_t launch_fold_jobs(const FoldJob* d_jobs, const uint2* d_work, uint32_t nwork, cudaStream_t s);
 cudaError_t launch_fold_qm31_inv(const uint4* prev, const uint4* inv, const uint32_t* ch, uint4* out, uint64_t n_out, cudaStream_t s);
-cudaError_t launch_pcs_prefix(PcsInstance* d_inst, uint32_t ninst, cudaStream_t s);
-cudaError_t launch_pcs_finalize(PcsInstance* d_inst, const uint32_t* d_ids, uint32_t nids, cudaStream_t s);
+cudaError_t launch_pcs_base(const PcsInstance* d_inst, uint32_t ninst, cudaStream_t s);
+cudaError_t launch_pcs_prefix(const PcsInstance* d_inst, uint32_t ninst, cudaStream_t s);
+// Final layers of at most this many values are folded by the tail kernel itself.
+static constexpr uint64_t kTailFold = 512;
+enum PcsTailParts : uint32_t { kTailFoldPart = 1, kTailBind = 2, kTailQueries = 4 };
+cudaError_t launch_pcs_tail(const PcsInstance* d_inst, const uint32_t* d_ids, uint32_t nids, uint32_t parts, cudaStream_t s);
 cudaError_t launch_pcs_grind(PcsInstance* d_inst, uint32_t id, uint64_t start, uint64_t count, unsigned long long* d_found, cudaStream_t s);
-cudaError_t launch_pcs_queries(PcsInstance* d_inst, const uint32_t* d_ids, uint32_t nids, cudaStream_t s);
 cudaError_t launch_pcs_emit(PcsInstance* d_inst, const uint32_t* d_ids, uint32_t nids, uint32_t max_queries, cudaStream_t s);
 // Encoded queries (proof codec layout) of one instance's resident layers and trees.
 cudaError_t launch_query_extract(const PcsInstance* d_inst, const uint32_t* d_pairs, uint32_t count, uint8_t* d_out, cudaStream_t s);

@@ -7,6 +7,7 @@
 // (Metal :1987-2032); transcript and proof layout CircleProofFormat.swift:475-983.
 #include "azk_field.cuh"
 #include "azk_internal.h"
+#include "azk_transcript_warp.cuh"
 
 namespace azk {
 
@@ -552,80 +553,138 @@ cudaError_t launch_fold_qm31_inv(const uint4* prev, const uint4* inv, const uint
 // ---------------------------------------------------------------------------
 // Circle FRI PCS V1 transcript (CircleProofFormat.swift:684-983)
 // ---------------------------------------------------------------------------
-__device__ void absorb_domain_codec(Transcript& t, uint32_t logn) {
-  // CircleDomainDescriptorCodecV1.encode (CircleProofFormat.swift:75-93)
-  FrameBuf f;
-  f.n = 0;
-  const uint8_t magic[8] = {0x41, 0x5a, 0x4b, 0x43, 0x44, 0x56, 0x31, 0x00};
-  for (int i = 0; i < 8; i++) fb_u8(f, magic[i]);
-  fb_u32(f, 1);
-  fb_u32(f, kP);
-  fb_u32(f, 31);
-  fb_u32(f, 2);
-  fb_u32(f, 1268011823u);
-  fb_u32(f, logn);
-  fb_u32(f, (uint32_t)((1ull << (31 - (logn + 1))) & 0x7FFFFFFFu));
-  fb_u32(f, logn - 1);
-  fb_u32(f, 1);
-  tr_absorb(t, f.b, f.n);
-}
+// CircleDomainDescriptorCodecV1.encode (CircleProofFormat.swift:75-93): the magic,
+// then u32 fields.
+struct DomainCodec {
+  static constexpr FrameBase base = {{0x00315644434B5A41ull, 0, 0, 0, 0, 0}, 8};
+};
 
-__global__ void pcs_prefix_kernel(PcsInstance* __restrict__ inst, uint32_t ninst) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+static constexpr int kSpongeWarps = 4;  // transcripts per CTA of the prefix kernel
+
+// The part of the transcript before round 0, one warp per instance.  `publics` ==
+// 0: header, domain, security parameters and the
+// public-input frame into *base, which depend on the parameters only; `publics`:
+// *base with the public digest absorbed, into *transcript.
+__global__ void __launch_bounds__(32 * kSpongeWarps) pcs_prefix_kernel(const PcsInstance* __restrict__ inst, uint32_t ninst, uint32_t publics) {
+  __shared__ __align__(16) uint64_t smem[kSpongeWarps * kWarpKeccakWords];
+  const uint32_t w = threadIdx.x >> 5, i = blockIdx.x * kSpongeWarps + w;
   if (i >= ninst) return;
-  PcsInstance& I = inst[i];
-  Transcript t;
-  tr_reset(t);
-  FrameBuf f;
-  circle_frame(f, 0);  // header
-  fb_u32(f, 1);
-  fb_u32(f, 1);
-  fb_u32(f, kP);
-  fb_u32(f, 2);
-  fb_u32(f, 1268011823u);
-  tr_absorb(t, f.b, f.n);
-  absorb_domain_codec(t, I.logn);
-  circle_frame(f, 1);  // security
-  fb_u32(f, I.log_blowup);
-  fb_u32(f, I.queries);
-  fb_u32(f, 1);
-  fb_u32(f, I.grinding_bits);
-  fb_u32(f, I.log_blowup * I.queries + I.grinding_bits);
-  tr_absorb(t, f.b, f.n);
-  circle_frame(f, 2);  // public input
-  fb_u32(f, 32);
-  tr_absorb(t, f.b, f.n);
-  uint64_t pub[4] = {I.pub[0], I.pub[1], I.pub[2], I.pub[3]};
-  tr_absorb_digest(t, pub);
-  *I.transcript = t;
+  const PcsInstance& I = inst[i];
+  WarpSponge sp(smem + w * kWarpKeccakWords);
+  const uint32_t lane = sp.lane;
+  if (publics) sp.load(I.base);
+#pragma unroll 1
+  for (uint32_t step = publics ? 4 : 0; step < (publics ? 5 : 4); step++) {
+    uint64_t word;
+    if (step == 0) {
+      const uint32_t p[5] = {1, 1, kP, 2, 1268011823u};
+      word = frame_word<CircleFrame>(lane, 0, p);
+    } else if (step == 1) {
+      const uint32_t p[9] = {1, kP, 31, 2, 1268011823u, I.logn, (uint32_t)((1ull << (31 - (I.logn + 1))) & 0x7FFFFFFFu), I.logn - 1, 1};
+      word = frame_word<DomainCodec>(lane, 0, p);
+    } else if (step == 2) {
+      const uint32_t p[5] = {I.log_blowup, I.queries, 1, I.grinding_bits, I.log_blowup * I.queries + I.grinding_bits};
+      word = frame_word<CircleFrame>(lane, 1, p);
+    } else if (step == 3) {
+      const uint32_t p[1] = {32};
+      word = frame_word<CircleFrame>(lane, 2, p);
+    } else {
+      word = sp.digest_word(I.pub);
+    }
+    sp.absorb(word);
+  }
+  sp.store(publics ? I.transcript : I.base);
 }
 
-cudaError_t launch_pcs_prefix(PcsInstance* d_inst, uint32_t ninst, cudaStream_t s) {
+cudaError_t launch_pcs_base(const PcsInstance* d_inst, uint32_t ninst, cudaStream_t s) {
   if (!ninst) return cudaSuccess;
-  pcs_prefix_kernel<<<(ninst + 63) / 64, 64, 0, s>>>(d_inst, ninst);
+  pcs_prefix_kernel<<<(ninst + kSpongeWarps - 1) / kSpongeWarps, 32 * kSpongeWarps, 0, s>>>(d_inst, ninst, 0);
+  return cudaGetLastError();
+}
+cudaError_t launch_pcs_prefix(const PcsInstance* d_inst, uint32_t ninst, cudaStream_t s) {
+  if (!ninst) return cudaSuccess;
+  pcs_prefix_kernel<<<(ninst + kSpongeWarps - 1) / kSpongeWarps, 32 * kSpongeWarps, 0, s>>>(d_inst, ninst, 1);
   return cudaGetLastError();
 }
 
-// Final-layer binding: frame (count, bytes) then the packed final layer.
-__global__ void pcs_finalize_kernel(PcsInstance* __restrict__ inst, const uint32_t* __restrict__ ids, uint32_t nids) {
-  uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= nids) return;
-  PcsInstance& I = inst[ids[j]];
-  Transcript t = *I.transcript;
-  uint64_t cnt = 1ull << (I.logn - I.rounds);
-  FrameBuf f;
-  circle_frame(f, 5);
-  fb_u64(f, cnt);
-  fb_u64(f, cnt * 16);
-  tr_absorb(t, f.b, f.n);
-  const uint8_t* fl = reinterpret_cast<const uint8_t*>(I.layers + layer_offset(I.logn, I.rounds));
-  tr_absorb(t, fl, (uint32_t)(cnt * 16));
-  *I.transcript = t;
+// The transcript after the last round, one CTA per instance: the final fold (when
+// the final layer has at most kTailFold values; larger ones come from fold_kernel),
+// the final-layer binding (frame, then the packed layer) and the query indices (the
+// nonce when there is one, the query frame, q pair indices mod N/2).  `parts`: which
+// of the three (the queries run apart when a nonce is searched before them).  A chain of dependent permutations by one warp: 68 + 14 us by one
+// thread, 25 us so (64-value layer, 32 queries).
+__global__ void __launch_bounds__(128) pcs_tail_kernel(const PcsInstance* __restrict__ inst, const uint32_t* __restrict__ ids, uint32_t parts) {
+  __shared__ __align__(16) uint64_t smem[kWarpKeccakWords];
+  const PcsInstance& I = inst[ids[blockIdx.x]];
+  const uint64_t cnt = 1ull << (I.logn - I.rounds);
+  uint4* const fl = I.layers + layer_offset(I.logn, I.rounds);
+  if ((parts & kTailFoldPart) && cnt <= kTailFold) {
+    const uint32_t k = I.rounds;  // >= 1
+    const uint4* prev = I.layers + layer_offset(I.logn, k - 1);
+    const uint32_t* inv = I.inv + (k == 1 ? 0 : (1ull << I.logn) - ((1ull << I.logn) >> (k - 1)));
+    const uint32_t* c = I.challenges + 4 * (k - 1);
+    const qm31 ch = {__ldcg(c), __ldcg(c + 1), __ldcg(c + 2), __ldcg(c + 3)};
+    for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x) {
+      const uint4 p = __ldg(prev + 2 * i), q = __ldg(prev + 2 * i + 1);
+      const qm31 r = fri_fold_pair(qm31{p.x, p.y, p.z, p.w}, qm31{q.x, q.y, q.z, q.w}, __ldg(inv + i), ch);
+      fl[i] = make_uint4(r.a, r.b, r.c, r.d);
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x >= 32 || !(parts & (kTailBind | kTailQueries))) return;
+  WarpSponge sp(smem);
+  const uint32_t lane = sp.lane;
+  sp.load(I.transcript);
+  // blocks of the final layer: 2 cnt words, the last block holding fewer than 17
+  const uint64_t words = 2 * cnt, blocks = words / 17 + 1;
+  const uint64_t* fw = reinterpret_cast<const uint64_t*>(fl);
+  const uint64_t first = (parts & kTailBind) ? 0 : blocks + 1;
+  const uint64_t end = (parts & kTailQueries) ? blocks + 4 : blocks + 1;
+#pragma unroll 1
+  for (uint64_t step = first; step < end; step++) {
+    uint64_t word = 0;
+    if (step == 0) {
+      const uint32_t p[4] = {(uint32_t)cnt, (uint32_t)(cnt >> 32), (uint32_t)(cnt * 16), (uint32_t)((cnt * 16) >> 32)};
+      word = frame_word<CircleFrame>(lane, 5, p);
+    } else if (step <= blocks) {
+      const uint64_t left = words - 17 * (step - 1);
+      if (lane < 17 && lane < left) word = fw[17 * (step - 1) + lane];
+      if (left < 17) {
+        if (lane == left) word = 0x06;
+        if (lane == 16) word ^= kPadEnd;
+      }
+    } else if (step == blocks + 1) {
+      if (!I.has_nonce) continue;
+      const uint32_t p[2] = {I.grinding_bits, 8};
+      word = frame_word<CircleFrame>(lane, 7, p);
+    } else if (step == blocks + 2) {
+      if (!I.has_nonce) continue;
+      word = lane == 0 ? I.nonce : lane == 1 ? 0x06ull : lane == 16 ? kPadEnd : 0ull;
+    } else {
+      const uint64_t half = 1ull << (I.logn - 1);
+      const uint32_t p[3] = {I.queries, (uint32_t)half, (uint32_t)(half >> 32)};
+      word = frame_word<CircleFrame>(lane, 6, p);
+    }
+    sp.absorb(word);
+  }
+  sp.store(I.transcript);
+  if (!(parts & kTailQueries)) return;
+  // 34 words per squeezed block; the modulus is a power of two, so none is rejected
+  const uint32_t mask = (1u << (I.logn - 1)) - 1;
+#pragma unroll 1
+  for (uint32_t base = 0;;) {
+    const uint32_t q = base + 2 * lane;
+    if (lane < 17 && q < I.queries) I.query_pairs[q] = (uint32_t)sp.a & mask;
+    if (lane < 17 && q + 1 < I.queries) I.query_pairs[q + 1] = (uint32_t)(sp.a >> 32) & mask;
+    base += 34;
+    if (base >= I.queries) break;
+    sp.absorb(0);
+  }
 }
 
-cudaError_t launch_pcs_finalize(PcsInstance* d_inst, const uint32_t* d_ids, uint32_t nids, cudaStream_t s) {
+cudaError_t launch_pcs_tail(const PcsInstance* d_inst, const uint32_t* d_ids, uint32_t nids, uint32_t parts, cudaStream_t s) {
   if (!nids) return cudaSuccess;
-  pcs_finalize_kernel<<<(nids + 63) / 64, 64, 0, s>>>(d_inst, d_ids, nids);
+  pcs_tail_kernel<<<nids, 128, 0, s>>>(d_inst, d_ids, parts);
   return cudaGetLastError();
 }
 
@@ -669,28 +728,6 @@ cudaError_t launch_pcs_grind(PcsInstance* d_inst, uint32_t id, uint64_t start, u
   return cudaGetLastError();
 }
 
-// Optional grinding absorb, then the query frame and q pair indices mod N/2.
-__global__ void pcs_queries_kernel(PcsInstance* __restrict__ inst, const uint32_t* __restrict__ ids, uint32_t nids) {
-  uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= nids) return;
-  PcsInstance& I = inst[ids[j]];
-  Transcript t = *I.transcript;
-  if (I.has_nonce) absorb_grinding(t, I.grinding_bits, I.nonce);
-  FrameBuf f;
-  circle_frame(f, 6);
-  fb_u32(f, I.queries);
-  fb_u64(f, 1ull << (I.logn - 1));
-  tr_absorb(t, f.b, f.n);
-  tr_squeeze_u32(t, I.queries, 1u << (I.logn - 1), I.query_pairs);
-  *I.transcript = t;
-}
-
-cudaError_t launch_pcs_queries(PcsInstance* d_inst, const uint32_t* d_ids, uint32_t nids, cudaStream_t s) {
-  if (!nids) return cudaSuccess;
-  pcs_queries_kernel<<<(nids + 63) / 64, 64, 0, s>>>(d_inst, d_ids, nids);
-  return cudaGetLastError();
-}
-
 // ---------------------------------------------------------------------------
 // Proof bytes (CirclePCSFRIProofCodecV1.encode, CircleProofFormat.swift:478-593).
 // Every field starts at a 4-byte multiple, so the proof is written with u32
@@ -719,45 +756,67 @@ __device__ void pcs_sibling(const PcsInstance& I, uint32_t k, uint64_t idx, uint
   }
 }
 
-// One value opening at byte offset `off`; returns its size.
-__device__ uint64_t pcs_write_opening(const PcsInstance& I, uint32_t k, uint64_t idx, uint8_t* b, uint64_t off) {
-  uint32_t depth = I.logn - k;
-  uint4 v = I.layers[layer_offset(I.logn, k) + idx];
+// The head of a value opening at byte offset `off`: index, value, depth.
+__device__ __forceinline__ void pcs_write_opening_head(const PcsInstance& I, uint32_t k, uint64_t idx, uint8_t* b, uint64_t off) {
+  const uint4 v = I.layers[layer_offset(I.logn, k) + idx];
   pw64(b, off, idx);
   pw32(b, off + 8, v.x);
   pw32(b, off + 12, v.y);
   pw32(b, off + 16, v.z);
   pw32(b, off + 20, v.w);
-  pw32(b, off + 24, depth);
-  for (uint32_t l = 0; l < depth; l++) {
+  pw32(b, off + 24, I.logn - k);
+}
+// One value opening at byte offset `off`.
+__device__ void pcs_write_opening(const PcsInstance& I, uint32_t k, uint64_t idx, uint8_t* b, uint64_t off) {
+  pcs_write_opening_head(I, k, idx, b, off);
+  for (uint32_t l = 0; l < I.logn - k; l++) {
     uint64_t d[4];
     pcs_sibling(I, k, idx, l, d);
     pwdig(b, off + 28 + 32ull * l, d);
   }
-  return opening_bytes(depth);
 }
 
 // One query (CircleFRIQueryV1 encoding: initial pair, layer count, then per layer
 // its index, pair index and the left and right value openings) at byte `qoff` of
-// `b`; the block's threads split the layers' openings.
+// `b`.  The block's first threads take the openings' level-0 siblings (each is a
+// leaf digest, recomputed by one permutation); all of them then copy the other
+// digests and the openings' heads, 32 slots (levels 1 .. 30, head in slot 0) per
+// opening.  One thread per opening made a chain of 22 loads and took 23 us at 2^22.
+static constexpr uint32_t kEmitThreads = 128;
+__device__ __forceinline__ uint64_t layer_query_offset(uint32_t logn, uint32_t k) {
+  // 12 bytes, then 12 + 2 opening_bytes(logn - j) for each layer j < k
+  return 12 + (uint64_t)k * (12 + 2 * opening_bytes(logn)) - 32ull * k * (k - (k > 0));
+}
 __device__ void emit_query(const PcsInstance& I, uint64_t pair, uint8_t* b, uint64_t qoff) {
   const uint32_t R = I.rounds;
   if (threadIdx.x == 0) {
     pw64(b, qoff, pair);
     pw32(b, qoff + 8, R);
   }
-  // thread (k, side) writes layer k's left (side 0) or right opening
-  for (uint32_t t = threadIdx.x; t < 2 * R; t += blockDim.x) {
-    uint32_t k = t >> 1, side = t & 1;
-    uint64_t off = qoff + 12;
-    for (uint32_t j = 0; j < k; j++) off += 12 + 2 * opening_bytes(I.logn - j);
-    uint64_t pk = pair >> k;
-    if (side == 0) {
-      pw32(b, off, k);
-      pw64(b, off + 4, pk);
+  for (uint32_t t = threadIdx.x; t < 2 * R; t += kEmitThreads) {
+    const uint32_t k = t >> 1, side = t & 1;
+    const uint32_t depth = I.logn - k;
+    if (depth == 0) continue;
+    uint64_t d[4];
+    pcs_sibling(I, k, 2 * (pair >> k) + side, 0, d);
+    pwdig(b, qoff + layer_query_offset(I.logn, k) + 12 + (side ? opening_bytes(depth) : 0) + 28, d);
+  }
+  for (uint32_t t = threadIdx.x; t < 64 * R; t += kEmitThreads) {
+    const uint32_t k = t >> 6, side = (t >> 5) & 1, l = t & 31;
+    const uint32_t depth = I.logn - k;
+    const uint64_t pk = pair >> k, idx = 2 * pk + side;
+    const uint64_t off = qoff + layer_query_offset(I.logn, k), oo = off + 12 + (side ? opening_bytes(depth) : 0);
+    if (l == 0) {
+      if (side == 0) {
+        pw32(b, off, k);
+        pw64(b, off + 4, pk);
+      }
+      pcs_write_opening_head(I, k, idx, b, oo);
+    } else if (l < depth) {
+      uint64_t d[4];
+      pcs_sibling(I, k, idx, l, d);
+      pwdig(b, oo + 28 + 32ull * l, d);
     }
-    uint64_t oo = off + 12 + (side ? opening_bytes(I.logn - k) : 0);
-    pcs_write_opening(I, k, 2 * pk + side, b, oo);
   }
 }
 
@@ -829,7 +888,7 @@ __global__ void pcs_emit_kernel(const PcsInstance* __restrict__ inst, const uint
 cudaError_t launch_pcs_emit(PcsInstance* d_inst, const uint32_t* d_ids, uint32_t nids, uint32_t max_queries, cudaStream_t s) {
   if (!nids) return cudaSuccess;
   dim3 grid(nids, max_queries + 1);
-  pcs_emit_kernel<<<grid, 64, 0, s>>>(d_inst, d_ids, max_queries);
+  pcs_emit_kernel<<<grid, kEmitThreads, 0, s>>>(d_inst, d_ids, max_queries);
   return cudaGetLastError();
 }
 
@@ -843,55 +902,49 @@ __global__ void query_extract_kernel(const PcsInstance* __restrict__ inst, const
 
 cudaError_t launch_query_extract(const PcsInstance* d_inst, const uint32_t* d_pairs, uint32_t count, uint8_t* d_out, cudaStream_t s) {
   if (!count) return cudaSuccess;
-  query_extract_kernel<<<count, 64, 0, s>>>(d_inst, d_pairs, d_out);
+  query_extract_kernel<<<count, kEmitThreads, 0, s>>>(d_inst, d_pairs, d_out);
   return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------
 // QM31 fold-chain transcript (QM31FRIFold.swift:91-125, 769-862)
 // ---------------------------------------------------------------------------
-__global__ void qm31_prefix_kernel(Transcript* t, uint64_t input_count, uint32_t rounds) {
-  if (threadIdx.x || blockIdx.x) return;
-  Transcript s;
-  tr_reset(s);
-  FrameBuf f;
-  qm31_frame(f, 0);
-  fb_u64(f, input_count);
-  fb_u32(f, rounds);
-  fb_u32(f, kP);
-  fb_u32(f, 4);
-  fb_u32(f, 32);
-  tr_absorb(s, f.b, f.n);
-  *t = s;
+__global__ void __launch_bounds__(32) qm31_prefix_kernel(Transcript* t, uint64_t input_count, uint32_t rounds) {
+  __shared__ __align__(16) uint64_t smem[kWarpKeccakWords];
+  WarpSponge sp(smem);
+  const uint32_t p[6] = {(uint32_t)input_count, (uint32_t)(input_count >> 32), rounds, kP, 4, 32};
+  sp.absorb(frame_word<Qm31Frame>(sp.lane, 0, p));
+  sp.store(t);
 }
 
 cudaError_t launch_qm31_transcript_prefix(Transcript* d_t, uint64_t input_count, uint32_t rounds, cudaStream_t s) {
-  qm31_prefix_kernel<<<1, 1, 0, s>>>(d_t, input_count, rounds);
+  qm31_prefix_kernel<<<1, 32, 0, s>>>(d_t, input_count, rounds);
   return cudaGetLastError();
 }
 
 // Challenges from caller-supplied commitments: kind 1 = Circle V1 rounds (prefix
 // already absorbed), kind 2 = QM31 fold-chain rounds.
-__global__ void transcript_rounds_kernel(Transcript* t, uint32_t kind, const uint64_t* roots, uint32_t rounds, uint64_t input_count, uint32_t* ch) {
-  if (threadIdx.x || blockIdx.x) return;
-  Transcript s = *t;
-  uint64_t cnt = input_count;
+__global__ void __launch_bounds__(32) transcript_rounds_kernel(Transcript* t, uint32_t kind, const uint64_t* roots, uint32_t rounds,
+                                                               uint64_t input_count, uint32_t* ch) {
+  __shared__ __align__(16) uint64_t smem[kWarpKeccakWords];
+  WarpSponge sp(smem);
+  sp.load(t);
+#pragma unroll 1
   for (uint32_t r = 0; r < rounds; r++) {
-    uint64_t root[4] = {roots[4 * r], roots[4 * r + 1], roots[4 * r + 2], roots[4 * r + 3]};
+    const RoundFrames f = kind == kRootCircleRound ? circle_round_frames(sp.lane, r) : qm31_round_frames(sp.lane, r, input_count >> r);
+#pragma unroll 1
+    for (uint32_t step = 0; step < 3; step++) sp.absorb(step == 0 ? f.commit : step == 1 ? sp.digest_word(roots + 4 * r) : f.challenge);
     uint32_t c[4];
-    if (kind == kRootCircleRound)
-      circle_round(s, r, root, c);
-    else
-      qm31_round(s, r, cnt, root, c);
-    for (int k = 0; k < 4; k++) ch[4 * r + k] = c[k];
-    cnt >>= 1;
+    sp.squeeze4_m31(c);
+    if (sp.lane == 0)
+      for (int k = 0; k < 4; k++) ch[4 * r + k] = c[k];
   }
-  *t = s;
+  sp.store(t);
 }
 
 cudaError_t launch_transcript_rounds_given(Transcript* d_t, uint32_t kind, const uint64_t* d_roots, uint32_t rounds, uint64_t input_count,
                                            uint32_t* d_ch, cudaStream_t s) {
-  transcript_rounds_kernel<<<1, 1, 0, s>>>(d_t, kind, d_roots, rounds, input_count, d_ch);
+  transcript_rounds_kernel<<<1, 32, 0, s>>>(d_t, kind, d_roots, rounds, input_count, d_ch);
   return cudaGetLastError();
 }
 

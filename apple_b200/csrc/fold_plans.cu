@@ -156,7 +156,7 @@ struct azk_fold_chain_plan {
   std::vector<uint64_t> offset;   // element offset of round r's layer in the layer log
   std::vector<uint64_t> inv_off;  // element offset of round r's inverse-domain layer
   uint64_t layer_log = 0, inv_total = 0;
-  DevBuf ev, inv, layers, out, ch, cm, tr;
+  DevBuf ev, inv, layers, out, ch, cm, tr, base;
   // Merkle mode: one tree's inner nodes and counters (rounds run one after another)
   DevBuf inner, counters, jobs, work;
   std::vector<TreeJob> tree_jobs;
@@ -194,28 +194,39 @@ void chain_fold_all(azk_fold_chain_plan* p, const uint4* ev, const uint4* inv, u
 
 // Merkle-bound chain.  Layer r (r >= 1) is written into `log` at offset[r]; layer
 // 0 is read from `ev` (copied into log[0] first when `copy_first`).  With
-// `first_root` (device), round 0's commitment is that root instead of a tree.
+// `first_root` (device), round 0's commitment is that root instead of a tree.  The
+// fold into layer r runs inside round r's tree launch (the leaf is folded, stored
+// and hashed); only the final fold is a launch of its own.
 void chain_merkle(azk_fold_chain_plan* p, const uint4* ev, const uint4* inv, uint4* log, bool copy_first, uint4* out, const uint64_t* first_root) {
-  if (p->root_kind == kRootCircleRound)
-    AZK_CU(launch_pcs_prefix(p->pcs.as<PcsInstance>(), 1, p->s));
-  else
-    AZK_CU(launch_qm31_transcript_prefix(p->tr.as<Transcript>(), p->n_in, p->rounds, p->s));
   if (copy_first) AZK_CU(cudaMemcpyAsync(log, ev, kQ * p->n_in, cudaMemcpyDeviceToDevice, p->s));
   const uint4* cur = copy_first ? log : ev;
   // per-round layer pointers in the tree jobs: rewritten for this call
-  for (uint32_t r = 0; r < p->rounds; r++) p->tree_jobs[r].layer = r == 0 ? cur : p->layer_at(log, r);
+  for (uint32_t r = 0; r < p->rounds; r++) {
+    TreeJob& j = p->tree_jobs[r];
+    if (r == 0) {
+      j.layer = cur;
+    } else {
+      j.layer = r == 1 ? cur : p->layer_at(log, r - 1);
+      j.inv = reinterpret_cast<const uint32_t*>(inv + p->inv_off[r - 1]);
+      j.out_layer = p->layer_at(log, r);
+    }
+  }
   AZK_CU(cudaMemcpyAsync(p->jobs.p, p->tree_jobs.data(), sizeof(TreeJob) * p->rounds, cudaMemcpyHostToDevice, p->s));
   for (uint32_t r = 0; r < p->rounds; r++) {
     if (r == 0 && first_root) {
+      if (p->root_kind == kRootCircleRound)
+        AZK_CU(launch_pcs_prefix(p->pcs.as<PcsInstance>(), 1, p->s));
+      else
+        AZK_CU(cudaMemcpyAsync(p->tr.p, p->base.p, sizeof(Transcript), cudaMemcpyDeviceToDevice, p->s));
       AZK_CU(cudaMemcpyAsync(p->cm.p, first_root, 32, cudaMemcpyDeviceToDevice, p->s));
       AZK_CU(launch_transcript_rounds_given(p->tr.as<Transcript>(), p->root_kind, p->cm.as<uint64_t>(), 1, p->n_in, p->ch.as<uint32_t>(), p->s));
     } else {
       AZK_CU(launch_tree_jobs(p->jobs.as<TreeJob>(), p->work.as<uint2>() + p->work_range[r].first, (uint32_t)p->work_range[r].second,
-                              p->tree_jobs[r].tile_log, kLeafQM31, tree_threads(p->sched, p->tree_jobs[r].logn), p->s));
+                              p->tree_jobs[r].tile_log, p->tree_jobs[r].kind, tree_threads(p->sched, p->tree_jobs[r].logn), p->s));
     }
-    uint4* next = r + 1 == p->rounds ? out : p->layer_at(log, r + 1);
-    chain_fold(p, r, r == 0 ? cur : p->layer_at(log, r), inv, next);
   }
+  const uint32_t last = p->rounds - 1;
+  chain_fold(p, last, last == 0 ? cur : p->layer_at(log, last), inv, out);
 }
 
 const uint4* dev_q(const void* b, uint64_t off) { return reinterpret_cast<const uint4*>(static_cast<const uint8_t*>(b) + off); }
@@ -285,6 +296,7 @@ azk_status azk_fold_chain_plan_create(azk_ctx* ctx, uint64_t input_count, uint32
     p->ch.alloc(16ull * rounds, "QM31FRIFoldChain.Challenges");
     p->cm.alloc(32ull * rounds, "QM31FRIFoldChain.Commitments");
     p->tr.alloc(sizeof(Transcript), "QM31FRIFoldChain.Transcript");
+    p->base.alloc(sizeof(Transcript), "QM31FRIFoldChain.TranscriptBase");
     if (p->merkle_capable()) {
       // one committed tree at a time: the round-0 tree is the largest
       p->sched = resolve_schedule(nullptr, kTuned_pcs_single, kTunedThreads_pcs_single);
@@ -295,9 +307,11 @@ azk_status azk_fold_chain_plan_create(azk_ctx* ctx, uint64_t input_count, uint32
         const uint32_t lg = logn - r;
         TreeJob j{};
         j.logn = lg;
-        j.kind = kLeafQM31;
+        j.kind = r == 0 ? kLeafQM31 : kLeafFoldQ;
         j.tile_log = tree_tile_log(p->sched, lg);
         j.group_log = std::max<uint32_t>(1, std::min(p->sched.group_log, j.tile_log));
+        if (r == 0) j.base = p->base.as<Transcript>();
+        if (r > 0) j.fold_ch = p->ch.as<uint32_t>() + 4 * (r - 1);
         j.root_action = kRootQM31Round;
         j.round = r;
         j.frame_in_count = input_count >> r;
@@ -320,6 +334,7 @@ azk_status azk_fold_chain_plan_create(azk_ctx* ctx, uint64_t input_count, uint32
       }
       AZK_CU(cudaMemsetAsync(p->counters.p, 0, p->counters.bytes, p->s));
       AZK_CU(cudaMemcpyAsync(p->work.p, work.data(), sizeof(uint2) * work.size(), cudaMemcpyHostToDevice, p->s));
+      AZK_CU(launch_qm31_transcript_prefix(p->base.as<Transcript>(), p->n_in, p->rounds, p->s));
       sync_stream(p->s);
     }
     *out = p.release();
@@ -983,12 +998,15 @@ azk_status azk_circle_merkle_chain_plan_create(azk_ctx* ctx, uint32_t log_size, 
     I.log_blowup = log_blowup;
     I.grinding_bits = grinding_bits;
     std::memcpy(I.pub, public_digest, 32);
+    I.base = c->base.as<Transcript>();
     I.transcript = c->tr.as<Transcript>();
     c->pcs.alloc(sizeof(PcsInstance), "CircleFRIMerkleChain.Instance");
     AZK_CU(cudaMemcpyAsync(c->pcs.p, &I, sizeof(PcsInstance), cudaMemcpyHostToDevice, c->s));
+    AZK_CU(launch_pcs_base(c->pcs.as<PcsInstance>(), 1, c->s));
     sync_stream(c->s);
     c->root_kind = kRootCircleRound;
     for (auto& j : c->tree_jobs) j.root_action = kRootCircleRound;
+    c->tree_jobs[0].pub = c->pcs.as<PcsInstance>()->pub;
     *out = p.release();
   });
 }

@@ -43,12 +43,6 @@ __device__ __forceinline__ void leaf_digest(const TreeJob& job, uint64_t leaf, c
   if constexpr (KIND == kLeafQM31) {
     uint4 v = __ldg(job.layer + leaf);
     sha3_16((uint64_t)v.x | ((uint64_t)v.y << 32), (uint64_t)v.z | ((uint64_t)v.w << 32), d);
-  } else if constexpr (KIND == kLeafFold) {
-    uint4 p = __ldg(job.layer + 2 * leaf), q = __ldg(job.layer + 2 * leaf + 1);
-    uint32_t t = __ldg(job.inv + leaf);
-    qm31 r = fri_fold_pair(qm31{p.x, p.y, p.z, p.w}, qm31{q.x, q.y, q.z, q.w}, t, qm31{ch[0], ch[1], ch[2], ch[3]});
-    job.out_layer[leaf] = make_uint4(r.a, r.b, r.c, r.d);
-    sha3_16((uint64_t)r.a | ((uint64_t)r.b << 32), (uint64_t)r.c | ((uint64_t)r.d << 32), d);
   } else if constexpr (KIND == kLeafDigest) {
     ld_dig(reinterpret_cast<const uint64_t*>(job.raw) + 4 * leaf, d);
   } else {
@@ -56,18 +50,31 @@ __device__ __forceinline__ void leaf_digest(const TreeJob& job, uint64_t leaf, c
   }
 }
 
+// Value e of the layer that a fold kind produces.
+template <uint32_t KIND>
+__device__ __forceinline__ uint4 folded_value(const TreeJob& job, uint64_t e, const uint32_t (&ch)[4]) {
+  const uint4 p = __ldg(job.layer + 2 * e), q = __ldg(job.layer + 2 * e + 1);
+  const qm31 pos = {p.x, p.y, p.z, p.w}, neg = {q.x, q.y, q.z, q.w}, c = {ch[0], ch[1], ch[2], ch[3]};
+  qm31 r;
+  if constexpr (KIND == kLeafFoldQ) {
+    const uint4 t = __ldg(reinterpret_cast<const uint4*>(job.inv) + e);
+    r = fri_fold_pair_q(pos, neg, qm31{t.x, t.y, t.z, t.w}, c);
+  } else {
+    r = fri_fold_pair(pos, neg, __ldg(job.inv + e), c);
+  }
+  return make_uint4(r.a, r.b, r.c, r.d);
+}
+
 // Sets up the sponge input of one leaf (message lanes, suffix and end padding)
 // and returns how many permutations it takes (2 for a 136-byte raw leaf).
 template <uint32_t KIND>
 __device__ __forceinline__ uint32_t leaf_setup(const TreeJob& job, uint64_t leaf, const uint32_t (&ch)[4], uint64_t (&a)[25]) {
-  if constexpr (KIND == kLeafQM31 || KIND == kLeafFold) {
+  if constexpr (KIND == kLeafQM31 || KIND == kLeafFold || KIND == kLeafFoldQ) {
     uint4 v;
     if constexpr (KIND == kLeafQM31) {
       v = __ldg(job.layer + leaf);
     } else {
-      uint4 p = __ldg(job.layer + 2 * leaf), q = __ldg(job.layer + 2 * leaf + 1);
-      qm31 r = fri_fold_pair(qm31{p.x, p.y, p.z, p.w}, qm31{q.x, q.y, q.z, q.w}, __ldg(job.inv + leaf), qm31{ch[0], ch[1], ch[2], ch[3]});
-      v = make_uint4(r.a, r.b, r.c, r.d);
+      v = folded_value<KIND>(job, leaf, ch);
       job.out_layer[leaf] = v;
     }
     a[0] = (uint64_t)v.x | ((uint64_t)v.y << 32);
@@ -84,9 +91,7 @@ __device__ __forceinline__ uint32_t leaf_setup(const TreeJob& job, uint64_t leaf
       if constexpr (KIND == kLeafQM31x4) {
         v = __ldg(job.layer + e);
       } else {
-        uint4 p = __ldg(job.layer + 2 * e), q = __ldg(job.layer + 2 * e + 1);
-        qm31 r = fri_fold_pair(qm31{p.x, p.y, p.z, p.w}, qm31{q.x, q.y, q.z, q.w}, __ldg(job.inv + e), qm31{ch[0], ch[1], ch[2], ch[3]});
-        v = make_uint4(r.a, r.b, r.c, r.d);
+        v = folded_value<KIND>(job, e, ch);
         job.out_layer[e] = v;
       }
       a[2 * m] = (uint64_t)v.x | ((uint64_t)v.y << 32);
@@ -234,12 +239,6 @@ __device__ __noinline__ void subtree_phase(const TreeJob& job, uint32_t items, u
 __device__ __forceinline__ ulonglong2 pack_qm31(uint4 v) {
   return make_ulonglong2((uint64_t)v.x | ((uint64_t)v.y << 32), (uint64_t)v.z | ((uint64_t)v.w << 32));
 }
-// Value e of the layer that a fold kind produces.
-__device__ __forceinline__ uint4 folded_value(const TreeJob& job, uint64_t e, const uint32_t (&ch)[4]) {
-  const uint4 p = __ldg(job.layer + 2 * e), q = __ldg(job.layer + 2 * e + 1);
-  const qm31 r = fri_fold_pair(qm31{p.x, p.y, p.z, p.w}, qm31{q.x, q.y, q.z, q.w}, __ldg(job.inv + e), qm31{ch[0], ch[1], ch[2], ch[3]});
-  return make_uint4(r.a, r.b, r.c, r.d);
-}
 // Word i (< 17) of a raw message of `len` bytes with its suffix (none at len 136).
 __device__ __forceinline__ uint64_t raw_message_word(const TreeJob& job, const uint8_t* p, uint32_t i) {
   const uint32_t full = job.len >> 3, rem = job.len & 7;
@@ -261,12 +260,12 @@ __device__ __forceinline__ uint4 pair_leaf(const TreeJob& job, uint64_t leaf, bo
     uint32_t a[25];
 #pragma unroll
     for (int i = 0; i < 25; i++) a[i] = 0;
-    if constexpr (KIND == kLeafQM31 || KIND == kLeafFold) {
+    if constexpr (KIND == kLeafQM31 || KIND == kLeafFold || KIND == kLeafFoldQ) {
       uint4 v;
       if constexpr (KIND == kLeafQM31) {
         v = __ldg(job.layer + leaf);
       } else {
-        v = folded_value(job, leaf, ch);
+        v = folded_value<KIND>(job, leaf, ch);
         if (ok && q == 0) job.out_layer[leaf] = v;
       }
       const ulonglong2 w = pack_qm31(v);
@@ -281,7 +280,7 @@ __device__ __forceinline__ uint4 pair_leaf(const TreeJob& job, uint64_t leaf, bo
         if constexpr (KIND == kLeafQM31x4) {
           v = __ldg(job.layer + e);
         } else {
-          v = folded_value(job, e, ch);
+          v = folded_value<KIND>(job, e, ch);
           if (ok) job.out_layer[e] = v;
         }
         const ulonglong2 w = pack_qm31(v);
@@ -418,7 +417,7 @@ __device__ __noinline__ void top_levels(uint64_t* top, uint32_t count, const Tre
     sp.load(job.base ? job.base : job.transcript);
     uint64_t* const node = top + 8 * 4 + 4 * 3;  // the fourth node above eight digests
 #pragma unroll 1
-    for (uint32_t step = job.base ? kPublic : kNode; step <= kChallenge; step++) {
+    for (uint32_t step = job.pub ? kPublic : kNode; step <= kChallenge; step++) {
       uint64_t word = 0, keep = 0;
       if (step == kPublic) {
         word = sp.digest_word(job.pub);
@@ -491,7 +490,7 @@ __device__ __forceinline__ void tree_tile_body(const TreeJob& job, const uint64_
   uint64_t* bufB = sm + 4 * M;
 
   uint32_t ch[4] = {0, 0, 0, 0};
-  if constexpr (KIND == kLeafFold || KIND == kLeafFoldx4) {
+  if constexpr (KIND == kLeafFold || KIND == kLeafFoldx4 || KIND == kLeafFoldQ) {
     if (threadIdx.x < 4) s_ch[threadIdx.x] = __ldcg(job.fold_ch + threadIdx.x);
     __syncthreads();
 #pragma unroll
@@ -611,6 +610,7 @@ cudaError_t prepare_tree_kernels() {
   if (e == cudaSuccess) e = prepare_kind<kLeafDigest>();
   if (e == cudaSuccess) e = prepare_kind<kLeafQM31x4>();
   if (e == cudaSuccess) e = prepare_kind<kLeafFoldx4>();
+  if (e == cudaSuccess) e = prepare_kind<kLeafFoldQ>();
   return e;
 }
 
@@ -662,6 +662,7 @@ cudaError_t launch_tree_jobs(const TreeJob* d_jobs, const uint2* d_work, uint32_
     case kLeafDigest: return launch_kind<kLeafDigest>(d_jobs, d_work, nwork, max_tile_log, threads, d_queue, s);
     case kLeafQM31x4: return launch_kind<kLeafQM31x4>(d_jobs, d_work, nwork, max_tile_log, threads, d_queue, s);
     case kLeafFoldx4: return launch_kind<kLeafFoldx4>(d_jobs, d_work, nwork, max_tile_log, threads, d_queue, s);
+    case kLeafFoldQ: return launch_kind<kLeafFoldQ>(d_jobs, d_work, nwork, max_tile_log, threads, d_queue, s);
     default: return cudaErrorInvalidValue;
   }
 }

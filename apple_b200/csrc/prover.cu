@@ -46,7 +46,7 @@ struct Engine {
   bool any_grinding = false;
 
   Arena arena;
-  std::vector<uint64_t> off_input, off_layers, off_trees, off_tr, off_ch, off_cm, off_qp, off_claim, off_proof, off_cnt;
+  std::vector<uint64_t> off_input, off_layers, off_trees, off_base, off_tr, off_ch, off_cm, off_qp, off_claim, off_proof, off_cnt;
   std::vector<uint64_t> proof_len, proof_off;
   uint64_t proof_total = 0;
   uint64_t off_inst = 0, off_flag = 0, off_info = 0, off_queue = 0;  // off_queue: two words per round (persistent trees)
@@ -255,7 +255,7 @@ struct Engine {
     }
     // ---- memory plan ----
     auto resz = [&](std::vector<uint64_t>& v) { v.assign(n, 0); };
-    for (auto* v : {&off_input, &off_layers, &off_trees, &off_tr, &off_ch, &off_cm, &off_qp, &off_claim, &off_proof, &off_cnt}) resz(*v);
+    for (auto* v : {&off_input, &off_layers, &off_trees, &off_base, &off_tr, &off_ch, &off_cm, &off_qp, &off_claim, &off_proof, &off_cnt}) resz(*v);
     proof_len.assign(n, 0);
     proof_off.assign(n, 0);
     for (size_t i = 0; i < n; i++) {
@@ -264,6 +264,7 @@ struct Engine {
       off_input[i] = arena.reserve(16 * N);
       off_layers[i] = arena.reserve(16 * 2 * N);
       off_trees[i] = arena.reserve(32 * 2 * N);
+      off_base[i] = arena.reserve(sizeof(Transcript));
       off_tr[i] = arena.reserve(sizeof(Transcript));
       off_ch[i] = arena.reserve(16ull * c2.rounds);
       off_cm[i] = arena.reserve(32ull * c2.rounds);
@@ -305,6 +306,7 @@ struct Engine {
       I.trees = arena.at<uint64_t>(off_trees[i]);
       I.tw = dom.tw;
       I.inv = dom.inv;
+      I.base = arena.at<Transcript>(off_base[i]);
       I.transcript = arena.at<Transcript>(off_tr[i]);
       I.challenges = arena.at<uint32_t>(off_ch[i]);
       I.commitments = arena.at<uint64_t>(off_cm[i]);
@@ -316,6 +318,7 @@ struct Engine {
         AZK_CU(cudaMemcpyAsync(arena.at<uint64_t>(off_claim[i]), c2.claimed.data(), 8 * c2.claimed.size(), cudaMemcpyHostToDevice, s));
     }
     AZK_CU(cudaMemcpyAsync(d_inst(), h_inst.data(), sizeof(PcsInstance) * n, cudaMemcpyHostToDevice, s));
+    AZK_CU(launch_pcs_base(d_inst(), (uint32_t)n, s));
     ids.resize(n);
     for (size_t i = 0; i < n; i++) ids[i] = (uint32_t)i;
     d_ids.alloc(4 * n, "PCS.Ids");
@@ -361,6 +364,8 @@ struct Engine {
         j.group_log = std::max<uint32_t>(1, std::min(sched.group_log, tl));
         if (k == 0) {
           j.layer = I.layers;
+          j.base = I.base;
+          j.pub = d_inst()[i].pub;
         } else {
           j.layer = I.layers + layer_offset(c2.logn, k - 1);
           j.inv = I.inv + (k - 1 == 0 ? 0 : (1ull << c2.logn) - ((1ull << c2.logn) >> (k - 1)));
@@ -391,6 +396,7 @@ struct Engine {
         if (c2.rounds != k) continue;
         const PcsInstance& I = h_inst[i];
         uint64_t N = 1ull << c2.logn;
+        if ((N >> k) <= kTailFold) continue;  // folded by the tail kernel
         FoldJob f{N >> k, I.layers + layer_offset(c2.logn, k - 1), I.inv + (k - 1 == 0 ? 0 : N - (N >> (k - 1))), I.challenges + 4 * (k - 1),
                   I.layers + layer_offset(c2.logn, k)};
         uint32_t fid = (uint32_t)fold_jobs.size();
@@ -424,7 +430,7 @@ struct Engine {
       for (auto c3 : st) launches += c3 ? 1 : 0;
     for (auto c3 : tstep_cnt) launches += c3 ? 1 : 0;
     for (auto c3 : fstep_cnt) launches += c3 ? 1 : 0;
-    launches += 4;  // prefix, finalize, queries, emit
+    launches += has_proofs() ? 2 : 1;  // tail and emission (with a nonce search the tail runs in two parts)
     ensure_events(fft.steps() + 2 * rmax + 8);
   }
 
@@ -472,9 +478,6 @@ struct Engine {
         prof_end();
       }
     }
-    prof_begin(3);
-    AZK_CU(launch_pcs_prefix(d_inst(), na, s));
-    prof_end();
     for (uint32_t k = 0; k <= rmax; k++) {
       if (k < rmax) {
         prof_begin(1);
@@ -488,7 +491,7 @@ struct Engine {
       }
     }
     prof_begin(3);
-    AZK_CU(launch_pcs_finalize(d_inst(), d_ids.as<uint32_t>(), na, s));
+    AZK_CU(launch_pcs_tail(d_inst(), d_ids.as<uint32_t>(), na, kTailFoldPart | kTailBind | (has_proofs() && !any_grinding ? kTailQueries : 0u), s));
     prof_end();
   }
   // Proof bytes exist only for 16-byte leaves (the reference's verifier opens one
@@ -497,7 +500,7 @@ struct Engine {
   void enqueue_tail_batched() {
     if (!has_proofs()) return;
     prof_begin(3);
-    AZK_CU(launch_pcs_queries(d_inst(), d_ids.as<uint32_t>(), active(), s));
+    if (any_grinding) AZK_CU(launch_pcs_tail(d_inst(), d_ids.as<uint32_t>(), active(), kTailQueries, s));
     AZK_CU(launch_pcs_emit(d_inst(), d_ids.as<uint32_t>(), active(), qmax, s));
     prof_end();
   }
@@ -505,16 +508,16 @@ struct Engine {
     if (from_coeffs)
       for (size_t st = 0; st < fft.steps(); st++)
         if (fft.inst_range[st][i].second) fft.launch_step_for(st, i, s);
-    AZK_CU(launch_pcs_prefix(d_inst() + i, 1, s));
     const uint32_t* id = d_ids.as<uint32_t>() + i;
     for (uint32_t k = 0; k <= cfg[i].rounds; k++) {
       if (k < cfg[i].rounds) launch_tree_range(k, tstep_inst[k][i].first, tstep_inst[k][i].second, layer_log(i, k));
       if (k == cfg[i].rounds) launch_fold_range(fstep_inst[k][i].first, fstep_inst[k][i].second);
     }
-    AZK_CU(launch_pcs_finalize(d_inst(), id, 1, s));
+    const bool one_tail = has_proofs() && !cfg[i].grinding;
+    AZK_CU(launch_pcs_tail(d_inst(), id, 1, kTailFoldPart | kTailBind | (one_tail ? kTailQueries : 0u), s));
     if (!has_proofs()) return;
     grind_instance(i);
-    AZK_CU(launch_pcs_queries(d_inst(), id, 1, s));
+    if (!one_tail) AZK_CU(launch_pcs_tail(d_inst(), id, 1, kTailQueries, s));
     AZK_CU(launch_pcs_emit(d_inst(), id, 1, cfg[i].queries, s));
   }
 
@@ -837,11 +840,9 @@ azk_status azk_circle_merkle_fold_chain(azk_ctx* ctx, uint32_t logn, const uint3
     e.check_input_canonical(e.h_inst[0].layers, 4 * N);
     e.set_publics(pub);
     GpuTimer g(e.s);
-    AZK_CU(launch_pcs_prefix(e.d_inst(), 1, e.s));
-    for (uint32_t k = 0; k <= rounds; k++) {
-      if (k < rounds) e.launch_tree_range(k, e.tstep_inst[k][0].first, e.tstep_inst[k][0].second, e.layer_log(0, k));
-      if (k == rounds) e.launch_fold_range(e.fstep_inst[k][0].first, e.fstep_inst[k][0].second);
-    }
+    for (uint32_t k = 0; k < rounds; k++) e.launch_tree_range(k, e.tstep_inst[k][0].first, e.tstep_inst[k][0].second, e.layer_log(0, k));
+    e.launch_fold_range(e.fstep_inst[rounds][0].first, e.fstep_inst[rounds][0].second);
+    AZK_CU(launch_pcs_tail(e.d_inst(), e.d_ids.as<uint32_t>(), 1, kTailFoldPart, e.s));
     g.stop();
     double gs = g.seconds();
     e.trace(0, cm_out, ch_out, final_out, nullptr);
