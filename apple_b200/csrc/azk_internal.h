@@ -212,15 +212,43 @@ cudaError_t launch_gather_openings(const TreeJob* d_job, const uint64_t* d_idx, 
 cudaError_t launch_domain_tables(uint32_t logn, uint32_t* d_tw, uint32_t* d_inv, cudaStream_t s);
 cudaError_t launch_domain_points(uint32_t logn, uint32_t* d_xy, cudaStream_t s);
 cudaError_t launch_widen_m31(const uint32_t* d_in, uint4* d_out, uint64_t n, cudaStream_t s);
-// Witness columns -> FFT basis (witness_kernels.cu): factorial tables of n
-// entries (seg: ceil(n/1024) words of scratch), then the transform of two columns
-// of count_x / count_y monomial coefficients into 2n interleaved QM31.
+// Witness columns -> FFT basis (witness_kernels.cu, witness_fft.cu): factorial
+// tables k!, 1/k!, 2^(1-k) k! of n entries (seg: ceil(n/1024) words of scratch).
 cudaError_t launch_witness_tables(uint64_t n, uint32_t* fact, uint32_t* seg, uint32_t* ifact, uint32_t* scale, cudaStream_t s);
-cudaError_t launch_witness_transform(const uint4* x, uint64_t count_x, const uint4* y, uint64_t count_y, uint64_t n, const uint32_t* ifact,
-                                     const uint32_t* scale, uint4* ax, uint4* ay, uint4* px, uint4* py, uint4* cx, uint4* cy, uint4* out,
-                                     cudaStream_t s);
-// QM31 values of each partial-sum buffer (px, py) the transform needs at capacity n.
+// Chebyshev coefficients of two columns by the direct sum: count_x / count_y
+// monomial coefficients to n values each at cx, cy.  ax, ay: n QM31 of scratch each;
+// px, py: witness_partial_values(n) each.
+cudaError_t launch_witness_chebyshev(const uint4* x, uint64_t count_x, const uint4* y, uint64_t count_y, uint64_t n, const uint32_t* ifact,
+                                     const uint32_t* scale, uint4* ax, uint4* ay, uint4* px, uint4* py, uint4* cx, uint4* cy, cudaStream_t s);
+// QM31 values of each partial-sum buffer (px, py) the direct sum needs at n.
 uint64_t witness_partial_values(uint64_t n);
+// The same by fast convolutions of 2^lm = 2n values (witness_fft.cu).
+struct WitnessConv {
+  uint32_t lm, table, flip, pad;
+  const uint4 *x, *y;  // monomial columns
+  uint64_t count_x, count_y;
+  const uint32_t *fact, *ifact;  // 2n entries
+  const uint2* roots;            // n CM31 roots, bit-reversed
+  uint8_t *c, *c2, *c3;          // values between the convolutions (n, n / 2, n / 2 per column)
+  uint64_t c_stride;             // bytes from one column's to the next's
+  void* t;                       // 2n values per column
+  void* u[2];                    // the parity step's two products, likewise
+  uint64_t t_stride;
+  const uint2* k[2];             // transforms of the fixed sequences
+  uint8_t* o[2];                 // a convolution's outputs, o_stride bytes between columns
+  uint64_t o_stride, outputs;
+};
+struct WitnessKernels {
+  const uint2* k[3];  // transforms of 1/j!, 1/(2j)!, 1/(2j-1)!, 2n CM31 values each
+};
+cudaError_t prepare_witness_fft();
+cudaError_t launch_witness_roots(uint2* roots, uint32_t log, cudaStream_t s);
+cudaError_t launch_witness_fft_tables(WitnessConv a, const WitnessKernels& kr, cudaStream_t s);
+// Two columns (lifted: every coefficient an M31) to 2 * capacity interleaved
+// FFT-basis values.
+cudaError_t launch_witness_fft(const WitnessConv& a, const WitnessKernels& kr, bool lifted, uint4* out, uint64_t capacity, cudaStream_t s);
+// The line-basis step alone, from Chebyshev coefficients in a.c (n = 2^(lm - 1) each).
+cudaError_t launch_witness_line(const WitnessConv& a, uint4* out, uint64_t capacity, cudaStream_t s);
 
 // FFT pass kernels.  kFftQM31: four-limb tiles (fft_pass_q_kernel); kFftM31Small:
 // one-limb transforms below 2^12 values, one pass (fft_pass_m31_kernel);

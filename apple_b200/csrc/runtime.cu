@@ -2,6 +2,7 @@
 // Keccak-f batch, SHA3/Keccak batch hashing, raw/prehashed Merkle commitment,
 // Circle FFT codeword, single folds and fold chains.
 #include <algorithm>
+#include <map>
 #include <cstdlib>
 
 #include "azk_field.cuh"
@@ -269,6 +270,7 @@ azk_status azk_ctx_create(int device, azk_ctx** out) {
     AZK_CU(cudaSetDevice(device));
     AZK_CU(prepare_tree_kernels());
     AZK_CU(prepare_fft_kernels());
+    AZK_CU(prepare_witness_fft());
     auto* c = new azk_ctx();
     c->device = device;
     c->sm_count = prop.multiProcessorCount;
@@ -976,36 +978,115 @@ void azk_codeword_plan_destroy(azk_codeword_plan* p) { delete p; }
 }  // extern "C"
 
 // ---- witness columns -> FFT basis (CircleWitnessToFFTBasisPlanV1) ----
+// Work is sized by the columns given: n = the power of two that holds the longer one
+// (at least kWitnessMinLog, or the capacity), not by the capacity.  Columns of at
+// least 2^kWitnessFftLog take the fast convolutions, shorter ones the direct sum.
+// Columns of at least 2^kWitnessFftLog take the fast convolutions, shorter ones the
+// direct sum (two full QM31 columns on B200, direct / convolutions: 2^12 74 / 100 us,
+// 2^13 160 / 111 us, 2^14 425 / 116 us, 2^19 175,900 / 886 us).
+static constexpr uint32_t kWitnessMinLog = 11, kWitnessFftLog = 13;
+
 struct azk_witness_plan {
   azk_ctx* ctx;
   std::mutex mu;
   cudaStream_t s = nullptr;
   uint32_t logn;
   uint64_t n;  // coefficient capacity = half the domain
-  DevBuf fact, seg, ifact, scale, ax, ay, px, py, cx, cy, xin, yin, out, flag;
+  DevBuf tables, flag;
+  uint32_t *fact = nullptr, *ifact = nullptr, *scale = nullptr;  // in `tables`
+  DevBuf xin, yin, out;                  // host columns and result (made on first use)
+  DevBuf work;                           // scratch, sized for the largest call so far
+  DevBuf roots;                          // CM31 roots for convolutions of up to 2 * roots_n values
+  uint64_t roots_n = 0;
+  std::map<uint32_t, DevBuf> sequences;  // by lm: transforms of the three fixed sequences
   ~azk_witness_plan() {
     if (s) cudaStreamDestroy(s);
+  }
+  void host_columns() {
+    if (xin.p) return;
+    out.alloc(32 * n, "Witness.Output");
+    yin.alloc(16 * n, "Witness.Columns");
+    xin.alloc(16 * n, "Witness.Columns");
   }
 };
 
 static void witness_run(azk_witness_plan* p, const uint4* x, uint64_t nx, const uint4* y, uint64_t ny, uint4* out, azk_stats* st, const Timer& t) {
-  // canonicality of both columns (CircleWitnessFFTBasis.swift:374-385)
-  AZK_CU(cudaMemsetAsync(p->flag.p, 0, 4, p->s));
-  if (nx) AZK_CU(launch_check_canonical(reinterpret_cast<const uint32_t*>(x), 4 * nx, p->flag.as<uint32_t>(), p->s));
-  if (ny) AZK_CU(launch_check_canonical(reinterpret_cast<const uint32_t*>(y), 4 * ny, p->flag.as<uint32_t>(), p->s));
-  uint32_t bad = 0;
-  AZK_CU(cudaMemcpyAsync(&bad, p->flag.p, 4, cudaMemcpyDeviceToHost, p->s));
+  // canonicality of both columns (CircleWitnessFFTBasis.swift:374-385), and whether
+  // every coefficient is a lifted M31
+  const uint32_t init[8] = {0, 0, 0, 0, 1, 0, 0, 0};
+  uint32_t* bad = p->flag.as<uint32_t>();
+  InputInfo* info = reinterpret_cast<InputInfo*>(bad + 4);
+  AZK_CU(cudaMemcpyAsync(bad, init, sizeof(init), cudaMemcpyHostToDevice, p->s));
+  if (nx) AZK_CU(launch_scan_input(x, nx, bad, info, p->s));
+  if (ny) AZK_CU(launch_scan_input(y, ny, bad, info, p->s));
+  uint32_t found[8];
+  AZK_CU(cudaMemcpyAsync(found, bad, sizeof(found), cudaMemcpyDeviceToHost, p->s));
   sync_stream(p->s);
-  layout(bad == 0, "witness coefficients contain a non-canonical field element");
+  layout(found[0] == 0, "witness coefficients contain a non-canonical field element");
+  const bool lifted = found[4] != 0;
+
+  uint32_t ln = std::min<uint32_t>(kWitnessMinLog, ilog2(p->n));
+  while ((1ull << ln) < std::max(nx, ny)) ln++;
+  const uint64_t n = 1ull << ln;
+  const bool direct = ln < kWitnessFftLog;
+  // scratch: one allocation, sliced for this call.  Values are QM31 in two columns,
+  // or (convolutions of lifted columns) CM31 in one.
+  const uint64_t col = direct || !lifted ? 16 * n : 8 * n, cols = direct || !lifted ? 2 : 1;
+  const uint64_t partial = direct ? 16 * witness_partial_values(n) : 0;
+  const uint64_t need = direct ? cols * (2 * col + partial) : cols * (col + 3 * 2 * col + col);
+  if (p->work.bytes < need) p->work.alloc(need, "Witness.Work");
+  uint8_t* w = p->work.as<uint8_t>();
+  auto take = [&w](uint64_t bytes) {
+    uint8_t* r = w;
+    w += bytes;
+    return r;
+  };
+  WitnessConv a{};
+  a.lm = ln + 1;
+  a.x = x, a.y = y;
+  a.count_x = nx, a.count_y = ny;
+  a.fact = p->fact, a.ifact = p->ifact;
+  a.c = take(cols * col);
+  a.c_stride = col;
+  if (!direct) {
+    if (p->roots_n < n) {
+      p->roots_n = 0;
+      p->roots.alloc(8 * n, "Witness.Roots");
+      AZK_CU(launch_witness_roots(p->roots.as<uint2>(), ln, p->s));
+      p->roots_n = n;
+    }
+    a.roots = p->roots.as<uint2>();
+    a.t_stride = 2 * col;
+    a.t = take(cols * 2 * col);
+    a.u[0] = take(cols * 2 * col);
+    a.u[1] = take(cols * 2 * col);
+    a.c2 = take(cols * col / 2);
+    a.c3 = take(cols * col / 2);
+  }
   GpuTimer g(p->s);
-  AZK_CU(launch_witness_transform(x, nx, y, ny, p->n, p->ifact.as<uint32_t>(), p->scale.as<uint32_t>(), p->ax.as<uint4>(), p->ay.as<uint4>(),
-                                  p->px.as<uint4>(), p->py.as<uint4>(), p->cx.as<uint4>(), p->cy.as<uint4>(), out, p->s));
+  if (direct) {
+    uint4* c = reinterpret_cast<uint4*>(a.c);
+    uint4 *ax = reinterpret_cast<uint4*>(take(col)), *ay = reinterpret_cast<uint4*>(take(col));
+    uint4 *px = reinterpret_cast<uint4*>(take(partial)), *py = reinterpret_cast<uint4*>(take(partial));
+    AZK_CU(launch_witness_chebyshev(x, nx, y, ny, n, a.ifact, p->scale, ax, ay, px, py, c, c + n, p->s));
+    AZK_CU(launch_witness_line(a, out, p->n, p->s));
+  } else {
+    auto sequences = [n](const DevBuf& b) { return WitnessKernels{{b.as<uint2>(), b.as<uint2>() + 2 * n, b.as<uint2>() + 4 * n}}; };
+    auto seq = p->sequences.find(a.lm);
+    if (seq == p->sequences.end()) {
+      DevBuf b(3 * 16 * n, "Witness.Sequences");
+      AZK_CU(launch_witness_fft_tables(a, sequences(b), p->s));
+      seq = p->sequences.emplace(a.lm, std::move(b)).first;
+    }
+    AZK_CU(launch_witness_fft(a, sequences(seq->second), lifted, out, p->n, p->s));
+  }
   g.stop();
   fill_stats(st, t, 0, g.seconds());
 }
 
 static void witness_columns_to_device(azk_witness_plan* w, const uint32_t* x, uint64_t nx, const uint32_t* y, uint64_t ny, void* dout) {
   std::lock_guard<std::mutex> lk(w->mu);
+  w->host_columns();
   Timer t;
   if (nx) AZK_CU(cudaMemcpyAsync(w->xin.p, x, 16 * nx, cudaMemcpyHostToDevice, w->s));
   if (ny) AZK_CU(cudaMemcpyAsync(w->yin.p, y, 16 * ny, cudaMemcpyHostToDevice, w->s));
@@ -1025,16 +1106,15 @@ azk_status azk_witness_plan_create(azk_ctx* ctx, uint32_t log_size, azk_witness_
     p->n = 1ull << (log_size - 1);
     p->s = new_stream();
     const uint64_t n = p->n;
-    p->fact.alloc(4 * n, "Witness.Factorials");
-    p->seg.alloc(4 * ((n + 1023) / 1024), "Witness.Segments");
-    p->ifact.alloc(4 * n, "Witness.InverseFactorials");
-    p->scale.alloc(4 * n, "Witness.Scale");
-    for (DevBuf* b : {&p->ax, &p->ay, &p->cx, &p->cy, &p->xin, &p->yin}) b->alloc(16 * n, "Witness.Scratch");
-    p->px.alloc(16 * witness_partial_values(n), "Witness.PartialSums");
-    p->py.alloc(16 * witness_partial_values(n), "Witness.PartialSums");
-    p->out.alloc(32 * n, "Witness.Output");
-    p->flag.alloc(16, "Witness.Flag");
-    AZK_CU(launch_witness_tables(n, p->fact.as<uint32_t>(), p->seg.as<uint32_t>(), p->ifact.as<uint32_t>(), p->scale.as<uint32_t>(), p->s));
+    const uint64_t entries = n >> kWitnessFftLog ? 2 * n : n;  // the convolutions need k! for k < 2n
+    const uint64_t slice = align_up(4 * entries, 256);
+    p->tables.alloc(3 * slice + 4 * ((entries + 1023) / 1024), "Witness.Factorials");
+    p->fact = p->tables.as<uint32_t>();
+    p->ifact = p->fact + slice / 4;
+    p->scale = p->ifact + slice / 4;
+    uint32_t* seg = p->scale + slice / 4;
+    p->flag.alloc(32, "Witness.Flag");
+    AZK_CU(launch_witness_tables(entries, p->fact, seg, p->ifact, p->scale, p->s));
     sync_stream(p->s);
     *out = p.release();
   });
@@ -1049,6 +1129,7 @@ azk_status azk_witness_plan_execute(azk_witness_plan* p, const uint32_t* x, uint
     // CircleWitnessFFTBasis.swift:349-353
     layout(nx <= p->n && ny <= p->n && nx + ny > 0);
     std::lock_guard<std::mutex> lk(p->mu);
+    p->host_columns();
     Timer t;
     if (nx) AZK_CU(cudaMemcpyAsync(p->xin.p, x, 16 * nx, cudaMemcpyHostToDevice, p->s));
     if (ny) AZK_CU(cudaMemcpyAsync(p->yin.p, y, 16 * ny, cudaMemcpyHostToDevice, p->s));

@@ -11,10 +11,11 @@
 // so with a_k = x_k * 2^(1-k) * k! the Chebyshev coefficient of T_m is
 //   c_m = sum_j a_(m+2j) / (j! (m+j)!)            (halved for m = 0),
 // computed here from factorial tables without storing any matrix: each term is
-// one M31 product of two table entries and a QM31-by-M31 product.  L is the
-// reference's split recursion (low[i] -= high[half-i]/2 after doubling the high
-// half), run level by level: the pair (i, s-i) of a block of size s becomes
-// (c_i - c_(s-i), 2 c_(s-i)).
+// one M31 product of two table entries and a QM31-by-M31 product.  This file has
+// that direct sum, which serves short columns; long ones take the convolutions of
+// witness_fft.cu, which also has L: the reference's split recursion (low[i] -=
+// high[half-i]/2 after doubling the high half), run level by level: the pair
+// (i, s-i) of a block of size s becomes (c_i - c_(s-i), 2 c_(s-i)).
 #include "azk_field.cuh"
 #include "azk_internal.h"
 
@@ -161,57 +162,6 @@ __global__ void chebyshev_sum_kernel(const uint4* __restrict__ px, const uint4* 
   cy[m] = make_uint4(sy.a, sy.b, sy.c, sy.d);
 }
 
-__device__ __forceinline__ void line_pair(uint4& lo, uint4& hi) {
-  const qm31 l = {lo.x, lo.y, lo.z, lo.w}, h = {hi.x, hi.y, hi.z, hi.w};
-  const qm31 nl = q_sub(l, h), nh = q_add(h, h);
-  lo = make_uint4(nl.a, nl.b, nl.c, nl.d);
-  hi = make_uint4(nh.a, nh.b, nh.c, nh.d);
-}
-
-// One level of the Chebyshev -> line-basis recursion for blocks of size s > 1024:
-// pair (i, s - i), 1 <= i < s/2, of every block.
-__global__ void line_level_kernel(uint4* __restrict__ v, uint64_t n, uint64_t s) {
-  const uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const uint64_t half = s >> 1;
-  const uint64_t per = half - 1;  // pairs per block
-  if (per == 0 || g >= (n / s) * per) return;
-  const uint64_t b = g / per, i = g % per + 1;
-  uint4 lo = v[b * s + i], hi = v[b * s + s - i];
-  line_pair(lo, hi);
-  v[b * s + i] = lo;
-  v[b * s + s - i] = hi;
-}
-
-// The levels s <= 1024 of one 1024-value tile (or the whole vector if shorter) in
-// shared memory, for both columns, then the interleaved output
-// out[2i] = x line basis, out[2i+1] = y line basis.
-static constexpr uint32_t kLineTile = 1024;  // 2 x 16 KiB of static shared memory
-
-__global__ void __launch_bounds__(512) line_tile_kernel(const uint4* __restrict__ cx, const uint4* __restrict__ cy, uint64_t n, uint32_t top,
-                                                         uint4* __restrict__ out) {
-  __shared__ uint4 sx[kLineTile], sy[kLineTile];
-  const uint32_t T = n < kLineTile ? (uint32_t)n : kLineTile;
-  const uint64_t base = (uint64_t)blockIdx.x * T;
-  for (uint32_t t = threadIdx.x; t < T; t += blockDim.x) {
-    sx[t] = cx[base + t];
-    sy[t] = cy[base + t];
-  }
-  __syncthreads();
-  for (uint32_t s = top; s >= 2; s >>= 1) {
-    const uint32_t half = s >> 1, per = half - 1;
-    for (uint32_t g = threadIdx.x; g < (T / s) * per; g += blockDim.x) {
-      const uint32_t b = g / per, i = g % per + 1;
-      line_pair(sx[b * s + i], sx[b * s + s - i]);
-      line_pair(sy[b * s + i], sy[b * s + s - i]);
-    }
-    __syncthreads();
-  }
-  for (uint32_t t = threadIdx.x; t < T; t += blockDim.x) {
-    out[2 * (base + t)] = sx[t];
-    out[2 * (base + t) + 1] = sy[t];
-  }
-}
-
 cudaError_t launch_witness_tables(uint64_t n, uint32_t* fact, uint32_t* seg, uint32_t* ifact, uint32_t* scale, cudaStream_t s) {
   const uint32_t nseg = (uint32_t)((n + 1023) / 1024);
   fact_segments_kernel<<<nseg, 1024, 0, s>>>(fact, seg, n);
@@ -235,12 +185,8 @@ uint64_t witness_partial_values(uint64_t n) {
   return (uint64_t)kWitnessBlockTarget * kChebM + n;
 }
 
-// x, y: count_x / count_y monomial coefficients (QM31); capacity n = half the
-// domain; out: 2n QM31.  ax, ay, cx, cy: n QM31 each of scratch; px, py:
-// witness_partial_values(n) QM31 each.
-cudaError_t launch_witness_transform(const uint4* x, uint64_t count_x, const uint4* y, uint64_t count_y, uint64_t n, const uint32_t* ifact,
-                                     const uint32_t* scale, uint4* ax, uint4* ay, uint4* px, uint4* py, uint4* cx, uint4* cy, uint4* out,
-                                     cudaStream_t s) {
+cudaError_t launch_witness_chebyshev(const uint4* x, uint64_t count_x, const uint4* y, uint64_t count_y, uint64_t n, const uint32_t* ifact,
+                                     const uint32_t* scale, uint4* ax, uint4* ay, uint4* px, uint4* py, uint4* cx, uint4* cy, cudaStream_t s) {
   const uint64_t count = count_x > count_y ? count_x : count_y;
   witness_scale_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(x, count_x, scale, ax, n);
   witness_scale_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(y, count_y, scale, ay, n);
@@ -249,13 +195,6 @@ cudaError_t launch_witness_transform(const uint4* x, uint64_t count_x, const uin
   const uint64_t per_slice = (chunks + slices - 1) / slices;
   chebyshev_kernel<<<dim3((unsigned)((n + kChebM - 1) / kChebM), slices), kChebM, 0, s>>>(ax, ay, count, ifact, px, py, n, per_slice ? per_slice : 1);
   chebyshev_sum_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(px, py, slices, cx, cy, n);
-  for (uint64_t sz = n; sz > kLineTile; sz >>= 1) {
-    const uint64_t pairs = (n / sz) * ((sz >> 1) - 1);
-    line_level_kernel<<<(unsigned)((pairs + 255) / 256), 256, 0, s>>>(cx, n, sz);
-    line_level_kernel<<<(unsigned)((pairs + 255) / 256), 256, 0, s>>>(cy, n, sz);
-  }
-  const uint32_t T = n < kLineTile ? (uint32_t)n : kLineTile;
-  line_tile_kernel<<<(unsigned)(n / T), 512, 0, s>>>(cx, cy, n, T, out);
   return cudaGetLastError();
 }
 
