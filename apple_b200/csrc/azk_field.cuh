@@ -68,36 +68,50 @@ __host__ __device__ __forceinline__ qm31 q_sub(qm31 x, qm31 y) { return {m31_sub
 __host__ __device__ __forceinline__ qm31 q_mul_m31(qm31 x, uint32_t s) { return {m31_mul(x.a, s), m31_mul(x.b, s), m31_mul(x.c, s), m31_mul(x.d, s)}; }
 __host__ __device__ __forceinline__ qm31 q_half(qm31 x) { return {m31_half(x.a), m31_half(x.b), m31_half(x.c), m31_half(x.d)}; }
 
-// CM31 product (re, im) = (ac - bd, ad + bc), each term reduced as in the reference.
-__host__ __device__ __forceinline__ void cm_mul(uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t& re, uint32_t& im) {
-  re = m31_sub(m31_mul(a, c), m31_mul(b, d));
-  im = m31_add(m31_mul(a, d), m31_mul(b, c));
+// v < 2^64 -> v mod p, canonical: the three 31-bit parts, the upper two (at most
+// p + 3 together) reduced before the third is added.
+__host__ __device__ __forceinline__ uint32_t m31_reduce64(uint64_t v) {
+  const uint32_t t = m31_reduce_once(((uint32_t)(v >> 31) & kP) + (uint32_t)(v >> 62));
+  return m31_reduce_once(((uint32_t)v & kP) + t);
 }
-// QM31 product: (x0 + x1 u)(y0 + y1 u) = x0 y0 + (2+i) x1 y1 + (x0 y1 + x1 y0) u
-__host__ __device__ __forceinline__ qm31 q_mul(qm31 x, qm31 y) {
-  uint32_t acr, aci, bdr, bdi, adr, adi, bcr, bci;
-  cm_mul(x.a, x.b, y.a, y.b, acr, aci);
-  cm_mul(x.c, x.d, y.c, y.d, bdr, bdi);
-  cm_mul(x.a, x.b, y.c, y.d, adr, adi);
-  cm_mul(x.c, x.d, y.a, y.b, bcr, bci);
-  // (2 + i)(r + i s) = (2r - s) + i(2s + r); field arithmetic is exact, so adds
-  // stand in for the reference's multiplications by 2 and 1 with equal results.
-  uint32_t nr = m31_sub(m31_add(bdr, bdr), bdi);
-  uint32_t ni = m31_add(m31_add(bdi, bdi), bdr);
-  return {m31_add(acr, nr), m31_add(aci, ni), m31_add(adr, bcr), m31_add(adi, bci)};
+// QM31 product (x0 + x1 u)(y0 + y1 u) = x0 y0 + (2+i) x1 y1 + (x0 y1 + x1 y0) u, with
+// u^2 = 2 + i and (2 + i)(r + i s) = (2r - s) + i(2s + r): each limb of the result is
+// four products of x's limbs by values made from y once.  Four products of values
+// <= p are below 2^64, so a limb is reduced once; reducing each product by itself
+// took about twice the instructions (QM31 folds are bound by integer issue).
+struct qm31_factor {
+  uint32_t a, b, nb, c, d, nd, e, f, nf;  // b, -b, d, -d, e = 2c - d, f = 2d + c
+};
+__host__ __device__ __forceinline__ qm31_factor q_factor(qm31 y) {
+  qm31_factor k;
+  k.a = y.a, k.b = y.b, k.nb = kP - y.b, k.c = y.c, k.d = y.d, k.nd = kP - y.d;
+  k.e = m31_sub(m31_add(y.c, y.c), y.d);
+  k.f = m31_add(m31_add(y.d, y.d), y.c);
+  k.nf = kP - k.f;
+  return k;
 }
+// z + x y for limbs of z at most 2p (unreduced sums of two values): z + four products
+// stays below 2^64.
+__host__ __device__ __forceinline__ qm31 q_mul_add(qm31 x, const qm31_factor& k, qm31 z) {
+  auto dot = [&](uint32_t p, uint32_t q, uint32_t r, uint32_t s, uint32_t add) {
+    return m31_reduce64((uint64_t)x.a * p + add + (uint64_t)x.b * q + (uint64_t)x.c * r + (uint64_t)x.d * s);
+  };
+  return {dot(k.a, k.nb, k.e, k.nf, z.a), dot(k.b, k.a, k.f, k.e, z.b), dot(k.c, k.nd, k.a, k.nb, z.c), dot(k.d, k.c, k.b, k.a, z.d)};
+}
+__host__ __device__ __forceinline__ qm31 q_mul(qm31 x, const qm31_factor& k) { return q_mul_add(x, k, qm31{0, 0, 0, 0}); }
+__host__ __device__ __forceinline__ qm31 q_mul(qm31 x, qm31 y) { return q_mul(x, q_factor(y)); }
 
 // One FRI fold of the pair (pos, neg) with inverse-domain value t (an M31) and
 // challenge ch: ((pos + neg) + ch * ((pos - neg) * t)) / 2  (QM31FRIFold.swift:30-41).
 __host__ __device__ __forceinline__ qm31 fri_fold_pair(qm31 pos, qm31 neg, uint32_t t, qm31 ch) {
   qm31 even = q_add(pos, neg);
   qm31 odd = q_mul_m31(q_sub(pos, neg), t);
-  return q_half(q_add(even, q_mul(ch, odd)));
+  return q_half(q_add(even, q_mul(odd, ch)));
 }
 
 // The same with a QM31 inverse-domain value.
 __host__ __device__ __forceinline__ qm31 fri_fold_pair_q(qm31 pos, qm31 neg, qm31 t, qm31 ch) {
-  return q_half(q_add(q_add(pos, neg), q_mul(ch, q_mul(q_sub(pos, neg), t))));
+  return q_half(q_add(q_add(pos, neg), q_mul(q_mul(q_sub(pos, neg), t), ch)));
 }
 
 // ---- circle group over M31 (CircleDomain.swift:3-101) ----

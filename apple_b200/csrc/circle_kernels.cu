@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(256) fold_qm31_inv_kernel(const uint4* __restr
   __shared__ uint32_t s_ch[4];
   if (threadIdx.x < 4) s_ch[threadIdx.x] = __ldcg(chp + threadIdx.x);
   __syncthreads();
-  const qm31 ch = {s_ch[0], s_ch[1], s_ch[2], s_ch[3]};
+  const qm31_factor ch = q_factor(qm31{s_ch[0], s_ch[1], s_ch[2], s_ch[3]});
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_out; i += 2 * stride) {
     const uint64_t i2 = i + stride;
@@ -530,13 +530,13 @@ __global__ void __launch_bounds__(256) fold_qm31_inv_kernel(const uint4* __restr
     {
       qm31 pos = {p.x, p.y, p.z, p.w}, neg = {q.x, q.y, q.z, q.w};
       qm31 odd = q_mul(q_sub(pos, neg), qm31{t.x, t.y, t.z, t.w});
-      qm31 r = q_half(q_add(q_add(pos, neg), q_mul(ch, odd)));
+      qm31 r = q_half(q_add(q_add(pos, neg), q_mul(odd, ch)));
       out[i] = make_uint4(r.a, r.b, r.c, r.d);
     }
     if (two) {
       qm31 pos = {p2.x, p2.y, p2.z, p2.w}, neg = {q2.x, q2.y, q2.z, q2.w};
       qm31 odd = q_mul(q_sub(pos, neg), qm31{t2.x, t2.y, t2.z, t2.w});
-      qm31 r = q_half(q_add(q_add(pos, neg), q_mul(ch, odd)));
+      qm31 r = q_half(q_add(q_add(pos, neg), q_mul(odd, ch)));
       out[i2] = make_uint4(r.a, r.b, r.c, r.d);
     }
   }
@@ -547,6 +547,123 @@ cudaError_t launch_fold_qm31_inv(const uint4* prev, const uint4* inv, const uint
   uint64_t blocks = (n_out + 511) / 512;
   if (blocks > 148 * 16) blocks = 148 * 16;
   fold_qm31_inv_kernel<<<(unsigned)blocks, 256, 0, s>>>(prev, inv, ch, out, n_out);
+  return cudaGetLastError();
+}
+
+// Several folds with known challenges in one launch: a CTA takes a tile of kFoldTile
+// consecutive values through `rounds` rounds (at most kFoldTileRounds), the layers
+// between them in shared memory.  Round r's inverse-domain layer follows round
+// r - 1's in `inv`, QM31 values or (a canonical domain's) M31 words.  The halvings of
+// all rounds are one factor 2^-rounds on the outputs.  The first rounds are bound by
+// integer issue (about 85 instructions per fold), the last by latency.  A launch per
+// round with 16-byte inverses read and wrote every layer and left all but the first
+// few rounds to launch latency: 16 rounds of 2^22 values took 120 us, 49 us so; 10
+// rounds of 2^16 45 and 15 us.
+template <bool Q>
+struct FoldInv {
+  using type = uint32_t;
+};
+template <>
+struct FoldInv<true> {
+  using type = uint4;
+};
+// pos + neg + ch t (pos - neg); the sum of the two enters the product's accumulators.
+__device__ __forceinline__ qm31 fold_unscaled(uint4 p, uint4 q, uint32_t t, const qm31_factor& ch) {
+  const qm31 d = q_sub(qm31{p.x, p.y, p.z, p.w}, qm31{q.x, q.y, q.z, q.w});
+  const uint32_t t2 = t << 1;
+  const qm31 odd = {m31_mul_dbl(d.a, t2), m31_mul_dbl(d.b, t2), m31_mul_dbl(d.c, t2), m31_mul_dbl(d.d, t2)};
+  return q_mul_add(odd, ch, qm31{p.x + q.x, p.y + q.y, p.z + q.z, p.w + q.w});
+}
+__device__ __forceinline__ qm31 fold_unscaled(uint4 p, uint4 q, uint4 t, const qm31_factor& ch) {
+  const qm31 d = q_sub(qm31{p.x, p.y, p.z, p.w}, qm31{q.x, q.y, q.z, q.w});
+  return q_mul_add(q_mul(d, qm31{t.x, t.y, t.z, t.w}), ch, qm31{p.x + q.x, p.y + q.y, p.z + q.z, p.w + q.w});
+}
+template <bool Q>
+__global__ void __launch_bounds__(256, 4) fold_chain_kernel(const uint4* __restrict__ prev, uint64_t n_in, const void* __restrict__ inv_words,
+                                                         const uint32_t* __restrict__ chp, uint32_t rounds, uint4* __restrict__ out) {
+  using Inv = typename FoldInv<Q>::type;
+  const Inv* inv = static_cast<const Inv*>(inv_words);
+  __shared__ uint4 buf[kFoldTile / 2 + kFoldTile / 4];
+  __shared__ Inv s_inv[kFoldTile / 2];  // the tile's inverses of rounds 1, 2, ...: round r's at kFoldTile / 2 - (kFoldTile >> r)
+  __shared__ uint32_t s_ch[4 * kFoldTileRounds];
+  const uint64_t base = (uint64_t)blockIdx.x * kFoldTile;
+  uint32_t cnt = (uint32_t)(n_in - base < kFoldTile ? n_in - base : kFoldTile) >> 1;
+  if (threadIdx.x < 4 * rounds) s_ch[threadIdx.x] = __ldcg(chp + threadIdx.x);
+  uint64_t layer = n_in >> 1, n = n_in >> 1;  // first entry of round r's inverse layer, its input count
+  for (uint32_t r = 1; r < rounds; r++) {
+    for (uint32_t j = threadIdx.x; j < (cnt >> r); j += 256) s_inv[kFoldTile / 2 - (kFoldTile >> r) + j] = __ldg(inv + layer + (base >> (r + 1)) + j);
+    layer += n >> 1;
+    n >>= 1;
+  }
+  __syncthreads();
+  const uint32_t scale = 1u << ((31 - rounds) % 31);  // 2^-rounds
+  {
+    const qm31_factor ch = q_factor(qm31{s_ch[0], s_ch[1], s_ch[2], s_ch[3]});
+#pragma unroll 2
+    for (uint32_t j = threadIdx.x; j < cnt; j += 256) {
+      qm31 v = fold_unscaled(__ldg(prev + base + 2 * j), __ldg(prev + base + 2 * j + 1), __ldg(inv + base / 2 + j), ch);
+      if (rounds == 1) v = q_mul_m31(v, scale);
+      const uint4 w = make_uint4(v.a, v.b, v.c, v.d);
+      if (rounds == 1)
+        out[base / 2 + j] = w;
+      else
+        buf[j] = w;
+    }
+  }
+  uint4* src = buf;
+  uint4* dst = buf + kFoldTile / 2;
+  for (uint32_t r = 1; r < rounds; r++) {
+    // the first warp made the last 32 values and goes on alone
+    if (cnt > 32) {
+      __syncthreads();
+    } else {
+      if (threadIdx.x >= 32) return;
+      __syncwarp();
+    }
+    cnt >>= 1;
+    const qm31_factor ch = q_factor(qm31{s_ch[4 * r], s_ch[4 * r + 1], s_ch[4 * r + 2], s_ch[4 * r + 3]});
+    for (uint32_t j = threadIdx.x; j < cnt; j += 256) {
+      qm31 v = fold_unscaled(src[2 * j], src[2 * j + 1], s_inv[kFoldTile / 2 - (kFoldTile >> r) + j], ch);
+      if (r + 1 == rounds) v = q_mul_m31(v, scale);
+      const uint4 w = make_uint4(v.a, v.b, v.c, v.d);
+      if (r + 1 == rounds)
+        out[(base >> (r + 1)) + j] = w;
+      else
+        dst[j] = w;
+    }
+    uint4* const next = src;
+    src = dst;
+    dst = next;
+  }
+}
+
+// All `rounds` folds of n values: kFoldTileRounds a launch, the values between two
+// launches in `scratch` (n >> kFoldTileRounds of them).  `m31_inv`: inverse layers of
+// M31 words, else `inv` of QM31 values.  ch: 4 limbs per round on the device.
+// A long input is bound by its first rounds, and a CTA's last rounds are a chain with
+// a few threads busy: from kFoldLong values on a launch stops after kFoldLongRounds
+// (2^22 values, 16 rounds: 11 + 5 rounds 52 us, 5 + 11 rounds 47 us).
+static constexpr uint64_t kFoldLong = 1ull << 19;
+static constexpr uint32_t kFoldLongRounds = 5;
+cudaError_t launch_fold_chain(const uint4* prev, uint64_t n, const uint4* inv, const uint32_t* m31_inv, const uint32_t* ch, uint32_t rounds, uint4* scratch,
+                              uint4* out, cudaStream_t s) {
+  for (uint32_t done = 0; done < rounds;) {
+    const uint32_t most = n >= kFoldLong ? kFoldLongRounds : kFoldTileRounds;
+    const uint32_t r = rounds - done < most ? rounds - done : most;
+    uint4* o = done + r == rounds ? out : scratch;
+    const unsigned blocks = (unsigned)((n + kFoldTile - 1) / kFoldTile);
+    if (m31_inv)
+      fold_chain_kernel<false><<<blocks, 256, 0, s>>>(prev, n, m31_inv, ch + 4 * done, r, o);
+    else
+      fold_chain_kernel<true><<<blocks, 256, 0, s>>>(prev, n, inv, ch + 4 * done, r, o);
+    const uint64_t layers = n - (n >> r);
+    if (m31_inv) m31_inv += layers;
+    inv += layers;
+    n >>= r;
+    prev = scratch;
+    scratch += n;
+    done += r;
+  }
   return cudaGetLastError();
 }
 

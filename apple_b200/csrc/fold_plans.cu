@@ -45,6 +45,7 @@ struct azk_qm31_fold_plan {
   cudaStream_t s = nullptr;
   uint64_t n_in = 0, n_out = 0;
   DevBuf ev, inv, out, ch;
+  const uint32_t* m31_inv = nullptr;  // a canonical domain's inverse layer (the context's table): used instead of QM31 values
   ~azk_qm31_fold_plan() {
     if (s) cudaStreamDestroy(s);
   }
@@ -53,7 +54,10 @@ struct azk_qm31_fold_plan {
 static double qm31_fold_run(azk_qm31_fold_plan* p, const uint4* ev, const uint4* inv, uint4* out, const uint32_t ch[4]) {
   AZK_CU(cudaMemcpyAsync(p->ch.p, ch, 16, cudaMemcpyHostToDevice, p->s));
   GpuTimer g(p->s);
-  AZK_CU(launch_fold_qm31_inv(ev, inv, p->ch.as<uint32_t>(), out, p->n_out, p->s));
+  if (p->m31_inv)
+    AZK_CU(launch_fold_chain(ev, p->n_in, inv, p->m31_inv, p->ch.as<uint32_t>(), 1, nullptr, out, p->s));
+  else
+    AZK_CU(launch_fold_qm31_inv(ev, inv, p->ch.as<uint32_t>(), out, p->n_out, p->s));
   g.stop();
   return g.seconds();
 }
@@ -167,6 +171,9 @@ struct azk_fold_chain_plan {
   // PCS instance fields in `pcs` (log size, security parameters, public digest)
   uint32_t root_kind = kRootQM31Round;
   DevBuf pcs;
+  // a canonical domain's inverse layers (the context's table, laid out as the QM31
+  // layers are): the Circle plans fold with these words instead of 16-byte values
+  const uint32_t* m31_inv = nullptr;
   ~azk_fold_chain_plan() {
     if (s) cudaStreamDestroy(s);
   }
@@ -176,20 +183,10 @@ struct azk_fold_chain_plan {
 
 namespace {
 
-// Round r's fold from `prev` into `next` with challenge r (device limbs).
-void chain_fold(azk_fold_chain_plan* p, uint32_t r, const uint4* prev, const uint4* inv, uint4* next) {
-  AZK_CU(launch_fold_qm31_inv(prev, inv + p->inv_off[r], p->ch.as<uint32_t>() + 4 * r, next, p->count[r] / 2, p->s));
-}
-
-// Explicit or transcript mode (challenges already in p->ch): folds through the
-// plan's layer scratch into `out`.
+// Explicit or transcript mode (challenges already in p->ch): all folds into `out`,
+// the values between launches in the plan's layer scratch.
 void chain_fold_all(azk_fold_chain_plan* p, const uint4* ev, const uint4* inv, uint4* out) {
-  const uint4* prev = ev;
-  for (uint32_t r = 0; r < p->rounds; r++) {
-    uint4* next = r + 1 == p->rounds ? out : p->layer_at(p->layers.as<uint4>(), r + 1);
-    chain_fold(p, r, prev, inv, next);
-    prev = next;
-  }
+  AZK_CU(launch_fold_chain(ev, p->n_in, inv, p->m31_inv, p->ch.as<uint32_t>(), p->rounds, p->layers.as<uint4>(), out, p->s));
 }
 
 // Merkle-bound chain.  Layer r (r >= 1) is written into `log` at offset[r]; layer
@@ -207,7 +204,7 @@ void chain_merkle(azk_fold_chain_plan* p, const uint4* ev, const uint4* inv, uin
       j.layer = cur;
     } else {
       j.layer = r == 1 ? cur : p->layer_at(log, r - 1);
-      j.inv = reinterpret_cast<const uint32_t*>(inv + p->inv_off[r - 1]);
+      j.inv = p->m31_inv ? p->m31_inv + p->inv_off[r - 1] : reinterpret_cast<const uint32_t*>(inv + p->inv_off[r - 1]);
       j.out_layer = p->layer_at(log, r);
     }
   }
@@ -226,7 +223,8 @@ void chain_merkle(azk_fold_chain_plan* p, const uint4* ev, const uint4* inv, uin
     }
   }
   const uint32_t last = p->rounds - 1;
-  chain_fold(p, last, last == 0 ? cur : p->layer_at(log, last), inv, out);
+  AZK_CU(launch_fold_chain(last == 0 ? cur : p->layer_at(log, last), p->count[last], inv + p->inv_off[last], p->m31_inv ? p->m31_inv + p->inv_off[last] : nullptr,
+                           p->ch.as<uint32_t>() + 4 * last, 1, nullptr, out, p->s));
 }
 
 const uint4* dev_q(const void* b, uint64_t off) { return reinterpret_cast<const uint4*>(static_cast<const uint8_t*>(b) + off); }
@@ -870,6 +868,7 @@ azk_status azk_circle_fold_plan_create(azk_ctx* ctx, uint32_t log_size, azk_circ
     p->ctx = ctx;
     forward(ctx, azk_domain_plan_create(ctx, log_size, 0, 0, 1, &p->dom));
     forward(ctx, azk_qm31_fold_plan_create(ctx, 1ull << log_size, &p->fold));
+    p->fold->m31_inv = domain_tables(ctx, log_size).inv;
     *out = p.release();
   });
 }
@@ -927,6 +926,7 @@ azk_status azk_circle_fold_chain_plan_create(azk_ctx* ctx, uint32_t log_size, ui
     p->ctx = ctx;
     forward(ctx, azk_domain_plan_create(ctx, log_size, 0, 0, rounds, &p->dom));
     forward(ctx, azk_fold_chain_plan_create(ctx, 1ull << log_size, rounds, &p->chain));
+    p->chain->m31_inv = domain_tables(ctx, log_size).inv;
     *out = p.release();
   });
 }
@@ -1005,7 +1005,11 @@ azk_status azk_circle_merkle_chain_plan_create(azk_ctx* ctx, uint32_t log_size, 
     AZK_CU(launch_pcs_base(c->pcs.as<PcsInstance>(), 1, c->s));
     sync_stream(c->s);
     c->root_kind = kRootCircleRound;
-    for (auto& j : c->tree_jobs) j.root_action = kRootCircleRound;
+    c->m31_inv = domain_tables(ctx, log_size).inv;
+    for (auto& j : c->tree_jobs) {
+      j.root_action = kRootCircleRound;
+      if (j.kind == kLeafFoldQ) j.kind = kLeafFold;
+    }
     c->tree_jobs[0].pub = c->pcs.as<PcsInstance>()->pub;
     *out = p.release();
   });
