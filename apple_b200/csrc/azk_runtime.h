@@ -30,6 +30,13 @@ struct azk_ctx {
     uint32_t* inv = nullptr;
   };
   std::map<uint32_t, Domain> domains;
+  // Scratch of azk_sumcheck_prove for tables of at most 2^kSumcheckKeptLog words (12.6
+  // MB on the device, 4.2 MB page-locked), used under `mu`, freed with the context;
+  // larger tables take their own for the call.
+  static constexpr uint32_t kSumcheckKeptLog = 20;
+  void* sumcheck_dev = nullptr;
+  void* sumcheck_pin = nullptr;
+  uint64_t sumcheck_dev_bytes = 0, sumcheck_pin_bytes = 0;
 };
 
 namespace azk {
@@ -154,19 +161,30 @@ struct Timer {
   uint64_t ns() const { return (uint64_t)std::chrono::duration_cast<std::chrono::nanoseconds>(std::chrono::steady_clock::now() - t0).count(); }
 };
 
-// Wait for an event by polling it: a short spin, then sleeps growing from 20 to
-// 160 us, so a waiting thread takes little of a host core (the server's workers
-// share the host's cores with each other and with the threads that submit work).
+// Threads that share the host's cores with many others (the server's workers and
+// lane threads) set this for themselves; their waits then sleep early.
+inline thread_local bool t_shared_host = false;
+
+// Wait for an event by polling it.  A caller's own thread spins for up to 5 ms, as
+// CUDA's own synchronisation does (a sleep of 20 us lasts about 75 with the kernel's
+// timer slack: 25 to 100 us on calls whose device time is 30 to 250), and sleeps
+// between polls after that.  A server thread spins for a few polls, then sleeps
+// growing from 20 to 160 us, so a waiting thread takes little of a host core.
 // Not cudaEventSynchronize on a blocking-sync event, which sleeps until the
 // driver's completion interrupt: with the server's 32 workers waiting that way at
 // once, the device stopped starting work for 40-80 ms about every 2 s.
 inline void wait_event(cudaEvent_t e) {
+  const auto t0 = std::chrono::steady_clock::now();
   for (int k = 0;; k++) {
     const cudaError_t q = cudaEventQuery(e);
     if (q == cudaSuccess) return;
     if (q != cudaErrorNotReady) AZK_CU(q);
-    if (k < 8) continue;
-    std::this_thread::sleep_for(std::chrono::microseconds(k < 24 ? 20 : k < 48 ? 50 : 160));
+    if (t_shared_host) {
+      if (k < 8) continue;
+      std::this_thread::sleep_for(std::chrono::microseconds(k < 24 ? 20 : k < 48 ? 50 : 160));
+    } else if (std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(5)) {
+      std::this_thread::sleep_for(std::chrono::microseconds(20));
+    }
   }
 }
 
@@ -192,18 +210,75 @@ inline void sync_stream(cudaStream_t s) {
   wait_event(ev.e);
 }
 
-// CUDA events around a region of one stream.
+// A thread's timing events on its current device, kept from one timed region to the
+// next (creating and destroying a pair costs about as much as two launches); nested
+// regions take further pairs.  At most eight pairs, destroyed with the thread.
+struct TimingEvents {
+  struct Pair {
+    cudaEvent_t a = nullptr, b = nullptr;
+    int dev = -1;
+    bool busy = false;
+  };
+  Pair pair[8];
+  ~TimingEvents() {
+    for (auto& p : pair) {
+      if (p.a) cudaEventDestroy(p.a);
+      if (p.b) cudaEventDestroy(p.b);
+    }
+  }
+  static TimingEvents& mine() {
+    thread_local TimingEvents t;
+    return t;
+  }
+  // A free pair of the current device (an unused slot is filled), or null.
+  Pair* take() {
+    int dev = 0;
+    AZK_CU(cudaGetDevice(&dev));
+    Pair* empty = nullptr;
+    for (auto& p : pair) {
+      if (p.busy) continue;
+      if (p.a && p.b && p.dev == dev) {
+        p.busy = true;
+        return &p;
+      }
+      if (!p.a && !empty) empty = &p;
+    }
+    if (!empty) return nullptr;
+    cudaEvent_t a = nullptr, b = nullptr;
+    AZK_CU(cudaEventCreate(&a));
+    const cudaError_t e = cudaEventCreate(&b);
+    if (e != cudaSuccess) cudaEventDestroy(a);
+    AZK_CU(e);
+    empty->a = a;
+    empty->b = b;
+    empty->dev = dev;
+    empty->busy = true;
+    return empty;
+  }
+};
+
+// CUDA events around a region of one stream; used and destroyed by one thread.
 struct GpuTimer {
   cudaEvent_t a = nullptr, b = nullptr;
   cudaStream_t s;
-  bool owns = true;
+  TimingEvents::Pair* kept = nullptr;
+  bool owns = false;
   explicit GpuTimer(cudaStream_t st) : s(st) {
-    AZK_CU(cudaEventCreate(&a));
-    AZK_CU(cudaEventCreate(&b));
+    kept = TimingEvents::mine().take();
+    if (kept) {
+      a = kept->a;
+      b = kept->b;
+    } else {
+      owns = true;
+      AZK_CU(cudaEventCreate(&a));
+      AZK_CU(cudaEventCreate(&b));
+    }
     AZK_CU(cudaEventRecord(a, s));
   }
-  // With events the caller keeps (nothing created or destroyed per region).
-  GpuTimer(cudaStream_t st, cudaEvent_t ea, cudaEvent_t eb) : a(ea), b(eb), s(st), owns(false) { AZK_CU(cudaEventRecord(a, s)); }
+  // With events the caller keeps.
+  GpuTimer(cudaStream_t st, cudaEvent_t ea, cudaEvent_t eb) : a(ea), b(eb), s(st) { AZK_CU(cudaEventRecord(a, s)); }
+  GpuTimer(const GpuTimer&) = delete;
+  GpuTimer& operator=(const GpuTimer&) = delete;
   void stop() { AZK_CU(cudaEventRecord(b, s)); }
   double seconds() {
     float ms = 0;
@@ -212,6 +287,7 @@ struct GpuTimer {
     return ms / 1000.0;
   }
   ~GpuTimer() {
+    if (kept) kept->busy = false;
     if (!owns) return;
     if (a) cudaEventDestroy(a);
     if (b) cudaEventDestroy(b);
@@ -314,10 +390,11 @@ struct FftPlan {
   void launch_all(cudaStream_t s) const {
     for (size_t k = 0; k < steps(); k++) launch_step(k, s);
   }
-  // After the stream has finished the passes: fails with AZK_ERR_DEVICE_TIMEOUT (and
-  // clears the flag) when a pass kernel gave up waiting for its tile copies.
-  // `host_word`: page-locked memory for the readback (else a pageable word).
-  void check_status(cudaStream_t s, uint32_t* host_word = nullptr);
+  // Queue the readback of the status word into `host_word` (page-locked), and, once
+  // the stream has finished, fail with AZK_ERR_DEVICE_TIMEOUT (clearing the flag) when
+  // a pass kernel gave up waiting for its tile copies.
+  void queue_status(cudaStream_t s, uint32_t* host_word) const;
+  void check_status(cudaStream_t s, const uint32_t* host_word) const;
 };
 
 // Monomial -> interleaved circle FFT-basis coefficients, host-side like the

@@ -14,6 +14,7 @@
 #include <condition_variable>
 #include <deque>
 #include <set>
+#include <system_error>
 #include <thread>
 #include <tuple>
 #include <unordered_map>
@@ -56,7 +57,6 @@ struct Engine {
   uint32_t leaf_values = 1;  // all instances of an engine share the leaf size
   FftPlan fft;
   std::vector<FftJob> fft_transforms;
-  DevBuf d_scan;  // upload scan jobs, one per instance
   std::vector<uint8_t> fft_narrow;  // per instance: input known to be a lifted M31 polynomial
   // rounds: tree step k (kind QM31 at k == 0, fold+hash after), final folds at step k
   std::vector<TreeJob> tree_jobs;
@@ -87,15 +87,17 @@ struct Engine {
 
   // Kept for the engine's lifetime, so a run creates and destroys nothing: the
   // run's timing events, and page-locked words for the input scan's readbacks
-  // (two status words at 0 and 16, then the per-instance input descriptions and
-  // the scan's job list).
+  // (four status words 16 bytes apart, then a copy of the device's scan block: the
+  // flag, the per-instance input descriptions and the scan's job list).
   cudaEvent_t tm_a = nullptr, tm_b = nullptr;
   HostPinned hsmall;
   uint32_t* hword(int k) const { return reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(hsmall.p) + 16 * k); }
-  InputInfo* hinfo() const { return reinterpret_cast<InputInfo*>(static_cast<uint8_t*>(hsmall.p) + 64); }
-  ScanJob* hscan() const {
-    return reinterpret_cast<ScanJob*>(static_cast<uint8_t*>(hsmall.p) + 64 + align_up(sizeof(InputInfo) * cfg.size(), 16));
-  }
+  // The scan block, on the device (at off_flag) and in hsmall: the flag at 0, the
+  // input descriptions, the scan jobs -- one copy in and one out.
+  uint64_t scan_info_at() const { return 16; }
+  uint64_t scan_jobs_at() const { return 16 + align_up(sizeof(InputInfo) * cfg.size(), 16); }
+  uint64_t scan_bytes() const { return scan_jobs_at() + sizeof(ScanJob) * cfg.size(); }
+  uint8_t* hblock() const { return static_cast<uint8_t*>(hsmall.p) + 64; }
 
   // Per-stage CUDA events (profiling): stage kind 0 = FFT, 1 = tree (fold +
   // hash + transcript), 2 = final fold, 3 = transcript/queries/emission.
@@ -161,23 +163,21 @@ struct Engine {
   // of its engine's instances).
   void scan_inputs(const std::vector<uint64_t>& counts) {
     const size_t m = counts.size();
-    InputInfo* h = hinfo();
-    ScanJob* jobs = hscan();
-    uint32_t* f = hword(0);
-    for (size_t i = 0; i < m; i++) h[i] = InputInfo{1u, 0u, counts[i]};
-    AZK_CU(cudaMemcpyAsync(d_info(), h, sizeof(InputInfo) * m, cudaMemcpyHostToDevice, s_up));
-    AZK_CU(cudaMemsetAsync(d_flag(), 0, 4, s_up));
+    uint32_t* f = reinterpret_cast<uint32_t*>(hblock());
+    InputInfo* h = reinterpret_cast<InputInfo*>(hblock() + scan_info_at());
+    ScanJob* jobs = reinterpret_cast<ScanJob*>(hblock() + scan_jobs_at());
+    *f = 0;
     uint64_t max_n = 0;
     for (size_t i = 0; i < m; i++) {
       const uint64_t N = 1ull << cfg[i].logn;
+      h[i] = InputInfo{1u, 0u, counts[i]};
       jobs[i] = ScanJob{arena.at<uint4>(off_input[i]), counts[i], N, d_info() + i};
       max_n = std::max(max_n, N);
     }
-    if (!d_scan.p) d_scan.alloc(sizeof(ScanJob) * cfg.size(), "PCS.ScanJobs");
-    AZK_CU(cudaMemcpyAsync(d_scan.p, jobs, sizeof(ScanJob) * m, cudaMemcpyHostToDevice, s_up));
-    AZK_CU(launch_scan_inputs(d_scan.as<ScanJob>(), (uint32_t)m, max_n, d_flag(), s_up));
-    AZK_CU(cudaMemcpyAsync(f, d_flag(), 4, cudaMemcpyDeviceToHost, s_up));
-    AZK_CU(cudaMemcpyAsync(h, d_info(), sizeof(InputInfo) * m, cudaMemcpyDeviceToHost, s_up));
+    uint8_t* d = arena.at<uint8_t>(off_flag);
+    AZK_CU(cudaMemcpyAsync(d, hblock(), scan_jobs_at() + sizeof(ScanJob) * m, cudaMemcpyHostToDevice, s_up));
+    AZK_CU(launch_scan_inputs(reinterpret_cast<const ScanJob*>(d + scan_jobs_at()), (uint32_t)m, max_n, d_flag(), s_up));
+    AZK_CU(cudaMemcpyAsync(hblock(), d, scan_info_at() + sizeof(InputInfo) * m, cudaMemcpyDeviceToHost, s_up));
     sync_stream(s_up);
     layout(*f == 0, "input contains a non-canonical field element");
     std::vector<uint8_t> narrow(m);
@@ -243,7 +243,7 @@ struct Engine {
     size_t n = cfg.size();
     if (!tm_a) AZK_CU(cudaEventCreate(&tm_a));
     if (!tm_b) AZK_CU(cudaEventCreate(&tm_b));
-    hsmall.ensure(64 + align_up(sizeof(InputInfo) * n, 16) + sizeof(ScanJob) * n);
+    hsmall.ensure(64 + scan_bytes());
     leaf_values = cfg.empty() ? 1 : cfg[0].leaf_values;
     for (auto& i : cfg) {
       layout(i.leaf_values == leaf_values && (leaf_values == 1 || leaf_values == 4), "all instances of a batch share one leaf size (16 or 64 bytes)");
@@ -282,8 +282,8 @@ struct Engine {
     uint64_t off_proofs = arena.reserve(proof_total);
     for (size_t i = 0; i < n; i++) off_proof[i] = off_proofs + proof_off[i];
     off_inst = arena.reserve(sizeof(PcsInstance) * n);
-    off_flag = arena.reserve(16);
-    off_info = arena.reserve(sizeof(InputInfo) * n);
+    off_flag = arena.reserve(scan_bytes());
+    off_info = off_flag + scan_info_at();
     off_queue = arena.reserve(8ull * (rmax + 1));
     arena.commit("PCS.Arena");
     // counters and inputs start at zero
@@ -547,13 +547,17 @@ struct Engine {
   void set_publics(const uint8_t* pubs) {
     const size_t na = active();
     for (size_t i = 0; i < na; i++) std::memcpy(h_inst[i].pub, pubs + 32 * i, 32);
+    if (na == 1) {
+      AZK_CU(cudaMemcpyAsync(d_inst()[0].pub, pubs, 32, cudaMemcpyHostToDevice, s));
+      return;
+    }
     AZK_CU(cudaMemcpy2DAsync(reinterpret_cast<uint8_t*>(d_inst()) + offsetof(PcsInstance, pub), sizeof(PcsInstance), pubs, 32, 32, na,
                              cudaMemcpyHostToDevice, s));
   }
 
-  // Run the whole superstep; returns device seconds.
-  double run(bool from_coeffs, bool plain, uint64_t* submit_ns, const Timer& t) {
-    AZK_CU(cudaMemsetAsync(d_flag(), 0, 4, s));
+  // Queue the whole superstep and the readback of the FFT's status word; the caller
+  // queues its own copies, waits for the stream once and calls finish_run.
+  void run(bool from_coeffs, bool plain, uint64_t* submit_ns, const Timer& t) {
     GpuTimer g(s, tm_a, tm_b);
     if (plain) {
       ev_used = 0;
@@ -584,7 +588,16 @@ struct Engine {
     }
     if (submit_ns) *submit_ns = t.ns();
     g.stop();
-    return g.seconds();
+    if (from_coeffs) fft.queue_status(s, hword(2));
+    else *hword(2) = 0;
+  }
+  // After the stream has finished: fails if an FFT pass gave up, else the device
+  // seconds of the run.
+  double finish_run() {
+    fft.check_status(s, hword(2));
+    float ms = 0;
+    AZK_CU(cudaEventElapsedTime(&ms, tm_a, tm_b));
+    return ms / 1000.0;
   }
 
   // Reject non-canonical inputs (QM31CanonicalityCheck.swift): checked on the
@@ -679,18 +692,15 @@ static void pcs_ensure_claimed(azk_pcs_prover* p, const std::vector<uint64_t>& c
 static void pcs_prove_common(azk_pcs_prover* p, bool coeffs, const uint8_t pub[32], uint8_t* proof_out, bool proof_on_device, uint64_t* proof_len,
                              azk_stats* st, const Timer& t) {
   Engine& e = p->eng;
+  const uint64_t len = e.proof_len[0];
+  layout(*proof_len >= len, "proof buffer too small");
   e.set_publics(pub);
   uint64_t sub = 0;
-  double gs = e.run(coeffs, true, &sub, t);
-  if (coeffs) e.fft.check_status(e.s);
-  uint64_t len = e.proof_len[0];
-  layout(*proof_len >= len, "proof buffer too small");
-  *proof_len = len;
-  if (proof_on_device)
-    AZK_CU(cudaMemcpyAsync(proof_out, e.h_inst[0].proof, len, cudaMemcpyDeviceToDevice, e.s));
-  else
-    AZK_CU(cudaMemcpyAsync(proof_out, e.h_inst[0].proof, len, cudaMemcpyDeviceToHost, e.s));
+  e.run(coeffs, true, &sub, t);
+  AZK_CU(cudaMemcpyAsync(proof_out, e.h_inst[0].proof, len, proof_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, e.s));
   sync_stream(e.s);
+  const double gs = e.finish_run();
+  *proof_len = len;
   fill_stats(st, t, sub, gs);
 }
 
@@ -909,10 +919,9 @@ azk_status azk_batch_prove(azk_batch* b, const uint8_t* pubs, int plain, azk_sta
     Engine& e = b->eng;
     e.set_publics(pubs);
     uint64_t sub = 0;
-    double gs = e.run(true, plain != 0, &sub, t);
+    e.run(true, plain != 0, &sub, t);
     sync_stream(e.s);
-    e.fft.check_status(e.s);
-    fill_stats(st, t, sub, gs);
+    fill_stats(st, t, sub, e.finish_run());
   });
 }
 
@@ -939,6 +948,43 @@ azk_status azk_batch_download_proofs(azk_batch* b, uint8_t* out, uint64_t cap) {
       layout(pos + e.proof_len[i] <= cap, "proof buffer too small");
       AZK_CU(cudaMemcpyAsync(out + pos, e.h_inst[i].proof, e.proof_len[i], cudaMemcpyDeviceToHost, e.s));
       pos += e.proof_len[i];
+    }
+    sync_stream(e.s);
+  });
+}
+
+// First touch of large fresh result buffers by several threads: a copy into them
+// otherwise takes its page faults one after another on the calling thread (61 MB of
+// proofs in fresh pages: 30 ms, 6 ms into touched ones).
+static void touch_pages(void* const* outs, const std::vector<uint64_t>& bytes) {
+  uint64_t total = 0;
+  for (uint64_t n : bytes) total += n;
+  const unsigned threads = std::min(8u, std::max(1u, std::thread::hardware_concurrency() / 2));
+  if (total < (4ull << 20) || threads < 2) return;
+  auto touch = [&](unsigned t) {
+    for (size_t i = t; i < bytes.size(); i += threads)
+      for (uint64_t k = 0; k < bytes[i]; k += 4096) static_cast<volatile uint8_t*>(outs[i])[k] = 0;
+  };
+  std::vector<std::thread> pool;
+  try {
+    for (unsigned t = 1; t < threads; t++) pool.emplace_back(touch, t);
+  } catch (const std::system_error&) {
+    // fewer threads: the copy faults in what is left
+  }
+  touch(0);
+  for (auto& t : pool) t.join();
+}
+
+azk_status azk_batch_download_each(azk_batch* b, void* const* outs) {
+  return guarded(b ? b->ctx : nullptr, [&] {
+    layout(b && outs);
+    std::lock_guard<std::mutex> lk(b->mu);
+    Engine& e = b->eng;
+    layout(e.has_proofs(), "a 64-byte-leaf batch produces commitments, challenges and final layers (azk_batch_trace), not proof bytes");
+    for (size_t i = 0; i < e.cfg.size(); i++) layout(outs[i] != nullptr);
+    touch_pages(outs, e.proof_len);
+    for (size_t i = 0; i < e.cfg.size(); i++) {
+      AZK_CU(cudaMemcpyAsync(outs[i], e.h_inst[i].proof, e.proof_len[i], cudaMemcpyDeviceToHost, e.s));
     }
     sync_stream(e.s);
   });
@@ -1211,30 +1257,16 @@ void run_pcs_group(azk_server* sv, Resident& r, std::vector<std::shared_ptr<Serv
   for (size_t i = 0; i < m; i++)
     AZK_CU(cudaMemcpyAsync(pin + i * align_up(proof, 64), e->h_inst[i].proof, proof, cudaMemcpyDeviceToHost, e->s));
   sync_stream(e->s);
-  e->fft.check_status(e->s, e->hword(1));
+  e->finish_run();
   for (size_t i = 0; i < m; i++) g[i]->result.assign(pin + i * align_up(proof, 64), pin + i * align_up(proof, 64) + proof);
 }
 
-// Sum-check of one table through reusable device buffers (the single-table entry
-// point): evaluations upload, one kernel, results download.  Output words: claimed
-// sum, final evaluation, digest (8 words), sums at 0, sums at 1, challenges
-// (rounds each).  `evals` and `pin` (>= sumcheck_pinned_bytes) may be the same
-// page-locked buffer: the evaluations are consumed by the upload before the
-// results land.
 void sumcheck_alloc(SumcheckBufs& b, uint32_t logn) {
   const uint64_t n = 1ull << logn;
   b.ev.alloc(4 * n, "Sumcheck.Evals");
   b.scratch.alloc(4 * n, "Sumcheck.Scratch");
   b.rounds.alloc(12ull * logn + 64, "Sumcheck.Rounds");
   b.out.alloc(sizeof(SumcheckOut), "Sumcheck.Out");
-}
-// The SumcheckOut a table's kernel fills (per-round arrays in b.rounds).
-SumcheckOut sumcheck_out_ptrs(const SumcheckBufs& b, uint32_t logn) {
-  SumcheckOut o{};
-  o.r0 = b.rounds.as<uint32_t>();
-  o.r1 = o.r0 + logn;
-  o.challenges = o.r1 + logn;
-  return o;
 }
 std::vector<uint32_t> sumcheck_words(const SumcheckOut& r, const uint32_t* rounds_h, uint32_t logn) {
   std::vector<uint32_t> words = {r.claimed_sum, r.final_eval};
@@ -1245,23 +1277,39 @@ std::vector<uint32_t> sumcheck_words(const SumcheckOut& r, const uint32_t* round
   words.insert(words.end(), rounds_h, rounds_h + 3 * logn);
   return words;
 }
-std::vector<uint32_t> sumcheck_run(SumcheckBufs& b, const uint32_t* evals, uint32_t logn, cudaStream_t s, uint8_t* pin, double* gpu_s = nullptr) {
-  const uint64_t n = 1ull << logn;
-  if (!b.ev.p) sumcheck_alloc(b, logn);
-  AZK_CU(cudaMemcpyAsync(b.ev.p, evals, 4 * n, cudaMemcpyHostToDevice, s));
-  SumcheckOut* h = reinterpret_cast<SumcheckOut*>(pin + align_up(4 * n, 64));
-  uint32_t* rounds_h = reinterpret_cast<uint32_t*>(h + 1);
-  *h = sumcheck_out_ptrs(b, logn);
-  AZK_CU(cudaMemcpyAsync(b.out.p, h, sizeof(SumcheckOut), cudaMemcpyHostToDevice, s));
-  std::unique_ptr<GpuTimer> gt;
-  if (gpu_s) gt.reset(new GpuTimer(s));
-  AZK_CU(launch_sumcheck(b.ev.as<uint32_t>(), logn, b.scratch.as<uint32_t>(), b.out.as<SumcheckOut>(), s));
-  if (gt) gt->stop();
-  AZK_CU(cudaMemcpyAsync(h, b.out.p, sizeof(SumcheckOut), cudaMemcpyDeviceToHost, s));
-  AZK_CU(cudaMemcpyAsync(rounds_h, b.rounds.p, 12ull * logn, cudaMemcpyDeviceToHost, s));
+// Device memory of one table proved alone: evaluations, the output record, the
+// per-round words behind it (so one copy brings both back), the folding scratch.
+struct SumcheckLayout {
+  uint64_t out, rounds, back, scratch, total;
+  explicit SumcheckLayout(uint32_t logn) {
+    out = align_up(4ull << logn, 64);
+    rounds = out + sizeof(SumcheckOut);
+    back = sizeof(SumcheckOut) + 12ull * logn;
+    scratch = align_up(out + back, 256);
+    total = scratch + (4ull << logn);
+  }
+  uint64_t host_bytes() const { return out + back; }
+};
+// Sum-check of one table (the single-table entry point) in `dev`, with `pin` (page-
+// locked, host_bytes) as staging.  Output words: claimed sum, final evaluation,
+// digest (8 words), sums at 0, sums at 1, challenges (rounds each).
+std::vector<uint32_t> sumcheck_run(uint8_t* dev, uint8_t* pin, const uint32_t* evals, uint32_t logn, cudaStream_t s, double* gpu_s) {
+  const SumcheckLayout l(logn);
+  std::memcpy(pin, evals, 4ull << logn);
+  SumcheckOut* h = reinterpret_cast<SumcheckOut*>(pin + l.out);
+  *h = SumcheckOut{};
+  h->r0 = reinterpret_cast<uint32_t*>(dev + l.rounds);
+  h->r1 = h->r0 + logn;
+  h->challenges = h->r1 + logn;
+  AZK_CU(cudaMemcpyAsync(dev, pin, l.rounds, cudaMemcpyHostToDevice, s));
+  GpuTimer gt(s);
+  AZK_CU(launch_sumcheck(reinterpret_cast<const uint32_t*>(dev), logn, reinterpret_cast<uint32_t*>(dev + l.scratch),
+                         reinterpret_cast<SumcheckOut*>(dev + l.out), s));
+  gt.stop();
+  AZK_CU(cudaMemcpyAsync(h, dev + l.out, l.back, cudaMemcpyDeviceToHost, s));
   sync_stream(s);
-  if (gt) *gpu_s = gt->seconds();
-  return sumcheck_words(*h, rounds_h, logn);
+  *gpu_s = gt.seconds();
+  return sumcheck_words(*h, reinterpret_cast<const uint32_t*>(pin + l.rounds), logn);
 }
 
 // Evict the least recently used cached shape of worker `w` into `dropped` (freed by
@@ -1522,6 +1570,7 @@ void lane_touch(SumcheckSlot& sl, cudaStream_t s) {
 // Lane launcher: whenever tables wait and a lane stream is idle, one batched
 // launch proves up to kLaneBatch of them.
 void lane_launcher(azk_server* sv) {
+  t_shared_host = true;
   cudaSetDevice(sv->ctx->device);
   for (;;) {
     int sid = -1;
@@ -1603,6 +1652,7 @@ void lane_launcher(azk_server* sv) {
 // 200 us, nothing queued behind the kernels), and publishes a finished batch's
 // results from its slots' mapped staging.
 void lane_completer(azk_server* sv) {
+  t_shared_host = true;
   cudaSetDevice(sv->ctx->device);
   for (;;) {
     std::vector<int> inflight;
@@ -1656,6 +1706,7 @@ void lane_completer(azk_server* sv) {
 }
 
 void worker_loop(azk_server* sv, int w) {
+  t_shared_host = true;
   cudaSetDevice(sv->ctx->device);
   // everything this worker runs (uploads and proof kernels) goes on its one stream:
   // its groups run one at a time, and one stream per worker keeps each worker on
@@ -1805,12 +1856,39 @@ azk_status azk_sumcheck_prove(azk_ctx* ctx, const uint32_t* evals, uint64_t coun
     std::lock_guard<std::mutex> lk(ctx->mu);
     Timer t;
     uint32_t logn = ilog2(count);
-    SumcheckBufs b;
-    Staging staging;
-    uint8_t* pin = staging.ensure(sumcheck_pinned_bytes(logn));
-    std::memcpy(pin, evals, 4ull << logn);
+    AZK_CU(cudaSetDevice(ctx->device));
+    const SumcheckLayout l(logn);
+    DevBuf own;
+    HostPinned own_pin;
+    uint8_t *dev, *pin;
+    if (logn <= azk_ctx::kSumcheckKeptLog) {
+      // allocating and freeing both for every call took 2 to 3 ms of a 2^18 table's 18
+      if (ctx->sumcheck_dev_bytes < l.total) {
+        if (ctx->sumcheck_dev) cudaFree(ctx->sumcheck_dev);
+        ctx->sumcheck_dev = nullptr;
+        ctx->sumcheck_dev_bytes = 0;
+        DevBuf b(l.total, "Sumcheck.Table");
+        std::swap(ctx->sumcheck_dev, b.p);
+        ctx->sumcheck_dev_bytes = l.total;
+      }
+      if (ctx->sumcheck_pin_bytes < l.host_bytes()) {
+        if (ctx->sumcheck_pin) cudaFreeHost(ctx->sumcheck_pin);
+        ctx->sumcheck_pin = nullptr;
+        ctx->sumcheck_pin_bytes = 0;
+        HostPinned b;
+        b.ensure(l.host_bytes());
+        std::swap(ctx->sumcheck_pin, b.p);
+        ctx->sumcheck_pin_bytes = l.host_bytes();
+      }
+      dev = static_cast<uint8_t*>(ctx->sumcheck_dev);
+      pin = static_cast<uint8_t*>(ctx->sumcheck_pin);
+    } else {
+      own.alloc(l.total, "Sumcheck.Table");
+      dev = own.as<uint8_t>();
+      pin = static_cast<uint8_t*>(own_pin.ensure(l.host_bytes()));
+    }
     double gpu_s = 0.0;
-    std::vector<uint32_t> w = sumcheck_run(b, reinterpret_cast<const uint32_t*>(pin), logn, ctx->stream, pin, &gpu_s);
+    const std::vector<uint32_t> w = sumcheck_run(dev, pin, evals, logn, ctx->stream, &gpu_s);
     *claimed_sum = w[0];
     *final_eval = w[1];
     std::memcpy(digest, w.data() + 2, 32);
