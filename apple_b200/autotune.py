@@ -60,7 +60,7 @@ def shape_grid(logs=range(6, 23), concurrents=(1, 8, 64), max_leaves=1 << 24):
                 continue
             shapes.append((lg, 16, 0, c))
             shapes.append((lg, 16, 1, c))
-            if lg <= 20:
+            if lg <= 20 or c == 1:
                 shapes.append((lg, 64, 0, c))
     return shapes
 
@@ -299,6 +299,10 @@ class Tuner:
         cands = [(t, th) for t in tile_candidates(lg) for th in self.threads if (lg, lb, fold, c, t, th) in self._table]
         return min(cands, key=lambda s: self._table[(lg, lb, fold, c, s[0], s[1])])
 
+    def has_timings(self, shape) -> bool:
+        lg, lb, fold, c = shape
+        return any((lg, lb, fold, c, t, th) in self._table for t in tile_candidates(lg) for th in self.threads)
+
     def measured(self, shape, sched):
         return self._table.get((*shape, *sched))
 
@@ -356,28 +360,32 @@ class Tuner:
             out["heuristic"].append(h / best - 1.0)
         return {k: {"mean": float(np.mean(v)), "max": float(np.max(v)), "n": len(v)} for k, v in out.items()}
 
-    def layer_table(self, concurrent=1, leaf_bytes=16, fold=1, logs=range(1, 27), threads=256) -> dict:
+    def layer_table(self, concurrent=1, leaf_bytes=16, fold=1, logs=range(1, 27), threads=256, verify=0) -> dict:
         """{layer log size: treelet depth} for an azk_schedule's layer_treelet (the
         commit kernel's thread count is one per launch, so the table is chosen at a
-        fixed `threads`; over the measured shapes that costs at most a few percent)."""
+        fixed `threads`; over the measured shapes that costs at most a few percent).
+        Of the shapes measured, the model's top `verify` are timed and the fastest kept."""
         table = {}
         for lg in logs:
             if lg < 2:
                 table[lg] = 1
                 continue
-            t, _ = self.choose((lg, leaf_bytes, fold, concurrent), threads=threads)
+            shape = (lg, leaf_bytes, fold, concurrent)
+            t, _ = self.choose(shape, threads=threads, verify=verify if self.has_timings(shape) else 0)
             table[lg] = int(t)
         return table
 
-    def layer_tables(self, concurrent=1, leaf_bytes=16, fold=1, logs=range(1, 27)):
+    def layer_tables(self, concurrent=1, leaf_bytes=16, fold=1, logs=range(1, 27), verify=0):
         """({layer log: treelet depth}, {layer log: threads}): the model's pick over
-        depth and threads per CTA for each layer size."""
+        depth and threads per CTA for each layer size (of its top `verify`, timed, for
+        the shapes measured)."""
         tiles, threads = {}, {}
         for lg in logs:
             if lg < 2:
                 tiles[lg], threads[lg] = 1, 256
                 continue
-            t, th = self.choose((lg, leaf_bytes, fold, concurrent))
+            shape = (lg, leaf_bytes, fold, concurrent)
+            t, th = self.choose(shape, verify=verify if self.has_timings(shape) else 0)
             tiles[lg], threads[lg] = int(t), int(th)
         return tiles, threads
 
@@ -419,6 +427,8 @@ TABLE_SHAPES = {
 # at most 1 % (log 6-18), and the largest layers (2^19-2^22 leaves x 64) are
 # outside the measured grid, so the depth is chosen at the default 256 threads.
 FIXED_THREADS = {"pcs_batch": 256}
+# Candidates of each measured shape that the export times before it picks one.
+EXPORT_VERIFY = 4
 
 
 def export(tuner: Tuner, report: dict, json_path: str, header_path: str):
@@ -429,10 +439,10 @@ def export(tuner: Tuner, report: dict, json_path: str, header_path: str):
     for name, kw in TABLE_SHAPES.items():
         if name in FIXED_THREADS:
             th = FIXED_THREADS[name]
-            tiles = tuner.layer_table(threads=th, **kw)
+            tiles = tuner.layer_table(threads=th, verify=EXPORT_VERIFY, **kw)
             both[name] = (tiles, {lg: th for lg in tiles})
         else:
-            both[name] = tuner.layer_tables(**kw)
+            both[name] = tuner.layer_tables(verify=EXPORT_VERIFY, **kw)
     doc = {"device": _device_name(tuner.ctx), "report": report, "shapes": TABLE_SHAPES, "fixed_threads": FIXED_THREADS,
            "tables": {k: {str(lg): t for lg, t in v[0].items()} for k, v in both.items()},
            "thread_tables": {k: {str(lg): t for lg, t in v[1].items()} for k, v in both.items()}}

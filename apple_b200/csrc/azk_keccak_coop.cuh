@@ -58,8 +58,11 @@ __host__ __device__ __forceinline__ uint64_t join64(uint32_t even, uint32_t odd)
 // exchanges are full-warp shuffles), so callers keep warps converged and clamp the
 // indices of lanes without work.
 // ---------------------------------------------------------------------------
+struct alignas(8) SplitRC {
+  uint32_t even, odd;
+};
 struct KeccakSplitRC {
-  uint32_t w[24][2];
+  SplitRC w[24];
 };
 constexpr uint32_t keccak_every_second_bit(uint64_t v) {
   uint32_t r = 0;
@@ -73,13 +76,16 @@ constexpr KeccakSplitRC keccak_split_rc() {
                            0x8000000000008003ULL, 0x8000000000008002ULL, 0x8000000000000080ULL, 0x000000000000800AULL, 0x800000008000000AULL,
                            0x8000000080008081ULL, 0x8000000000008080ULL, 0x0000000080000001ULL, 0x8000000080008008ULL};
   KeccakSplitRC r{};
-  for (int i = 0; i < 24; i++) {
-    r.w[i][0] = keccak_every_second_bit(rc[i]);
-    r.w[i][1] = keccak_every_second_bit(rc[i] >> 1);
-  }
+  for (int i = 0; i < 24; i++) r.w[i] = SplitRC{keccak_every_second_bit(rc[i]), keccak_every_second_bit(rc[i] >> 1)};
   return r;
 }
 __constant__ static const KeccakSplitRC kKeccakSplitRC = keccak_split_rc();
+// One uniform 8-byte load and a select: loads indexed or predicated by the lane's
+// parity cost a round 10 cycles.
+__device__ __forceinline__ uint32_t split_rc(int r, uint32_t q) {
+  const uint2 v = reinterpret_cast<const uint2*>(kKeccakSplitRC.w)[r];
+  return q ? v.y : v.x;
+}
 
 template <int I>
 __device__ __forceinline__ void pair_rho_pi_lane(const uint32_t (&a)[25], const uint32_t (&c)[5], const uint32_t (&r1)[5], uint32_t (&b)[25], uint32_t q) {
@@ -120,8 +126,8 @@ __device__ __forceinline__ void pair_round(uint32_t (&a)[25], uint32_t q, uint32
 __device__ __forceinline__ void pair_f1600(uint32_t (&a)[25], uint32_t q) {
 #pragma unroll 1
   for (int r = 0; r < 24; r += 2) {
-    pair_round(a, q, kKeccakSplitRC.w[r][q]);
-    pair_round(a, q, kKeccakSplitRC.w[r + 1][q]);
+    pair_round(a, q, split_rc(r, q));
+    pair_round(a, q, split_rc(r + 1, q));
   }
 }
 
@@ -196,7 +202,7 @@ struct WarpKeccak {
   uint64_t rc_mask;     // all ones on lane 0
   bool stores;
 
-  __device__ WarpKeccak(uint32_t lane, uint64_t* smem) : col(smem) {
+  __device__ __forceinline__ WarpKeccak(uint32_t lane, uint64_t* smem) : col(smem) {
     const uint32_t t = lane < 25 ? lane : 0;
     const uint32_t x = t % 5, y = t / 5;
     own = 6 * x + y;

@@ -74,9 +74,9 @@ struct WarpSponge {
   uint64_t a;
 
   // `smem`: kWarpKeccakWords words of shared memory of this warp's own.
-  __device__ WarpSponge(uint64_t* smem) : kf(threadIdx.x & 31, smem), lane(threadIdx.x & 31), a(0) {}
-  __device__ void load(const Transcript* t) { a = lane < 25 ? __ldcg(&t->st[lane]) : 0; }
-  __device__ void store(Transcript* t) const {
+  __device__ __forceinline__ WarpSponge(uint64_t* smem) : kf(threadIdx.x & 31, smem), lane(threadIdx.x & 31), a(0) {}
+  __device__ __forceinline__ void load(const Transcript* t) { a = lane < 25 ? __ldcg(&t->st[lane]) : 0; }
+  __device__ __forceinline__ void store(Transcript* t) const {
     if (lane < 25) t->st[lane] = a;
   }
   // One padded block (lane m < 17 passes message word m).
@@ -85,7 +85,7 @@ struct WarpSponge {
     kf.permute_small(a);
   }
   // Word `lane` of a padded 32-byte message.
-  __device__ uint64_t digest_word(const uint64_t* d) const { return lane < 4 ? d[lane] : lane == 4 ? 0x06ull : lane == 16 ? kPadEnd : 0ull; }
+  __device__ __forceinline__ uint64_t digest_word(const uint64_t* d) const { return lane < 4 ? d[lane] : lane == 4 ? 0x06ull : lane == 16 ? kPadEnd : 0ull; }
   // A message of `bytes` bytes (a multiple of 8) in global memory.
   __device__ __forceinline__ void absorb_words(const uint64_t* p, uint64_t bytes) {
     const uint64_t n = bytes / 8;
@@ -101,7 +101,7 @@ struct WarpSponge {
     }
   }
   // Four field elements (challenge limbs), in every lane; the state is unchanged.
-  __device__ void squeeze4_m31(uint32_t (&out)[4]) {
+  __device__ __forceinline__ void squeeze4_m31(uint32_t (&out)[4]) {
     const uint64_t w0 = __shfl_sync(0xffffffffu, a, 0), w1 = __shfl_sync(0xffffffffu, a, 1);
     const uint32_t c[4] = {(uint32_t)w0, (uint32_t)(w0 >> 32), (uint32_t)w1, (uint32_t)(w1 >> 32)};
     const uint32_t p = 2147483647u;

@@ -38,6 +38,10 @@ __device__ __forceinline__ void ld_dig_cg(const uint64_t* p, uint64_t (&d)[4]) {
   d[0] = a.x; d[1] = a.y; d[2] = b.x; d[3] = b.y;
 }
 
+// This thread's warp, as a value the compiler knows to be the same in all of the
+// warp's lanes.
+__device__ __forceinline__ uint32_t warp_index() { return __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0); }
+
 template <uint32_t KIND>
 __device__ __forceinline__ void leaf_digest(const TreeJob& job, uint64_t leaf, const uint32_t (&ch)[4], uint64_t (&d)[4]) {
   if constexpr (KIND == kLeafQM31) {
@@ -332,7 +336,7 @@ __device__ __noinline__ void pair_leaf_phase(const TreeJob& job, uint32_t items,
                                              uint64_t* out, uint64_t* top) {
   const uint32_t ch[4] = {c0, c1, c2, c3};
   const uint32_t lane = threadIdx.x & 31, q = lane & 1;
-  for (uint32_t base = threadIdx.x / 32 * 16; base < items; base += THREADS / 2) {
+  for (uint32_t base = warp_index() * 16; base < items; base += THREADS / 2) {
     const uint32_t i = base + (lane >> 1);
     const bool ok = i < items;
     const uint64_t leaf = idx0 + (ok ? i : items - 1);
@@ -349,7 +353,7 @@ __device__ __noinline__ void pair_leaf_phase(const TreeJob& job, uint32_t items,
 template <int THREADS>
 __device__ __noinline__ void pair_levels(uint64_t* a, uint64_t* b, uint64_t* top, const uint64_t* nodes, uint32_t n, const TreeJob& job, uint32_t level,
                                          uint64_t idx0) {
-  const uint32_t lane = threadIdx.x & 31, q = lane & 1;
+  const uint32_t warp = warp_index(), lane = threadIdx.x & 31, q = lane & 1;
   uint64_t* src = a;
   uint64_t* dst = b;
   if (nodes != nullptr) dst = a;
@@ -358,7 +362,7 @@ __device__ __noinline__ void pair_levels(uint64_t* a, uint64_t* b, uint64_t* top
     idx0 >>= 1;
     level++;
     uint64_t* lv = job.inner + 4 * (inner_offset(job.logn, level) + idx0);
-    for (uint32_t base = threadIdx.x / 32 * 16; base < n; base += THREADS / 2) {
+    for (uint32_t base = warp * 16; base < n; base += THREADS / 2) {
       const uint32_t i = base + (lane >> 1);
       const bool ok = i < n;
       const uint32_t j = ok ? i : n - 1;
@@ -406,7 +410,7 @@ __device__ __forceinline__ void warp_parent(const WarpKeccak& kf, const uint64_t
 template <int THREADS>
 __device__ __noinline__ void top_levels(uint64_t* top, uint32_t count, const TreeJob& job, uint32_t level, uint64_t idx0, bool root, uint64_t* warp_smem) {
   static_assert(THREADS >= 128, "four warps");
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t act = root ? job.root_action : (uint32_t)kRootNone;
   if (warp >= 4) return;
   if (warp == 3 && act != kRootNone) {
