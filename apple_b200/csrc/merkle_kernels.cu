@@ -248,10 +248,9 @@ __device__ __forceinline__ uint64_t raw_message_word(const TreeJob& job, const u
   const uint32_t full = job.len >> 3, rem = job.len & 7;
   if (i > full || i > 16) return 0;
   if (i < full && job.aligned8) return __ldg(reinterpret_cast<const uint64_t*>(p) + i);
-  uint64_t v = i < full ? 0 : (uint64_t)job.suffix << (8 * rem);
   const uint32_t n = i < full ? 8 : rem;
-  for (uint32_t k = 0; k < n; k++) v |= (uint64_t)__ldg(p + 8 * i + k) << (8 * k);
-  return v;
+  const uint64_t v = i < full ? 0 : (uint64_t)job.suffix << (8 * rem);
+  return n ? v | UnalignedWords(p).word(i, n) : v;
 }
 
 // Digest of one leaf by a pair of lanes, in split form.  `ok`: the pair's leaf is
