@@ -104,24 +104,35 @@ struct WarpSponge {
   __device__ __forceinline__ void squeeze4_m31(uint32_t (&out)[4]) {
     const uint64_t w0 = __shfl_sync(0xffffffffu, a, 0), w1 = __shfl_sync(0xffffffffu, a, 1);
     const uint32_t c[4] = {(uint32_t)w0, (uint32_t)(w0 >> 32), (uint32_t)w1, (uint32_t)(w1 >> 32)};
-    const uint32_t p = 2147483647u;
     bool over = false;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
       over |= c[k] >= 0xFFFFFFFEu;
-      const uint32_t s = (c[k] & p) + (c[k] >> 31);
-      out[k] = s >= p ? s - p : s;
+      out[k] = mod_p(c[k]);
     }
-    if (over) {
-      __syncwarp();
-      if (lane < 25) kf.col[lane] = a;
-      __syncwarp();
-      uint32_t o[4];
-      squeeze_m31_slow(kf.col, 4, o);
-#pragma unroll
-      for (int k = 0; k < 4; k++) out[k] = o[k];
-      __syncwarp();
-    }
+    if (over) squeeze_slow(4, out);
+  }
+  __device__ __forceinline__ uint32_t squeeze1_m31() {
+    const uint32_t c = (uint32_t)__shfl_sync(0xffffffffu, a, 0);
+    uint32_t out[4] = {mod_p(c)};
+    if (c >= 0xFFFFFFFEu) squeeze_slow(1, out);
+    return out[0];
+  }
+
+ private:
+  static __device__ __forceinline__ uint32_t mod_p(uint32_t c) {  // c < 2^32 - 2
+    const uint32_t p = 2147483647u, s = (c & p) + (c >> 31);
+    return s >= p ? s - p : s;
+  }
+  __device__ __forceinline__ void squeeze_slow(uint32_t count, uint32_t (&out)[4]) {
+    __syncwarp();
+    if (lane < 25) kf.col[lane] = a;
+    __syncwarp();
+    uint32_t o[4];
+    squeeze_m31_slow(kf.col, count, o);
+    for (uint32_t k = 0; k < 4; k++)
+      if (k < count) out[k] = o[k];
+    __syncwarp();
   }
 };
 

@@ -11,18 +11,9 @@
 // batched kernel packs four tables into one CTA (sumcheck_packed_kernel).
 #include "azk_field.cuh"
 #include "azk_internal.h"
-#include "azk_keccak_coop.cuh"
+#include "azk_transcript_warp.cuh"
 
 namespace azk {
-
-__device__ void sc_frame(FrameBuf& f, uint8_t type) {
-  const char dom[] = "AppleZKProver.M31MultilinearSumcheck";
-  f.n = 0;
-  fb_u32(f, 36);
-  fb_str(f, dom, 36);
-  fb_u32(f, 1);
-  fb_u8(f, type);
-}
 
 // Byte k of the framed word-digest input: u32 len || "AppleZKProver.M31Sumcheck.Words.V1"
 // || u32 1 || u64 count || words (little-endian) (SumcheckOracle.swift:1288-1299).
@@ -187,21 +178,19 @@ __device__ void sumcheck_prove_group(const G& grp, SumcheckShared& sh, const uin
   }
   uint32_t zs = group_sum_m31(grp, z, sh.red, parity);
   uint32_t os = group_sum_m31(grp, o, sh.red, parity);
-  // group_sum_m31's value is valid in thread 0, which alone runs the transcript
-  // (the digest lanes are visible to it after the first sum's barrier)
+  // group_sum_m31's value is valid in thread 0, whose warp runs the transcript (the
+  // digest lanes are visible to it after the first sum's barrier)
   const uint32_t total = m31_add(zs, os);
-  Transcript tr;
-  if (t == 0) {
-    out->claimed_sum = total;
-    for (int i = 0; i < 4; i++) out->digest[i] = sh.digest[i];
-    tr_reset(tr);
-    FrameBuf f;
-    sc_frame(f, 0);
-    fb_u64(f, n);
-    fb_u32(f, log_n);
-    fb_u32(f, total);
-    for (int i = 0; i < 4; i++) fb_u64(f, sh.digest[i]);
-    tr_absorb(tr, f.b, f.n);
+  WarpSponge sp(sh.col);
+  if (t < 32) {
+    if (t == 0) {
+      out->claimed_sum = total;
+      for (int i = 0; i < 4; i++) out->digest[i] = sh.digest[i];
+    }
+    uint32_t p[12] = {(uint32_t)n, (uint32_t)(n >> 32), log_n, __shfl_sync(0xffffffffu, total, 0)};
+#pragma unroll
+    for (int i = 0; i < 4; i++) p[4 + 2 * i] = (uint32_t)sh.digest[i], p[5 + 2 * i] = (uint32_t)(sh.digest[i] >> 32);
+    sp.absorb(frame_word<SumcheckFrame>(sp.lane, 0, p));
   }
   const uint32_t* cur = evals;
   uint32_t* bufs[2] = {scratch, scratch + (n >> 1)};
@@ -215,23 +204,19 @@ __device__ void sumcheck_prove_group(const G& grp, SumcheckShared& sh, const uin
   }
   for (uint32_t r = 0; r < log_n; r++) {
     const uint64_t half = (n >> r) >> 1;
-    if (t == 0) {
-      r0[r] = zs;
-      r1[r] = os;
-      FrameBuf f;
-      sc_frame(f, 1);
-      fb_u32(f, r);
-      fb_u32(f, zs);
-      fb_u32(f, os);
-      tr_absorb(tr, f.b, f.n);
-      sc_frame(f, 2);
-      fb_u32(f, r);
-      fb_u32(f, kP);
-      tr_absorb(tr, f.b, f.n);
-      uint32_t c;
-      tr_squeeze_u32(tr, 1, kP, &c);
-      chs[r] = c;
-      sh.ch = c;
+    if (t < 32) {
+      const uint32_t z0 = __shfl_sync(0xffffffffu, zs, 0), o0 = __shfl_sync(0xffffffffu, os, 0);
+      const uint32_t pr[3] = {r, z0, o0}, pc[2] = {r, kP};
+      const uint64_t fr = frame_word<SumcheckFrame>(sp.lane, 1, pr), fc = frame_word<SumcheckFrame>(sp.lane, 2, pc);
+#pragma unroll 1
+      for (uint32_t step = 0; step < 2; step++) sp.absorb(step == 0 ? fr : fc);
+      const uint32_t c = sp.squeeze1_m31();
+      if (t == 0) {
+        r0[r] = z0;
+        r1[r] = o0;
+        chs[r] = c;
+        sh.ch = c;
+      }
     }
     grp.sync();
     const uint32_t c = sh.ch;
