@@ -549,14 +549,25 @@ __device__ __forceinline__ void tree_tile_body(const TreeJob& job, const uint64_
   }
 }
 
+// The job in shared memory: read once per CTA, not by every use in turn.
+__device__ __forceinline__ void fetch_job(TreeJob& to, const TreeJob* from) {
+  static_assert(sizeof(TreeJob) % 8 == 0, "whole words");
+  if (threadIdx.x < sizeof(TreeJob) / 8) reinterpret_cast<uint64_t*>(&to)[threadIdx.x] = __ldg(reinterpret_cast<const uint64_t*>(from) + threadIdx.x);
+  __syncthreads();
+}
+
 template <uint32_t KIND, int THREADS>
 __global__ void __launch_bounds__(THREADS, 512 / THREADS) tree_tiles_kernel(const TreeJob* __restrict__ jobs, const uint2* __restrict__ work) {
-  // launched before the kernel ahead of it in the stream has ended (launch_tiles):
-  // nothing is read or written before that kernel's memory is complete
+  __shared__ TreeJob job;
+  const uint2 w = work[blockIdx.x];
+  fetch_job(job, jobs + w.x);
+  // Launched before the kernel ahead of it in the stream has ended (launch_tiles): up
+  // to here only the work list and the job were read, which no kernel writes; layers,
+  // challenge, transcript, nodes and counters are touched once that kernel's memory is
+  // complete.
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const uint2 w = work[blockIdx.x];
-  tree_tile_body<KIND, THREADS>(jobs[w.x], w.y);
+  tree_tile_body<KIND, THREADS>(job, w.y);
 }
 
 // Persistent form: a grid of the resident CTAs pulls work items from a device
@@ -567,6 +578,7 @@ template <uint32_t KIND, int THREADS>
 __global__ void __launch_bounds__(THREADS, 512 / THREADS) tree_queue_kernel(const TreeJob* __restrict__ jobs, const uint2* __restrict__ work,
                                                                             uint32_t nwork, uint32_t* __restrict__ queue) {
   __shared__ uint32_t s_item;
+  __shared__ TreeJob job;
   for (;;) {
     if (threadIdx.x == 0) s_item = atomicAdd(queue, 1u);
     __syncthreads();
@@ -574,7 +586,8 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) tree_queue_kernel(cons
     __syncthreads();  // every thread has the item (and the last one's shared memory is free)
     if (item >= nwork) break;
     const uint2 w = work[item];
-    tree_tile_body<KIND, THREADS>(jobs[w.x], w.y);
+    fetch_job(job, jobs + w.x);
+    tree_tile_body<KIND, THREADS>(job, w.y);
   }
   if (threadIdx.x == 0) {
     __threadfence();
