@@ -196,6 +196,32 @@ struct LaunchCfg {
   uint32_t grid_cap = 0;   // 0: one CTA per work item
 };
 
+// Dependent launches: the kernel may be set up while the kernel ahead of it in the
+// stream ends, so a chain of short kernels does not pay the launch latency between
+// them.  Such a kernel calls dependent_begin() before it touches anything that an
+// earlier kernel writes or reads; there it waits for that kernel's memory to be
+// complete and lets its own successor be set up.
+#if defined(__CUDACC__)
+__device__ __forceinline__ void dependent_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... P, class... A>
+inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+#endif
+
 cudaError_t launch_int_issue_probe(int sm_count, cudaStream_t s, uint32_t* d_sink, double* ops_per_launch, uint32_t* blocks_out);
 cudaError_t prepare_tree_kernels();
 cudaError_t launch_tree_direct_raw(const TreeJob& job, cudaStream_t s);

@@ -158,6 +158,7 @@ __device__ __forceinline__ void bfly_q(qm31& l, qm31& r, uint32_t t) {
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS) fft_pass_q_kernel(const FftJob* __restrict__ jobs, const uint2* __restrict__ work) {
   extern __shared__ uint32_t fsm[];
+  dependent_begin();
   const uint2 w = work[blockIdx.x];
   const FftJob& job = jobs[w.x];
   const FftTile ft = fft_tile(job);
@@ -405,6 +406,7 @@ __device__ __forceinline__ void fft_m31_tile_stages(uint32_t* sv, const uint32_t
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS) fft_pass_m31_kernel(const FftJob* __restrict__ jobs, const uint2* __restrict__ work) {
   extern __shared__ uint32_t nsm[];
+  dependent_begin();
   const uint2 w = work[blockIdx.x];
   const FftJob& job = jobs[w.x];
   const FftTile ft = fft_tile(job);
@@ -463,11 +465,9 @@ cudaError_t launch_fft_pass(const FftJob* d_jobs, const uint2* d_work, uint32_t 
   if (nwork == 0) return cudaSuccess;
   switch (kind) {
     case kFftQM31:
-      fft_pass_q_kernel<kFftThreadsQ><<<nwork, kFftThreadsQ, kFftSmemQ, s>>>(d_jobs, d_work);
-      break;
+      return launch_dependent(fft_pass_q_kernel<kFftThreadsQ>, dim3(nwork), dim3(kFftThreadsQ), kFftSmemQ, s, d_jobs, d_work);
     case kFftM31Small:
-      fft_pass_m31_kernel<kFftThreadsM31><<<nwork, kFftThreadsM31, kFftSmemM31, s>>>(d_jobs, d_work);
-      break;
+      return launch_dependent(fft_pass_m31_kernel<kFftThreadsM31>, dim3(nwork), dim3(kFftThreadsM31), kFftSmemM31, s, d_jobs, d_work);
     case kFftM31Tile:
       return launch_fft_m31_tiles(d_jobs, d_work, nwork, s);
     case kFftM31Low:
@@ -586,6 +586,7 @@ __global__ void __launch_bounds__(256, 4) fold_chain_kernel(const uint4* __restr
   __shared__ uint4 buf[kFoldTile / 2 + kFoldTile / 4];
   __shared__ Inv s_inv[kFoldTile / 2];  // the tile's inverses of rounds 1, 2, ...: round r's at kFoldTile / 2 - (kFoldTile >> r)
   __shared__ uint32_t s_ch[4 * kFoldTileRounds];
+  dependent_begin();
   const uint64_t base = (uint64_t)blockIdx.x * kFoldTile;
   uint32_t cnt = (uint32_t)(n_in - base < kFoldTile ? n_in - base : kFoldTile) >> 1;
   if (threadIdx.x < 4 * rounds) s_ch[threadIdx.x] = __ldcg(chp + threadIdx.x);
@@ -652,10 +653,9 @@ cudaError_t launch_fold_chain(const uint4* prev, uint64_t n, const uint4* inv, c
     const uint32_t r = rounds - done < most ? rounds - done : most;
     uint4* o = done + r == rounds ? out : scratch;
     const unsigned blocks = (unsigned)((n + kFoldTile - 1) / kFoldTile);
-    if (m31_inv)
-      fold_chain_kernel<false><<<blocks, 256, 0, s>>>(prev, n, m31_inv, ch + 4 * done, r, o);
-    else
-      fold_chain_kernel<true><<<blocks, 256, 0, s>>>(prev, n, inv, ch + 4 * done, r, o);
+    const cudaError_t e = m31_inv ? launch_dependent(fold_chain_kernel<false>, dim3(blocks), dim3(256), 0, s, prev, n, m31_inv, ch + 4 * done, r, o)
+                                  : launch_dependent(fold_chain_kernel<true>, dim3(blocks), dim3(256), 0, s, prev, n, inv, ch + 4 * done, r, o);
+    if (e != cudaSuccess) return e;
     const uint64_t layers = n - (n >> r);
     if (m31_inv) m31_inv += layers;
     inv += layers;
@@ -664,7 +664,7 @@ cudaError_t launch_fold_chain(const uint4* prev, uint64_t n, const uint4* inv, c
     scratch += n;
     done += r;
   }
-  return cudaGetLastError();
+  return cudaSuccess;
 }
 
 // ---------------------------------------------------------------------------
@@ -734,6 +734,7 @@ __global__ void __launch_bounds__(128) pcs_tail_kernel(const PcsInstance* __rest
   __shared__ __align__(16) uint64_t smem[kWarpKeccakWords];
   const PcsInstance& I = inst[ids[blockIdx.x]];
   const uint64_t cnt = 1ull << (I.logn - I.rounds);
+  dependent_begin();
   uint4* const fl = I.layers + layer_offset(I.logn, I.rounds);
   if ((parts & kTailFoldPart) && cnt <= kTailFold) {
     const uint32_t k = I.rounds;  // >= 1
@@ -801,8 +802,7 @@ __global__ void __launch_bounds__(128) pcs_tail_kernel(const PcsInstance* __rest
 
 cudaError_t launch_pcs_tail(const PcsInstance* d_inst, const uint32_t* d_ids, uint32_t nids, uint32_t parts, cudaStream_t s) {
   if (!nids) return cudaSuccess;
-  pcs_tail_kernel<<<nids, 128, 0, s>>>(d_inst, d_ids, parts);
-  return cudaGetLastError();
+  return launch_dependent(pcs_tail_kernel, dim3(nids), dim3(128), 0, s, d_inst, d_ids, parts);
 }
 
 __device__ __forceinline__ void absorb_grinding(Transcript& t, uint32_t bits, uint64_t nonce) {
@@ -938,6 +938,7 @@ __device__ void emit_query(const PcsInstance& I, uint64_t pair, uint8_t* b, uint
 }
 
 __global__ void pcs_emit_kernel(const PcsInstance* __restrict__ inst, const uint32_t* __restrict__ ids, uint32_t max_queries) {
+  dependent_begin();
   const PcsInstance& I = inst[ids[blockIdx.x]];
   uint8_t* b = I.proof;
   const uint32_t R = I.rounds;
@@ -1005,8 +1006,7 @@ __global__ void pcs_emit_kernel(const PcsInstance* __restrict__ inst, const uint
 cudaError_t launch_pcs_emit(PcsInstance* d_inst, const uint32_t* d_ids, uint32_t nids, uint32_t max_queries, cudaStream_t s) {
   if (!nids) return cudaSuccess;
   dim3 grid(nids, max_queries + 1);
-  pcs_emit_kernel<<<grid, kEmitThreads, 0, s>>>(d_inst, d_ids, max_queries);
-  return cudaGetLastError();
+  return launch_dependent(pcs_emit_kernel, grid, dim3(kEmitThreads), 0, s, d_inst, d_ids, max_queries);
 }
 
 // Queries of committed resident layers (CircleFRIResidentQueryExtractorV1.extractQueries,

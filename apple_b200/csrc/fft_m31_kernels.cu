@@ -294,6 +294,7 @@ __device__ __forceinline__ void m31_tile(const FftJob& job, uint2 w, uint32_t* Y
 // specialised for their stage count, the others the general form.
 __global__ void __launch_bounds__(kThreads, 4) fft_m31_tile_kernel(const FftJob* __restrict__ jobs, const uint2* __restrict__ work) {
   __shared__ __align__(16) uint32_t Y[kTile];
+  dependent_begin();
   const uint2 w = work[blockIdx.x];
   const FftJob& job = jobs[w.x];
   switch (fft_pass_geom(job.logn, job.pass).m) {
@@ -323,6 +324,7 @@ __device__ __forceinline__ uint4 from_q(qm31 v) { return make_uint4(v.a, v.b, v.
 
 __global__ void __launch_bounds__(kThreads, 2) fft_q_tile_kernel(const FftJob* __restrict__ jobs, const uint2* __restrict__ work) {
   extern __shared__ __align__(16) uint4 Yq[];  // kTile values
+  dependent_begin();
   const uint2 w = work[blockIdx.x];
   const FftJob& job = jobs[w.x];
   const Pass p = make_pass(job, w.y);
@@ -408,6 +410,7 @@ __global__ void __launch_bounds__(kThreads, 4) fft_m31_low_tma_kernel(const FftJ
   __shared__ __align__(128) uint32_t X[kTile];  // bulk-copy landing buffer (linear)
   __shared__ __align__(16) uint32_t Y[kTile];   // swizzled working buffer
   __shared__ __align__(8) uint64_t bar;
+  dependent_begin();
   const uint32_t t = threadIdx.x;
   uint32_t item = blockIdx.x;
   if (item >= nwork) return;
@@ -470,14 +473,12 @@ cudaError_t prepare_fft_m31_kernels() {
 
 cudaError_t launch_fft_m31_tiles(const FftJob* d_jobs, const uint2* d_work, uint32_t nwork, cudaStream_t s) {
   if (nwork == 0) return cudaSuccess;
-  fft_m31_tile_kernel<<<nwork, kThreads, 0, s>>>(d_jobs, d_work);
-  return cudaGetLastError();
+  return launch_dependent(fft_m31_tile_kernel, dim3(nwork), dim3(kThreads), 0, s, d_jobs, d_work);
 }
 
 cudaError_t launch_fft_q_tiles(const FftJob* d_jobs, const uint2* d_work, uint32_t nwork, cudaStream_t s) {
   if (nwork == 0) return cudaSuccess;
-  fft_q_tile_kernel<<<nwork, kThreads, kTile * sizeof(uint4), s>>>(d_jobs, d_work);
-  return cudaGetLastError();
+  return launch_dependent(fft_q_tile_kernel, dim3(nwork), dim3(kThreads), kTile * sizeof(uint4), s, d_jobs, d_work);
 }
 
 cudaError_t launch_fft_m31_low(const FftJob* d_jobs, const uint2* d_work, uint32_t nwork, uint32_t* d_status, cudaStream_t s) {
@@ -486,8 +487,7 @@ cudaError_t launch_fft_m31_low(const FftJob* d_jobs, const uint2* d_work, uint32
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
   const uint32_t resident = (uint32_t)g_low_grid[dev];
   const uint32_t grid = resident && resident < nwork ? resident : nwork;
-  fft_m31_low_tma_kernel<<<grid, kThreads, 0, s>>>(d_jobs, d_work, nwork, d_status);
-  return cudaGetLastError();
+  return launch_dependent(fft_m31_low_tma_kernel, dim3(grid), dim3(kThreads), 0, s, d_jobs, d_work, nwork, d_status);
 }
 
 }  // namespace azk

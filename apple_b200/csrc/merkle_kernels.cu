@@ -561,12 +561,11 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) tree_tiles_kernel(cons
   __shared__ TreeJob job;
   const uint2 w = work[blockIdx.x];
   fetch_job(job, jobs + w.x);
-  // Launched before the kernel ahead of it in the stream has ended (launch_tiles): up
+  // Launched before the kernel ahead of it in the stream has ended (launch_kind): up
   // to here only the work list and the job were read, which no kernel writes; layers,
   // challenge, transcript, nodes and counters are touched once that kernel's memory is
   // complete.
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  dependent_begin();
   tree_tile_body<KIND, THREADS>(job, w.y);
 }
 
@@ -649,24 +648,6 @@ static uint32_t resident_grid(K kernel, int threads, size_t smem, uint32_t nwork
   return (uint32_t)(g < nwork ? g : nwork);
 }
 
-// A dependent launch: the commit launches of a fold chain follow one another, and
-// the launch's own latency overlaps the end of the kernel before it (which waits for
-// the last arriver's climb with most SMs idle).
-template <uint32_t KIND, int THREADS>
-static cudaError_t launch_tiles(const TreeJob* d_jobs, const uint2* d_work, uint32_t nwork, size_t smem, cudaStream_t s) {
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t c{};
-  c.gridDim = dim3(nwork);
-  c.blockDim = dim3(THREADS);
-  c.dynamicSmemBytes = smem;
-  c.stream = s;
-  c.attrs = &at;
-  c.numAttrs = 1;
-  return cudaLaunchKernelEx(&c, tree_tiles_kernel<KIND, THREADS>, d_jobs, d_work);
-}
-
 template <uint32_t KIND>
 static cudaError_t launch_kind(const TreeJob* d_jobs, const uint2* d_work, uint32_t nwork, uint32_t max_tile_log, uint32_t threads, uint32_t* queue,
                                cudaStream_t s) {
@@ -680,9 +661,11 @@ static cudaError_t launch_kind(const TreeJob* d_jobs, const uint2* d_work, uint3
       tree_queue_kernel<KIND, 256><<<resident_grid(tree_queue_kernel<KIND, 256>, 256, smem, nwork), 256, smem, s>>>(d_jobs, d_work, nwork, queue);
     return cudaGetLastError();
   }
-  if (threads == 128) return launch_tiles<KIND, 128>(d_jobs, d_work, nwork, smem, s);
-  if (threads == 512) return launch_tiles<KIND, 512>(d_jobs, d_work, nwork, smem, s);
-  return launch_tiles<KIND, 256>(d_jobs, d_work, nwork, smem, s);
+  // the commit launches of a fold chain follow one another, each ending in the last
+  // arriver's climb with most SMs idle
+  if (threads == 128) return launch_dependent(tree_tiles_kernel<KIND, 128>, dim3(nwork), dim3(128), smem, s, d_jobs, d_work);
+  if (threads == 512) return launch_dependent(tree_tiles_kernel<KIND, 512>, dim3(nwork), dim3(512), smem, s, d_jobs, d_work);
+  return launch_dependent(tree_tiles_kernel<KIND, 256>, dim3(nwork), dim3(256), smem, s, d_jobs, d_work);
 }
 
 cudaError_t launch_tree_jobs(const TreeJob* d_jobs, const uint2* d_work, uint32_t nwork, uint32_t max_tile_log, uint32_t kind, uint32_t threads,

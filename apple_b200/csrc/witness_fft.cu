@@ -249,6 +249,7 @@ __device__ __forceinline__ Val<W> conv_input(const WitnessConv& a, uint32_t colu
 template <int W, int STEP, uint32_t TL>
 __global__ void __launch_bounds__(kThreads) conv_high_kernel(const WitnessConv a) {
   constexpr uint32_t kTile = 1u << TL;
+  dependent_begin();
   extern __shared__ __align__(16) uint8_t smem[];
   Val<W>* sm = reinterpret_cast<Val<W>*>(smem);
   const uint32_t m = a.lm - TL, c = TL - m;
@@ -291,6 +292,7 @@ __global__ void __launch_bounds__(kThreads) conv_high_kernel(const WitnessConv a
 template <int W, uint32_t TL>
 __global__ void __launch_bounds__(kThreads) conv_low_kernel(const WitnessConv a) {
   constexpr uint32_t kTile = 1u << TL;
+  dependent_begin();
   extern __shared__ __align__(16) uint8_t smem[];
   Val<W>* sm = reinterpret_cast<Val<W>*>(smem);
   const uint64_t base = (uint64_t)blockIdx.x << TL;
@@ -320,6 +322,7 @@ __global__ void __launch_bounds__(kThreads) conv_low_kernel(const WitnessConv a)
 template <int W, uint32_t TL>
 __global__ void __launch_bounds__(kThreads) conv_out_kernel(const WitnessConv a) {
   constexpr uint32_t kTile = 1u << TL;
+  dependent_begin();
   extern __shared__ __align__(16) uint8_t smem[];
   Val<W>* sm = reinterpret_cast<Val<W>*>(smem);
   const uint32_t m = a.lm - TL, c = TL - m;
@@ -363,6 +366,7 @@ __device__ __forceinline__ Val<W> cheb_value(const WitnessConv& a, const uint8_t
 }
 template <int W>
 __global__ void __launch_bounds__(256) line_levels_kernel(const WitnessConv a, uint32_t lw, uint32_t k, uint32_t first) {
+  dependent_begin();
   uint8_t* c = a.c + blockIdx.y * a.c_stride;
   const uint64_t w = 1ull << lw, n = 1ull << (a.lm - 1);
   const uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -432,6 +436,7 @@ __global__ void __launch_bounds__(256) line_levels_kernel(const WitnessConv a, u
 template <int W>
 __global__ void __launch_bounds__(512) line_out_kernel(const WitnessConv a, uint32_t lt, uint32_t first, uint4* __restrict__ out) {
   extern __shared__ __align__(16) uint8_t smem[];
+  dependent_begin();
   const uint64_t n = 1ull << (a.lm - 1);
   const uint32_t T = 1u << lt;
   const uint64_t base = (uint64_t)blockIdx.x << lt;
@@ -475,10 +480,10 @@ template <int W, int STEP, uint32_t TL>
 cudaError_t run_conv_tiles(const WitnessConv& a, uint32_t columns, uint32_t outs, cudaStream_t s) {
   const uint32_t tiles = 1u << (a.lm - TL);
   const size_t smem = (size_t)4 * W << TL;
-  conv_high_kernel<W, STEP, TL><<<dim3(tiles, columns), kThreads, smem, s>>>(a);
-  conv_low_kernel<W, TL><<<dim3(tiles, columns, outs), kThreads, smem, s>>>(a);
-  if (STEP != kTable) conv_out_kernel<W, TL><<<dim3(tiles, columns, outs), kThreads, smem, s>>>(a);
-  return cudaGetLastError();
+  cudaError_t e = launch_dependent(conv_high_kernel<W, STEP, TL>, dim3(tiles, columns), dim3(kThreads), smem, s, a);
+  if (e == cudaSuccess) e = launch_dependent(conv_low_kernel<W, TL>, dim3(tiles, columns, outs), dim3(kThreads), smem, s, a);
+  if (e == cudaSuccess && STEP != kTable) e = launch_dependent(conv_out_kernel<W, TL>, dim3(tiles, columns, outs), dim3(kThreads), smem, s, a);
+  return e;
 }
 template <int W, int STEP>
 cudaError_t run_conv(const WitnessConv& a, uint32_t columns, uint32_t outs, cudaStream_t s) {
@@ -498,12 +503,12 @@ cudaError_t line_basis(const WitnessConv& a, uint32_t first, uint4* out, uint64_
   for (uint32_t ls = ln; ls > lt;) {
     const uint32_t k = ls - lt - 1 < (uint32_t)kLineK ? ls - lt - 1 : kLineK, lw = ls - k;
     const uint64_t threads = (n >> ls) * ((1ull << lw) / 2 + 1);
-    line_levels_kernel<W><<<dim3((unsigned)((threads + 255) / 256), columns), 256, 0, s>>>(a, lw, k, first);
+    const cudaError_t e = launch_dependent(line_levels_kernel<W>, dim3((unsigned)((threads + 255) / 256), columns), dim3(256), 0, s, a, lw, k, first);
+    if (e != cudaSuccess) return e;
     first = 0;
     ls = lw - 1;
   }
-  line_out_kernel<W><<<(unsigned)(capacity >> lt), 512, (size_t)columns * 4 * W << lt, s>>>(a, lt, first, out);
-  return cudaGetLastError();
+  return launch_dependent(line_out_kernel<W>, dim3((unsigned)(capacity >> lt)), dim3(512), (size_t)columns * 4 * W << lt, s, a, lt, first, out);
 }
 
 template <int W>
