@@ -131,6 +131,68 @@ __device__ __forceinline__ void pair_f1600(uint32_t (&a)[25], uint32_t q) {
   }
 }
 
+// The one-block digest of azk_keccak.cuh (keccak_digest) by a pair: the first round
+// without the zero lanes, the last without what its row 0 does not need.
+template <uint32_t NZ, int I>
+__device__ __forceinline__ void pair_rho_pi_first_lane(const uint32_t (&a)[25], const uint32_t (&c)[5], const uint32_t (&r1)[5], const uint32_t (&d)[5],
+                                                       uint32_t (&b)[25], uint32_t q) {
+  constexpr int x = I % 5, r = RhoPi<I>::rho;
+  uint32_t t;
+  if constexpr ((NZ >> I) & 1u) t = lop3_xor3(a[I], c[(x + 4) % 5], r1[(x + 1) % 5]);
+  else t = d[x];
+  if constexpr (r & 1) {
+    t = __shfl_xor_sync(0xffffffffu, t, 1);
+    t = __funnelshift_l(t, t, (uint32_t)((r + 1) / 2) - q);
+  } else if constexpr (r != 0) {
+    t = __funnelshift_l(t, t, r / 2);
+  }
+  b[RhoPi<I>::dst] = t;
+}
+template <uint32_t NZ, int... Is>
+__device__ __forceinline__ void pair_rho_pi_first(const uint32_t (&a)[25], const uint32_t (&c)[5], const uint32_t (&r1)[5], const uint32_t (&d)[5],
+                                                  uint32_t (&b)[25], uint32_t q, LaneSeq<Is...>) {
+  (pair_rho_pi_first_lane<NZ, Is>(a, c, r1, d, b, q), ...);
+}
+template <uint32_t NZ>
+__device__ __forceinline__ uint4 pair_digest(uint32_t (&a)[25], uint32_t q) {
+  uint32_t c[5], r1[5], d[5], b[25];
+#pragma unroll
+  for (int x = 0; x < 5; x++) {
+    c[x] = 0;
+#pragma unroll
+    for (int i = x; i < 25; i += 5)
+      if ((NZ >> i) & 1u) c[x] ^= a[i];
+  }
+#pragma unroll
+  for (int x = 0; x < 5; x++) {
+    const uint32_t p = __shfl_xor_sync(0xffffffffu, c[x], 1);
+    r1[x] = __funnelshift_l(p, p, 1u - q);
+  }
+#pragma unroll
+  for (int x = 0; x < 5; x++) d[x] = c[(x + 4) % 5] ^ r1[(x + 1) % 5];
+  pair_rho_pi_first<NZ>(a, c, r1, d, b, q, LaneSeq<1, 4, 8, 10, 12, 13, 14, 15, 16, 17, 18, 22, 0, 2, 3, 5, 6, 7, 9, 11, 19, 20, 21, 23, 24>{});
+#pragma unroll
+  for (int y = 0; y < 25; y += 5) {
+#pragma unroll
+    for (int x = 0; x < 5; x++) a[y + x] = lop3_chi(b[y + x], b[y + (x + 1) % 5], b[y + (x + 2) % 5]);
+  }
+  a[0] ^= split_rc(0, q);
+#pragma unroll 1
+  for (int r = 1; r < 23; r += 2) {
+    pair_round(a, q, split_rc(r, q));
+    pair_round(a, q, split_rc(r + 1, q));
+  }
+#pragma unroll
+  for (int x = 0; x < 5; x++) c[x] = lop3_xor3(lop3_xor3(a[x], a[x + 5], a[x + 10]), a[x + 15], a[x + 20]);
+#pragma unroll
+  for (int x = 0; x < 5; x++) {
+    const uint32_t p = __shfl_xor_sync(0xffffffffu, c[x], 1);
+    r1[x] = __funnelshift_l(p, p, 1u - q);
+  }
+  pair_rho_pi(a, c, r1, b, q, LaneSeq<12, 18, 0, 6, 24>{});
+  return make_uint4(lop3_chi(b[0], b[1], b[2]) ^ split_rc(23, q), lop3_chi(b[1], b[2], b[3]), lop3_chi(b[2], b[3], b[4]), lop3_chi(b[3], b[4], b[0]));
+}
+
 // Split form of small padding constants: suffix 0x06 or 0x01 in the lowest byte of
 // a lane, 0x80 in its highest byte.
 __device__ __forceinline__ uint32_t pair_suffix(uint32_t suffix, uint32_t q) {
@@ -162,14 +224,11 @@ __device__ __forceinline__ ulonglong2 pair_join_digest(uint4 v, uint32_t q) {
 // SHA3-256 of two digests (a Merkle parent), all in split form.
 __device__ __forceinline__ uint4 pair_hash_parent(uint4 l, uint4 r, uint32_t q) {
   uint32_t a[25];
-#pragma unroll
-  for (int i = 0; i < 25; i++) a[i] = 0;
   a[0] = l.x, a[1] = l.y, a[2] = l.z, a[3] = l.w;
   a[4] = r.x, a[5] = r.y, a[6] = r.z, a[7] = r.w;
   a[8] = pair_suffix(0x06, q);
   a[16] = pair_pad_end(q);
-  pair_f1600(a, q);
-  return make_uint4(a[0], a[1], a[2], a[3]);
+  return pair_digest<kLanes64>(a, q);
 }
 
 // ---------------------------------------------------------------------------

@@ -61,17 +61,17 @@ __device__ __forceinline__ void hash_message(const uint8_t* p, uint32_t len, uin
   if (len == 136) {
     keccak_f1600(a);
     a[0] ^= suffix;
+    a[16] ^= kPadEnd;
+    keccak_digest<kLanesAll>(a, out);
   } else {
     uint32_t lane = len >> 3;
     uint64_t v = (uint64_t)suffix << (8 * (len & 7));
 #pragma unroll
     for (uint32_t i = 0; i < 17; i++)
       if (i == lane) a[i] ^= v;
+    a[16] ^= kPadEnd;
+    keccak_digest<kLanesRate>(a, out);
   }
-  a[16] ^= kPadEnd;
-  keccak_f1600(a);
-#pragma unroll
-  for (int i = 0; i < 4; i++) out[i] = a[i];
 }
 
 }  // namespace azk

@@ -69,6 +69,29 @@ __device__ __forceinline__ uint4 folded_value(const TreeJob& job, uint64_t e, co
   return make_uint4(r.a, r.b, r.c, r.d);
 }
 
+// A raw message and its suffix into the first LANES (9, messages below 72 bytes, or
+// 17) of a zero state.  A compare, a select and an XOR for each lane of the rate took
+// 0.5 % of a tree of 2^22 64-byte leaves.
+template <uint32_t LANES>
+__device__ __forceinline__ void raw_setup(const TreeJob& job, const uint8_t* p, uint64_t (&a)[25]) {
+  const uint32_t full = job.len >> 3, rem = job.len & 7;
+  const UnalignedWords u(p);
+  uint64_t tail = (uint64_t)job.suffix << (8 * rem);
+  if (rem) tail |= u.word(full, rem);
+  if (job.aligned8) {
+#pragma unroll
+    for (uint32_t i = 0; i < LANES; i++)
+      if (i < full) a[i] = __ldg(reinterpret_cast<const uint64_t*>(p) + i);
+  } else {
+#pragma unroll
+    for (uint32_t i = 0; i < LANES; i++)
+      if (i < full) a[i] = u.word(i, 8);
+  }
+#pragma unroll
+  for (uint32_t i = 0; i < LANES; i++)
+    if (i == full) a[i] = tail;
+}
+
 // Sets up the sponge input of one leaf (message lanes, suffix and end padding)
 // and returns how many permutations it takes (2 for a 136-byte raw leaf).
 template <uint32_t KIND>
@@ -105,13 +128,10 @@ __device__ __forceinline__ uint32_t leaf_setup(const TreeJob& job, uint64_t leaf
     a[16] = kPadEnd;
     return 1;
   } else {
-    xor_message(a, job.raw + leaf * job.stride, job.len, job.aligned8 != 0);
+    const uint8_t* const p = job.raw + leaf * job.stride;
+    if (job.len < 72) raw_setup<9>(job, p, a);
+    else raw_setup<17>(job, p, a);
     if (job.len == 136) return 2;
-    const uint32_t lane = job.len >> 3;
-    const uint64_t v = (uint64_t)job.suffix << (8 * (job.len & 7));
-#pragma unroll
-    for (uint32_t i = 0; i < 17; i++)
-      if (i == lane) a[i] ^= v;
     a[16] ^= kPadEnd;
     return 1;
   }
@@ -173,54 +193,45 @@ __device__ __noinline__ void subtree_phase(const TreeJob& job, uint32_t items, u
   //   item:  0  1  -  2  3  -  -
   const uint32_t steps = h == 2 ? 7 : (h == 1 ? 3 : 1);
   for (uint32_t j = threadIdx.x; j < groups; j += THREADS) {
-    uint64_t X[4] = {0, 0, 0, 0}, Y[4] = {0, 0, 0, 0}, P[4] = {0, 0, 0, 0};
+    // A pair's right child is always the digest of the step before it; its left child
+    // waits in this thread's place of `out` (a leaf) or in the level it was stored to
+    // (the first pair): the memory pipe is idle, while carrying both in registers and
+    // selecting per step cost the integer pipe 1 % of all its instructions.
+    ulonglong2* const mine = reinterpret_cast<ulonglong2*>(out) + 2 * j;
+    uint64_t d[4] = {0, 0, 0, 0};
 #pragma unroll 1
     for (uint32_t k = 0; k < steps; k++) {
       const bool pair = (h == 2) ? (k == 2 || k == 5 || k == 6) : (h == 1 && k == 2);
       const uint32_t item = k < 2 ? k : k - 1;  // leaf steps only (h == 2: k = 0, 1, 3, 4)
       const uint64_t leaf = idx0 + (uint64_t)j * (1u << h) + item;
-      uint64_t d[4];
       if (!pair && KIND == kLeafDigest) {
         ld_dig_cg(digests + 4 * ((uint64_t)j * (1u << h) + item), d);
       } else {
         uint64_t a[25];
 #pragma unroll
-        for (int i = 0; i < 25; i++) a[i] = 0;
-        uint32_t perms = 1;
+        for (int i = 0; i < 17; i++) a[i] = 0;
         if (pair) {
-          const bool top = (h == 2 && k == 6);
+          const ulonglong2* const l = k == 6 ? reinterpret_cast<const ulonglong2*>(l1 + 8 * j) : mine;
+          const ulonglong2 l0 = l[0], l1v = l[1];
+          a[0] = l0.x, a[1] = l0.y, a[2] = l1v.x, a[3] = l1v.y;
 #pragma unroll
-          for (int i = 0; i < 4; i++) {
-            a[i] = top ? P[i] : X[i];
-            a[4 + i] = Y[i];
-          }
+          for (int i = 0; i < 4; i++) a[4 + i] = d[i];
           a[8] = 0x06;
           a[16] = kPadEnd;
-        } else {
-          perms = leaf_setup<KIND>(job, leaf, ch, a);
-        }
-#pragma unroll 1
-        for (uint32_t b = 0; b < perms; b++) {
-          if (b == 1) {
-            a[0] ^= job.suffix;
-            a[16] ^= kPadEnd;
-          }
-          keccak_f1600(a);
-        }
+        } else if (leaf_setup<KIND>(job, leaf, ch, a) == 2) {  // a full block, then the padding's own
 #pragma unroll
-        for (int i = 0; i < 4; i++) d[i] = a[i];
+          for (int i = 17; i < 25; i++) a[i] = 0;
+          keccak_f1600(a);
+          a[0] ^= job.suffix;
+          a[16] ^= kPadEnd;
+          keccak_digest<kLanesAll>(a, d);
+          goto hashed;
+        }
+        keccak_digest<KIND == kLeafRaw ? kLanesRate : kLanes64>(a, d);
+      hashed:
         if (!pair && job.leaf_digests) st_dig(job.leaf_digests + 4 * leaf, d);
       }
-      // route the step's digest
-      const bool toX = (h == 2) ? (k == 0 || k == 3) : (h == 1 && k == 0);
-      const bool toY = (h == 2) ? (k == 1 || k == 4 || k == 5) : (h == 1 && k == 1);
-      const bool toP = (h == 2 && k == 2);
-#pragma unroll
-      for (int i = 0; i < 4; i++) {
-        X[i] = toX ? d[i] : X[i];
-        Y[i] = toY ? d[i] : Y[i];
-        P[i] = toP ? d[i] : P[i];
-      }
+      if (steps > 1 && (k == 0 || k == 3)) mine[0] = make_ulonglong2(d[0], d[1]), mine[1] = make_ulonglong2(d[2], d[3]);
       if (h == 2 && k == 2) st_dig(l1 + 8 * j, d);
       if (h == 2 && k == 5) st_dig(l1 + 8 * j + 4, d);
       if (h == 2 && k == 6) st_dig(l2 + 4 * j, d);
@@ -303,17 +314,14 @@ __device__ __forceinline__ uint4 pair_leaf(const TreeJob& job, uint64_t leaf, bo
         if (m < 8) a[2 * m + 1] = w1;
       }
     }
-    const bool two = KIND == kLeafRaw && job.len == 136;  // a full block, then the padding's own
-    if (!two) a[16] ^= pair_pad_end(q);
-#pragma unroll 1
-    for (uint32_t b = 0; b < (two ? 2u : 1u); b++) {
-      if (b == 1) {
-        a[0] ^= pair_suffix(job.suffix, q);
-        a[16] ^= pair_pad_end(q);
-      }
+    if (KIND == kLeafRaw && job.len == 136) {  // a full block, then the padding's own
       pair_f1600(a, q);
+      a[0] ^= pair_suffix(job.suffix, q);
+      a[16] ^= pair_pad_end(q);
+      return pair_digest<kLanesAll>(a, q);
     }
-    return make_uint4(a[0], a[1], a[2], a[3]);
+    a[16] ^= pair_pad_end(q);
+    return pair_digest<KIND == kLeafRaw ? kLanesRate : KIND == kLeafQM31x4 || KIND == kLeafFoldx4 ? kLanes64 : kLanes16>(a, q);
   }
 }
 
