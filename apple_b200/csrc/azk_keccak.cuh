@@ -238,15 +238,19 @@ __device__ __forceinline__ void keccak_last_round(const uint64_t (&a)[25], uint6
   for (int x = 0; x < 4; x++) out[x] = chi_64(b[x], b[x + 1], b[(x + 2) % 5]);
   out[0] ^= rc;
 }
-template <uint32_t NZ>
-__device__ __forceinline__ void keccak_digest(uint64_t (&a)[25], uint64_t (&out)[4]) {
-  keccak_first_round<NZ>(a, kKeccakRC[0]);
+// Rounds 1 .. 23.
+__device__ __forceinline__ void keccak_digest_rest(uint64_t (&a)[25], uint64_t (&out)[4]) {
 #pragma unroll 1
   for (int r = 1; r < 23; r += 2) {
     keccak_round(a, kKeccakRC[r]);
     keccak_round(a, kKeccakRC[r + 1]);
   }
   keccak_last_round(a, kKeccakRC[23], out);
+}
+template <uint32_t NZ>
+__device__ __forceinline__ void keccak_digest(uint64_t (&a)[25], uint64_t (&out)[4]) {
+  keccak_first_round<NZ>(a, kKeccakRC[0]);
+  keccak_digest_rest(a, out);
 }
 #endif
 

@@ -25,30 +25,41 @@ namespace azk {
 // (r even), or the two words exchanged and rotated by (r + 1) / 2 (the new even
 // word) and (r - 1) / 2 (the new odd word).
 // ---------------------------------------------------------------------------
-// Even bits of x to the low half, odd bits to the high half (and back).
-__host__ __device__ __forceinline__ uint32_t unshuffle32(uint32_t x) {
+// Even bits of each 16-bit half of x to its low byte, odd bits to its high byte (and
+// back); the bytes of both words of a lane then move in two permutes.
+__host__ __device__ __forceinline__ uint32_t unshuffle16(uint32_t x) {
   uint32_t t;
   t = (x ^ (x >> 1)) & 0x22222222u; x ^= t ^ (t << 1);
   t = (x ^ (x >> 2)) & 0x0C0C0C0Cu; x ^= t ^ (t << 2);
   t = (x ^ (x >> 4)) & 0x00F000F0u; x ^= t ^ (t << 4);
-  t = (x ^ (x >> 8)) & 0x0000FF00u; x ^= t ^ (t << 8);
   return x;
 }
-__host__ __device__ __forceinline__ uint32_t shuffle32(uint32_t x) {
+__host__ __device__ __forceinline__ uint32_t shuffle16(uint32_t x) {
   uint32_t t;
-  t = (x ^ (x >> 8)) & 0x0000FF00u; x ^= t ^ (t << 8);
   t = (x ^ (x >> 4)) & 0x00F000F0u; x ^= t ^ (t << 4);
   t = (x ^ (x >> 2)) & 0x0C0C0C0Cu; x ^= t ^ (t << 2);
   t = (x ^ (x >> 1)) & 0x22222222u; x ^= t ^ (t << 1);
   return x;
+}
+// Bytes 0..3 are a's, 4..7 are b's; digit k of `sel` picks the result's byte k.
+template <uint32_t SEL>
+__host__ __device__ __forceinline__ uint32_t pick_bytes(uint32_t a, uint32_t b) {
+#if defined(__CUDA_ARCH__)
+  return __byte_perm(a, b, SEL);
+#else
+  const uint64_t v = ((uint64_t)b << 32) | a;
+  uint32_t r = 0;
+  for (int k = 0; k < 4; k++) r |= (uint32_t)((v >> (8 * ((SEL >> (4 * k)) & 7))) & 0xFF) << (8 * k);
+  return r;
+#endif
 }
 __host__ __device__ __forceinline__ void split64(uint64_t v, uint32_t& even, uint32_t& odd) {
-  const uint32_t lo = unshuffle32((uint32_t)v), hi = unshuffle32((uint32_t)(v >> 32));
-  even = (lo & 0xFFFFu) | (hi << 16);
-  odd = (lo >> 16) | (hi & 0xFFFF0000u);
+  const uint32_t lo = unshuffle16((uint32_t)v), hi = unshuffle16((uint32_t)(v >> 32));
+  even = pick_bytes<0x6420>(lo, hi);
+  odd = pick_bytes<0x7531>(lo, hi);
 }
 __host__ __device__ __forceinline__ uint64_t join64(uint32_t even, uint32_t odd) {
-  const uint32_t lo = shuffle32((even & 0xFFFFu) | (odd << 16)), hi = shuffle32((even >> 16) | (odd & 0xFFFF0000u));
+  const uint32_t lo = shuffle16(pick_bytes<0x5140>(even, odd)), hi = shuffle16(pick_bytes<0x7362>(even, odd));
   return ((uint64_t)hi << 32) | lo;
 }
 

@@ -207,9 +207,12 @@ __device__ __noinline__ void subtree_phase(const TreeJob& job, uint32_t items, u
       if (!pair && KIND == kLeafDigest) {
         ld_dig_cg(digests + 4 * ((uint64_t)j * (1u << h) + item), d);
       } else {
+        constexpr bool kValue = KIND == kLeafQM31 || KIND == kLeafFold || KIND == kLeafFoldQ;  // one 16-byte value
         uint64_t a[25];
+        if (!kValue) {
 #pragma unroll
-        for (int i = 0; i < 17; i++) a[i] = 0;
+          for (int i = 0; i < 17; i++) a[i] = 0;
+        }
         if (pair) {
           const ulonglong2* const l = k == 6 ? reinterpret_cast<const ulonglong2*>(l1 + 8 * j) : mine;
           const ulonglong2 l0 = l[0], l1v = l[1];
@@ -218,6 +221,7 @@ __device__ __noinline__ void subtree_phase(const TreeJob& job, uint32_t items, u
           for (int i = 0; i < 4; i++) a[4 + i] = d[i];
           a[8] = 0x06;
           a[16] = kPadEnd;
+          if (kValue) keccak_first_round<kLanes64>(a, kKeccakRC[0]);
         } else if (leaf_setup<KIND>(job, leaf, ch, a) == 2) {  // a full block, then the padding's own
 #pragma unroll
           for (int i = 17; i < 25; i++) a[i] = 0;
@@ -226,8 +230,11 @@ __device__ __noinline__ void subtree_phase(const TreeJob& job, uint32_t items, u
           a[16] ^= kPadEnd;
           keccak_digest<kLanesAll>(a, d);
           goto hashed;
+        } else if (kValue) {
+          keccak_first_round<kLanes16>(a, kKeccakRC[0]);
         }
-        keccak_digest<KIND == kLeafRaw ? kLanesRate : kLanes64>(a, d);
+        if (!kValue) keccak_first_round<KIND == kLeafRaw ? kLanesRate : kLanes64>(a, kKeccakRC[0]);
+        keccak_digest_rest(a, d);
       hashed:
         if (!pair && job.leaf_digests) st_dig(job.leaf_digests + 4 * leaf, d);
       }
