@@ -63,12 +63,7 @@ __host__ __device__ __forceinline__ uint64_t join64(uint32_t even, uint32_t odd)
   return ((uint64_t)hi << 32) | lo;
 }
 
-// ---------------------------------------------------------------------------
-// A pair of neighbouring lanes per permutation.  Lane parity q = 0 holds the 25
-// even words, q = 1 the 25 odd words.  Every lane of the warp takes part (the
-// exchanges are full-warp shuffles), so callers keep warps converged and clamp the
-// indices of lanes without work.
-// ---------------------------------------------------------------------------
+// Round constants in split form.
 struct alignas(8) SplitRC {
   uint32_t even, odd;
 };
@@ -91,6 +86,105 @@ constexpr KeccakSplitRC keccak_split_rc() {
   return r;
 }
 __constant__ static const KeccakSplitRC kKeccakSplitRC = keccak_split_rc();
+
+// ---------------------------------------------------------------------------
+// One thread per permutation, in split form: theta's rotation by one moves a word
+// (5 shifts a round instead of 10) and so does lane 1's, so a round is 174
+// instructions instead of 180.  For 16-byte messages and digests that stay in split
+// form; splitting and joining a digest costs 104.
+// ---------------------------------------------------------------------------
+struct SplitDigest {
+  uint4 even, odd;  // four lanes
+};
+template <int R>
+__device__ __forceinline__ void split_rotl(uint32_t e, uint32_t o, uint32_t& re, uint32_t& ro) {
+  if constexpr (R & 1) {
+    re = __funnelshift_l(o, o, (R + 1) / 2);
+    ro = __funnelshift_l(e, e, R / 2);
+  } else {
+    re = __funnelshift_l(e, e, R / 2);
+    ro = __funnelshift_l(o, o, R / 2);
+  }
+}
+// D of column x is c[x - 1] ^ rotl(c[x + 1], 1): r[x] holds the rotated even words
+// (the rotated odd words are ce).  Lanes outside NZ are zero.
+template <uint32_t NZ, int I>
+__device__ __forceinline__ void split_rho_pi_lane(const uint32_t (&e)[25], const uint32_t (&o)[25], const uint32_t (&ce)[5], const uint32_t (&co)[5],
+                                                  const uint32_t (&r)[5], uint32_t (&be)[25], uint32_t (&bo)[25]) {
+  constexpr int m = (I % 5 + 4) % 5, n = (I % 5 + 1) % 5;
+  uint32_t te, to;
+  if constexpr ((NZ >> I) & 1u) {
+    te = lop3_xor3(e[I], ce[m], r[n]);
+    to = lop3_xor3(o[I], co[m], ce[n]);
+  } else {
+    te = ce[m] ^ r[n];
+    to = co[m] ^ ce[n];
+  }
+  split_rotl<RhoPi<I>::rho>(te, to, be[RhoPi<I>::dst], bo[RhoPi<I>::dst]);
+}
+template <uint32_t NZ, int... Is>
+__device__ __forceinline__ void split_rho_pi(const uint32_t (&e)[25], const uint32_t (&o)[25], const uint32_t (&ce)[5], const uint32_t (&co)[5],
+                                             const uint32_t (&r)[5], uint32_t (&be)[25], uint32_t (&bo)[25], LaneSeq<Is...>) {
+  (split_rho_pi_lane<NZ, Is>(e, o, ce, co, r, be, bo), ...);
+}
+template <uint32_t NZ>
+__device__ __forceinline__ void split_columns(const uint32_t (&a)[25], uint32_t (&c)[5]) {
+#pragma unroll
+  for (int x = 0; x < 5; x++) {
+    if constexpr (NZ == kLanesAll) {
+      c[x] = lop3_xor3(lop3_xor3(a[x], a[x + 5], a[x + 10]), a[x + 15], a[x + 20]);
+    } else {
+      c[x] = 0;
+#pragma unroll
+      for (int i = x; i < 25; i += 5)
+        if ((NZ >> i) & 1u) c[x] ^= a[i];
+    }
+  }
+}
+template <uint32_t NZ>
+__device__ __forceinline__ void split_round(uint32_t (&e)[25], uint32_t (&o)[25], int round) {
+  uint32_t ce[5], co[5], r[5], be[25], bo[25];
+  split_columns<NZ>(e, ce);
+  split_columns<NZ>(o, co);
+#pragma unroll
+  for (int x = 0; x < 5; x++) r[x] = __funnelshift_l(co[x], co[x], 1);
+  split_rho_pi<NZ>(e, o, ce, co, r, be, bo, LaneSeq<0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 17, 18, 19, 20, 21, 22, 23, 24>{});
+#pragma unroll
+  for (int y = 0; y < 25; y += 5) {
+#pragma unroll
+    for (int x = 0; x < 5; x++) {
+      e[y + x] = lop3_chi(be[y + x], be[y + (x + 1) % 5], be[y + (x + 2) % 5]);
+      o[y + x] = lop3_chi(bo[y + x], bo[y + (x + 1) % 5], bo[y + (x + 2) % 5]);
+    }
+  }
+  e[0] ^= kKeccakSplitRC.w[round].even;
+  o[0] ^= kKeccakSplitRC.w[round].odd;
+}
+// Rounds 1 .. 23 of a one-block digest (see keccak_digest).
+__device__ __forceinline__ SplitDigest split_digest_rest(uint32_t (&e)[25], uint32_t (&o)[25]) {
+#pragma unroll 1
+  for (int i = 1; i < 23; i += 2) {
+    split_round<kLanesAll>(e, o, i);
+    split_round<kLanesAll>(e, o, i + 1);
+  }
+  uint32_t ce[5], co[5], r[5], be[25], bo[25];
+  split_columns<kLanesAll>(e, ce);
+  split_columns<kLanesAll>(o, co);
+#pragma unroll
+  for (int x = 0; x < 5; x++) r[x] = __funnelshift_l(co[x], co[x], 1);
+  split_rho_pi<kLanesAll>(e, o, ce, co, r, be, bo, LaneSeq<0, 6, 12, 18, 24>{});
+  return {make_uint4(lop3_chi(be[0], be[1], be[2]) ^ kKeccakSplitRC.w[23].even, lop3_chi(be[1], be[2], be[3]), lop3_chi(be[2], be[3], be[4]),
+                     lop3_chi(be[3], be[4], be[0])),
+          make_uint4(lop3_chi(bo[0], bo[1], bo[2]) ^ kKeccakSplitRC.w[23].odd, lop3_chi(bo[1], bo[2], bo[3]), lop3_chi(bo[2], bo[3], bo[4]),
+                     lop3_chi(bo[3], bo[4], bo[0]))};
+}
+
+// ---------------------------------------------------------------------------
+// A pair of neighbouring lanes per permutation.  Lane parity q = 0 holds the 25
+// even words, q = 1 the 25 odd words.  Every lane of the warp takes part (the
+// exchanges are full-warp shuffles), so callers keep warps converged and clamp the
+// indices of lanes without work.
+// ---------------------------------------------------------------------------
 // One uniform 8-byte load and a select: loads indexed or predicated by the lane's
 // parity cost a round 10 cycles.
 __device__ __forceinline__ uint32_t split_rc(int r, uint32_t q) {
