@@ -38,7 +38,12 @@ namespace {
 // tiles, 255 with short ones; of 2^14: 246 and 116; of 2^18 495 and no strided tile
 // with 64-byte rows).
 constexpr uint32_t kLongTile = 12, kShortTile = 10, kShortLog = 18;
-constexpr int kThreads = 256;
+// Threads of a tile's CTA.  A long tile's stages are chains of shared-memory round
+// trips in few CTAs (13 of 64 warps resident at 256 threads): lifted columns of 2^21
+// 1032 us with 256, 968 with 512, 972 with 1024; of 2^18 234, 196 and 186; QM31 ones of 2^21
+// 3241, 3072 and 3544.  A short tile has work for 256.
+template <uint32_t TL>
+constexpr int kConvThreads = TL >= 12 ? 512 : 256;
 
 // W limbs per value: 2 (one CM31) or 4 (two).
 template <int W>
@@ -126,14 +131,14 @@ __device__ __forceinline__ uint32_t slot(uint32_t i) { return i ^ ((i >> 3) & 1u
 // col), two per shared-memory round trip.  Row bit j's block is (hi << (m-1-j)) +
 // (row >> (j+1)).  Starts and ends with the tile in shared memory and every thread
 // past a barrier.  top: row bits >= top are already done (forward) or not wanted.
-template <int W>
+template <int W, int THREADS>
 __device__ __forceinline__ void forward_stages(Val<W>* sm, uint32_t m, uint32_t top, uint32_t c, uint64_t hi, const uint2* __restrict__ roots) {
   const uint32_t T = 1u << (m + c);
   int j = (int)top - 1;
   for (; j >= 1; j -= 2) {
     const uint32_t p = (uint32_t)j + c;  // stages on local bits p and p - 1
     const uint32_t low = (1u << (p - 1)) - 1;
-    for (uint32_t k = threadIdx.x; k < T / 4; k += kThreads) {
+    for (uint32_t k = threadIdx.x; k < T / 4; k += THREADS) {
       const uint32_t e = ((k & ~low) << 2) | (k & low);
       const uint64_t b = (hi << (m - 1 - j)) + (e >> (c + j + 1));
       const uint2 t1 = __ldg(roots + b);
@@ -149,7 +154,7 @@ __device__ __forceinline__ void forward_stages(Val<W>* sm, uint32_t m, uint32_t 
     __syncthreads();
   }
   if (j == 0) {
-    for (uint32_t k = threadIdx.x; k < T / 2; k += kThreads) {
+    for (uint32_t k = threadIdx.x; k < T / 2; k += THREADS) {
       const uint32_t low = (1u << c) - 1, e = ((k & ~low) << 1) | (k & low);
       const uint2 t = __ldg(roots + (hi << (m - 1)) + (e >> (c + 1)));
       const uint32_t s0 = slot(e), s1 = slot(e | (1u << c));
@@ -160,12 +165,12 @@ __device__ __forceinline__ void forward_stages(Val<W>* sm, uint32_t m, uint32_t 
     __syncthreads();
   }
 }
-template <int W>
+template <int W, int THREADS>
 __device__ __forceinline__ void inverse_stages(Val<W>* sm, uint32_t m, uint32_t c, uint64_t hi, const uint2* __restrict__ roots) {
   const uint32_t T = 1u << (m + c);
   uint32_t j = 0;
   if (m & 1) {
-    for (uint32_t k = threadIdx.x; k < T / 2; k += kThreads) {
+    for (uint32_t k = threadIdx.x; k < T / 2; k += THREADS) {
       const uint32_t low = (1u << c) - 1, e = ((k & ~low) << 1) | (k & low);
       const uint2 t = __ldg(roots + (hi << (m - 1)) + (e >> (c + 1)));
       const uint32_t s0 = slot(e), s1 = slot(e | (1u << c));
@@ -179,7 +184,7 @@ __device__ __forceinline__ void inverse_stages(Val<W>* sm, uint32_t m, uint32_t 
   for (; j + 1 < m + 0u; j += 2) {
     const uint32_t p = j + 1 + c;  // stages on local bits p - 1, then p
     const uint32_t low = (1u << (p - 1)) - 1;
-    for (uint32_t k = threadIdx.x; k < T / 4; k += kThreads) {
+    for (uint32_t k = threadIdx.x; k < T / 4; k += THREADS) {
       const uint32_t e = ((k & ~low) << 2) | (k & low);
       const uint64_t b = (hi << (m - 2 - j)) + (e >> (c + j + 2));
       const uint2 t1 = __ldg(roots + b);
@@ -247,8 +252,9 @@ __device__ __forceinline__ Val<W> conv_input(const WitnessConv& a, uint32_t colu
 // The strided pass of the forward transform (stages above bit 12): inputs from
 // conv_input (zero from n on, so the first stage only copies), all 2n values to `t`.
 template <int W, int STEP, uint32_t TL>
-__global__ void __launch_bounds__(kThreads) conv_high_kernel(const WitnessConv a) {
+__global__ void __launch_bounds__(kConvThreads<TL>) conv_high_kernel(const WitnessConv a) {
   constexpr uint32_t kTile = 1u << TL;
+  constexpr int kThreads = kConvThreads<TL>;
   dependent_begin();
   extern __shared__ __align__(16) uint8_t smem[];
   Val<W>* sm = reinterpret_cast<Val<W>*>(smem);
@@ -281,7 +287,7 @@ __global__ void __launch_bounds__(kThreads) conv_high_kernel(const WitnessConv a
     }
   }
   __syncthreads();
-  forward_stages<W>(sm, m, m - 1, c, 0, a.roots);
+  forward_stages<W, kThreads>(sm, m, m - 1, c, 0, a.roots);
   uint8_t* t = static_cast<uint8_t*>(a.t) + blockIdx.y * a.t_stride;
   for (uint32_t L = threadIdx.x; L < kTile; L += kThreads)
     stv<W>(t, ((uint64_t)(L >> c) << TL) | col0 | (L & ((1u << c) - 1)), sm[slot(L)]);
@@ -290,8 +296,9 @@ __global__ void __launch_bounds__(kThreads) conv_high_kernel(const WitnessConv a
 // The low stages on contiguous tiles: forward, times the fixed sequence's transform
 // (blockIdx.z picks one of two), inverse, from `t` to u[z].
 template <int W, uint32_t TL>
-__global__ void __launch_bounds__(kThreads) conv_low_kernel(const WitnessConv a) {
+__global__ void __launch_bounds__(kConvThreads<TL>) conv_low_kernel(const WitnessConv a) {
   constexpr uint32_t kTile = 1u << TL;
+  constexpr int kThreads = kConvThreads<TL>;
   dependent_begin();
   extern __shared__ __align__(16) uint8_t smem[];
   Val<W>* sm = reinterpret_cast<Val<W>*>(smem);
@@ -299,7 +306,7 @@ __global__ void __launch_bounds__(kThreads) conv_low_kernel(const WitnessConv a)
   const uint8_t* t = static_cast<const uint8_t*>(a.t) + blockIdx.y * a.t_stride;
   for (uint32_t L = threadIdx.x; L < kTile; L += kThreads) sm[slot(L)] = ldv<W>(t, base + L);
   __syncthreads();
-  forward_stages<W>(sm, TL, TL, 0, blockIdx.x, a.roots);
+  forward_stages<W, kThreads>(sm, TL, TL, 0, blockIdx.x, a.roots);
   if (a.k[0] == nullptr) {  // a fixed sequence's own transform
     for (uint32_t L = threadIdx.x; L < kTile; L += kThreads) {
       const Val<W> v = sm[slot(L)];
@@ -313,15 +320,16 @@ __global__ void __launch_bounds__(kThreads) conv_low_kernel(const WitnessConv a)
     sm[s] = cmul(sm[s], __ldg(kf + ((base + L) ^ a.flip)));
   }
   __syncthreads();
-  inverse_stages<W>(sm, TL, 0, blockIdx.x, a.roots);
+  inverse_stages<W, kThreads>(sm, TL, 0, blockIdx.x, a.roots);
   uint8_t* u = static_cast<uint8_t*>(a.u[blockIdx.z]) + blockIdx.y * a.t_stride;
   for (uint32_t L = threadIdx.x; L < kTile; L += kThreads) stv<W>(u, base + L, sm[slot(L)]);
 }
 
 // The strided inverse pass; the wanted outputs to o[z].
 template <int W, uint32_t TL>
-__global__ void __launch_bounds__(kThreads) conv_out_kernel(const WitnessConv a) {
+__global__ void __launch_bounds__(kConvThreads<TL>) conv_out_kernel(const WitnessConv a) {
   constexpr uint32_t kTile = 1u << TL;
+  constexpr int kThreads = kConvThreads<TL>;
   dependent_begin();
   extern __shared__ __align__(16) uint8_t smem[];
   Val<W>* sm = reinterpret_cast<Val<W>*>(smem);
@@ -331,7 +339,7 @@ __global__ void __launch_bounds__(kThreads) conv_out_kernel(const WitnessConv a)
   for (uint32_t L = threadIdx.x; L < kTile; L += kThreads)
     sm[slot(L)] = ldv<W>(u, ((uint64_t)(L >> c) << TL) | col0 | (L & ((1u << c) - 1)));
   __syncthreads();
-  inverse_stages<W>(sm, m, c, 0, a.roots);
+  inverse_stages<W, kThreads>(sm, m, c, 0, a.roots);
   uint8_t* o = a.o[blockIdx.z] + blockIdx.y * a.o_stride;
   for (uint32_t L = threadIdx.x; L < kTile / 2; L += kThreads) {
     const uint64_t i = ((uint64_t)(L >> c) << TL) | col0 | (L & ((1u << c) - 1));
@@ -480,9 +488,9 @@ template <int W, int STEP, uint32_t TL>
 cudaError_t run_conv_tiles(const WitnessConv& a, uint32_t columns, uint32_t outs, cudaStream_t s) {
   const uint32_t tiles = 1u << (a.lm - TL);
   const size_t smem = (size_t)4 * W << TL;
-  cudaError_t e = launch_dependent(conv_high_kernel<W, STEP, TL>, dim3(tiles, columns), dim3(kThreads), smem, s, a);
-  if (e == cudaSuccess) e = launch_dependent(conv_low_kernel<W, TL>, dim3(tiles, columns, outs), dim3(kThreads), smem, s, a);
-  if (e == cudaSuccess && STEP != kTable) e = launch_dependent(conv_out_kernel<W, TL>, dim3(tiles, columns, outs), dim3(kThreads), smem, s, a);
+  cudaError_t e = launch_dependent(conv_high_kernel<W, STEP, TL>, dim3(tiles, columns), dim3(kConvThreads<TL>), smem, s, a);
+  if (e == cudaSuccess) e = launch_dependent(conv_low_kernel<W, TL>, dim3(tiles, columns, outs), dim3(kConvThreads<TL>), smem, s, a);
+  if (e == cudaSuccess && STEP != kTable) e = launch_dependent(conv_out_kernel<W, TL>, dim3(tiles, columns, outs), dim3(kConvThreads<TL>), smem, s, a);
   return e;
 }
 template <int W, int STEP>
