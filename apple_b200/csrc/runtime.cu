@@ -979,7 +979,7 @@ void azk_codeword_plan_destroy(azk_codeword_plan* p) { delete p; }
 // least 2^kWitnessFftLog take the fast convolutions, shorter ones the direct sum.
 // Columns of at least 2^kWitnessFftLog take the fast convolutions, shorter ones the
 // direct sum (two full QM31 columns on B200, direct / convolutions: 2^12 74 / 100 us,
-// 2^13 160 / 111 us, 2^14 425 / 116 us, 2^19 175,900 / 886 us).
+// 2^13 160 / 111 us, 2^14 425 / 116 us, 2^19 175,900 / 828 us).
 static constexpr uint32_t kWitnessMinLog = 11, kWitnessFftLog = 13;
 
 struct azk_witness_plan {

@@ -25,7 +25,7 @@
 // sequence's transform and the inverse stages are one kernel, so a convolution is
 // three passes over memory.  What bounds them is integer issue: about
 // 52 instructions per QM31 butterfly.  Two columns of 2^19 QM31 (lifted M31)
-// coefficients: 0.88 (0.36) ms, against 175.9 ms for the direct sum's O(n^2).
+// coefficients: 0.83 (0.34) ms, against 175.9 ms for the direct sum's O(n^2).
 #include "azk_field.cuh"
 #include "azk_internal.h"
 

@@ -460,9 +460,9 @@ void azk_batch_destroy(azk_batch* b);
  * For a domain of 2^log_size points (log_size 1...22): x and y monomial
  * coefficient columns (QM31, at most 2^(log_size-1) each, not both empty) become
  * the interleaved FFT-basis buffer [x0, y0, x1, y1, ...] of 2^log_size QM31 that
- * azk_pcs_prover_prove_coefficients / azk_codeword_plan_execute take.  Work grows
- * with the square of the longer column (the reference's dense matrix), without a
- * matrix in memory.  Non-canonical coefficients fail with
+ * azk_pcs_prover_prove_coefficients / azk_codeword_plan_execute take.  No matrix in
+ * memory: short columns by a direct sum (the dense matrix's work), longer ones by
+ * convolutions of n log n work.  Non-canonical coefficients fail with
  * AZK_ERR_INVALID_INPUT_LAYOUT; so does a resident output that overlaps a column. */
 typedef struct azk_witness_plan azk_witness_plan;
 azk_status azk_witness_plan_create(azk_ctx* ctx, uint32_t log_size, azk_witness_plan** out);
