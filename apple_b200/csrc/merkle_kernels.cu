@@ -54,6 +54,14 @@ __device__ __forceinline__ void leaf_digest(const TreeJob& job, uint64_t leaf, c
   }
 }
 
+// The challenge of a fold kind, read by every thread beside its first values: through
+// shared memory and a barrier ahead of them it cost each round 400 to 750 cycles.
+template <uint32_t KIND>
+__device__ __forceinline__ void fold_challenge(const TreeJob& job, uint32_t (&ch)[4]) {
+#pragma unroll
+  for (int k = 0; k < 4; k++) ch[k] = KIND == kLeafFold || KIND == kLeafFoldx4 || KIND == kLeafFoldQ ? __ldcg(job.fold_ch + k) : 0u;
+}
+
 // Value e of the layer that a fold kind produces.
 template <uint32_t KIND>
 __device__ __forceinline__ uint4 folded_value(const TreeJob& job, uint64_t e, const uint32_t (&ch)[4]) {
@@ -168,9 +176,9 @@ static size_t tree_smem_bytes(uint32_t max_tile_log, uint32_t threads) {
 // leaf, leaf, pair, pair), which keeps the kernel's code small enough for the
 // instruction cache.
 template <uint32_t KIND, int THREADS>
-__device__ __noinline__ void subtree_phase(const TreeJob& job, uint32_t items, uint32_t h, uint64_t idx0, uint32_t c0, uint32_t c1, uint32_t c2,
-                                           uint32_t c3, uint64_t* out) {
-  const uint32_t ch[4] = {c0, c1, c2, c3};
+__device__ __noinline__ void subtree_phase(const TreeJob& job, uint32_t items, uint32_t h, uint64_t idx0, uint64_t* out) {
+  uint32_t ch[4];
+  fold_challenge<KIND>(job, ch);
   const uint32_t groups = items >> h;
   const uint64_t* digests = reinterpret_cast<const uint64_t*>(job.raw) + 4 * idx0;
   uint64_t* l1 = job.inner + 4 * (inner_offset(job.logn, 1) + (idx0 >> 1));
@@ -245,9 +253,9 @@ __device__ __noinline__ void subtree_phase(const TreeJob& job, uint32_t items, u
 // 2017 us; a fold's tree of 2^21 1105 -> 1067 us.  Longer leaves would lose the 6
 // instructions a round again to splitting their words.
 template <uint32_t KIND, int THREADS>
-__device__ __noinline__ void value_subtree_phase(const TreeJob& job, uint32_t items, uint32_t h, uint64_t idx0, uint32_t c0, uint32_t c1, uint32_t c2,
-                                                 uint32_t c3, uint64_t* out) {
-  const uint32_t ch[4] = {c0, c1, c2, c3};
+__device__ __noinline__ void value_subtree_phase(const TreeJob& job, uint32_t items, uint32_t h, uint64_t idx0, uint64_t* out) {
+  uint32_t ch[4];
+  fold_challenge<KIND>(job, ch);
   const uint32_t groups = items >> h, steps = h == 2 ? 7 : (h == 1 ? 3 : 1);
   uint64_t* l1 = job.inner + 4 * (inner_offset(job.logn, 1) + (idx0 >> 1));
   uint64_t* l2 = job.inner + 4 * (inner_offset(job.logn, 2) + (idx0 >> 2));
@@ -387,9 +395,9 @@ __device__ __forceinline__ void put_digest(uint64_t* buf, uint64_t* top, uint32_
 
 // Leaf phase by pairs of lanes (fewer leaves than threads).
 template <uint32_t KIND, int THREADS>
-__device__ __noinline__ void pair_leaf_phase(const TreeJob& job, uint32_t items, uint64_t idx0, uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3,
-                                             uint64_t* out, uint64_t* top) {
-  const uint32_t ch[4] = {c0, c1, c2, c3};
+__device__ __noinline__ void pair_leaf_phase(const TreeJob& job, uint32_t items, uint64_t idx0, uint64_t* out, uint64_t* top) {
+  uint32_t ch[4];
+  fold_challenge<KIND>(job, ch);
   const uint32_t lane = threadIdx.x & 31, q = lane & 1;
   for (uint32_t base = warp_index() * 16; base < items; base += THREADS / 2) {
     const uint32_t i = base + (lane >> 1);
@@ -470,21 +478,25 @@ __device__ __noinline__ void top_levels(uint64_t* top, uint32_t count, const Tre
   if (warp >= 4) return;
   if (warp == 3 && act != kRootNone) {
     // one permutation site for all of this warp's steps
-    enum { kPublic, kNode, kCommit, kRoot, kChallenge };
+    enum { kNode, kPublic, kCommit, kRoot, kChallenge };
     WarpSponge sp(warp_smem + kWarpKeccakWords * 3);
-    const RoundFrames f = act == kRootCircleRound ? circle_round_frames(lane, job.round) : qm31_round_frames(lane, job.round, job.frame_in_count);
     sp.load(job.base ? job.base : job.transcript);
+    const uint64_t state = sp.a;
+    RoundFrames f = {0, 0};
     uint64_t* const node = top + 8 * 4 + 4 * 3;  // the fourth node above eight digests
+    // the node that the other warps wait for first: the state's load and the frames
+    // ahead of it held the level above eight digests up by 1000 cycles (with the fold
+    // challenge, chain of 10 trees 537 -> 533 us, 2^10 opening 258 -> 252)
 #pragma unroll 1
-    for (uint32_t step = job.pub ? kPublic : kNode; step <= kChallenge; step++) {
-      uint64_t word = 0, keep = 0;
-      if (step == kPublic) {
-        word = sp.digest_word(job.pub);
-      } else if (step == kNode) {
-        if (count != 8) continue;
-        keep = sp.a;
+    for (uint32_t step = count == 8 ? kNode : kPublic; step <= kChallenge; step++) {
+      uint64_t word = 0;
+      if (step == kNode) {
         sp.a = lane < 8 ? top[24 + lane] : lane == 8 ? 0x06ull : lane == 16 ? kPadEnd : 0ull;
+      } else if (step == kPublic) {
+        if (!job.pub) continue;
+        word = sp.digest_word(job.pub);
       } else if (step == kCommit) {
+        f = act == kRootCircleRound ? circle_round_frames(lane, job.round) : qm31_round_frames(lane, job.round, job.frame_in_count);
         word = f.commit;
       } else if (step == kRoot) {
         asm volatile("bar.sync 2, 128;" ::: "memory");
@@ -496,7 +508,7 @@ __device__ __noinline__ void top_levels(uint64_t* top, uint32_t count, const Tre
       if (step == kNode) {
         uint64_t* const out = job.inner + 4 * (inner_offset(job.logn, level + 1) + (idx0 >> 1) + 3);
         if (lane < 4) node[lane] = out[lane] = sp.a;
-        sp.a = keep;
+        sp.a = state;
         asm volatile("bar.sync 1, 128;" ::: "memory");
       }
     }
@@ -541,32 +553,23 @@ __device__ __forceinline__ void tree_tile_body(const TreeJob& job, const uint64_
   __shared__ __align__(16) uint64_t warp_smem[4 * kWarpKeccakWords];
   __shared__ __align__(16) uint64_t top[kTopWords];
   __shared__ uint32_t s_last;
-  __shared__ uint32_t s_ch[4];
   const uint32_t tl = job.tile_log < job.logn ? job.tile_log : job.logn;
   const uint32_t T = 1u << tl;
   const uint32_t M = tree_phase_digests(T, THREADS);  // capacity of bufA; bufB holds half
   uint64_t* bufA = sm;
   uint64_t* bufB = sm + 4 * M;
 
-  uint32_t ch[4] = {0, 0, 0, 0};
-  if constexpr (KIND == kLeafFold || KIND == kLeafFoldx4 || KIND == kLeafFoldQ) {
-    if (threadIdx.x < 4) s_ch[threadIdx.x] = __ldcg(job.fold_ch + threadIdx.x);
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < 4; k++) ch[k] = s_ch[k];
-  }
-
   // 1) leaf digests (and the lowest levels of this tile, per thread)
   const uint64_t first = tile * T;
   uint32_t h = 0;
   if (T < THREADS) {
-    pair_leaf_phase<KIND, THREADS>(job, T, first, ch[0], ch[1], ch[2], ch[3], bufA, top);
+    pair_leaf_phase<KIND, THREADS>(job, T, first, bufA, top);
   } else {
     h = tree_subtree_height(T, THREADS);
     if constexpr (KIND == kLeafQM31 || KIND == kLeafFold || KIND == kLeafFoldQ)
-      value_subtree_phase<KIND, THREADS>(job, T, h, first, ch[0], ch[1], ch[2], ch[3], bufA);
+      value_subtree_phase<KIND, THREADS>(job, T, h, first, bufA);
     else
-      subtree_phase<KIND, THREADS>(job, T, h, first, ch[0], ch[1], ch[2], ch[3], bufA);
+      subtree_phase<KIND, THREADS>(job, T, h, first, bufA);
   }
   // 2) treelet: the levels above, to kStdDigests digests and then to the root
   uint32_t top_log = tl < kStdLog ? tl : kStdLog;
