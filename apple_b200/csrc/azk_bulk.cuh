@@ -46,6 +46,9 @@ __device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32
                : "memory");
 }
 
+// Orders ordinary stores of global memory that this thread may see before later
+// async-proxy (bulk copy) reads of it.
+__device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;\n" ::: "memory"); }
 // Orders this thread's earlier generic-proxy accesses of shared memory before
 // later async-proxy (bulk copy) writes to it.
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }

@@ -201,10 +201,30 @@ struct LaunchCfg {
 // them.  Such a kernel calls dependent_begin() before it touches anything that an
 // earlier kernel writes or reads; there it waits for that kernel's memory to be
 // complete and lets its own successor be set up.
+//
+// A dependent kernel is alive while the kernel ahead of it still writes, so what an
+// earlier kernel writes (layers, buffers exchanged between passes, challenges) is not
+// read-only for its lifetime: it is read by ld_written() or __ldcg(), never by
+// __ldg() or through a const __restrict__ parameter, which allow the read-only cache
+// and let the compiler move the load ahead of the wait.  Those are for what copies
+// and completed set-up work wrote: job and work lists, twiddles, inverse layers,
+// raw messages.
 #if defined(__CUDACC__)
 __device__ __forceinline__ void dependent_begin() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+// An ordinary cached load of global memory, ordered after dependent_begin() (both are
+// volatile).
+__device__ __forceinline__ uint4 ld_written(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(__cvta_generic_to_global(p)));
+  return v;
+}
+__device__ __forceinline__ uint32_t ld_written(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(__cvta_generic_to_global(p)));
+  return v;
 }
 template <class... P, class... A>
 inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {

@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(THREADS) fft_pass_q_kernel(const FftJob* __res
     for (uint32_t L = threadIdx.x; L < T; L += THREADS, gi += gstep) {
       uint4 v;
       if (ft.first)
-        v = gi < ft.count ? __ldg(job.in + gi) : make_uint4(0u, 0u, 0u, 0u);
+        v = gi < ft.count ? ld_written(job.in + gi) : make_uint4(0u, 0u, 0u, 0u);
       else
         v = job.out[gi];
       const uint32_t a = fpad(L);
@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(THREADS) fft_pass_m31_kernel(const FftJob* __r
     for (uint32_t L = threadIdx.x; L < T; L += THREADS, gi += gstep) {
       uint32_t v;
       if (ft.first)
-        v = gi < ft.count ? __ldg(in_a + 4 * gi) : 0u;
+        v = gi < ft.count ? ld_written(in_a + 4 * gi) : 0u;
       else
         v = job.narrow[gi];
       sv[fpad(L)] = v;
@@ -579,8 +579,8 @@ __device__ __forceinline__ qm31 fold_unscaled(uint4 p, uint4 q, uint4 t, const q
   return q_mul_add(q_mul(d, qm31{t.x, t.y, t.z, t.w}), ch, qm31{p.x + q.x, p.y + q.y, p.z + q.z, p.w + q.w});
 }
 template <bool Q>
-__global__ void __launch_bounds__(256, 4) fold_chain_kernel(const uint4* __restrict__ prev, uint64_t n_in, const void* __restrict__ inv_words,
-                                                         const uint32_t* __restrict__ chp, uint32_t rounds, uint4* __restrict__ out) {
+__global__ void __launch_bounds__(256, 4) fold_chain_kernel(const uint4* prev, uint64_t n_in, const void* __restrict__ inv_words, const uint32_t* chp,
+                                                         uint32_t rounds, uint4* out) {
   using Inv = typename FoldInv<Q>::type;
   const Inv* inv = static_cast<const Inv*>(inv_words);
   __shared__ uint4 buf[kFoldTile / 2 + kFoldTile / 4];
@@ -600,15 +600,23 @@ __global__ void __launch_bounds__(256, 4) fold_chain_kernel(const uint4* __restr
   const uint32_t scale = 1u << ((31 - rounds) % 31);  // 2^-rounds
   {
     const qm31_factor ch = q_factor(qm31{s_ch[0], s_ch[1], s_ch[2], s_ch[3]});
-#pragma unroll 2
-    for (uint32_t j = threadIdx.x; j < cnt; j += 256) {
-      qm31 v = fold_unscaled(__ldg(prev + base + 2 * j), __ldg(prev + base + 2 * j + 1), __ldg(inv + base / 2 + j), ch);
+    auto finish = [&](uint32_t j, uint4 p, uint4 q, Inv t) {
+      qm31 v = fold_unscaled(p, q, t, ch);
       if (rounds == 1) v = q_mul_m31(v, scale);
       const uint4 w = make_uint4(v.a, v.b, v.c, v.d);
       if (rounds == 1)
         out[base / 2 + j] = w;
       else
         buf[j] = w;
+    };
+    // the loads of two folds ahead of both: ld_written's order is the program's
+    for (uint32_t j = threadIdx.x; j < cnt; j += 512) {
+      const uint32_t k = j + 256 < cnt ? j + 256 : j;
+      const uint4 p = ld_written(prev + base + 2 * j), q = ld_written(prev + base + 2 * j + 1);
+      const uint4 p2 = ld_written(prev + base + 2 * k), q2 = ld_written(prev + base + 2 * k + 1);
+      const Inv t = __ldg(inv + base / 2 + j), t2 = __ldg(inv + base / 2 + k);
+      finish(j, p, q, t);
+      if (k != j) finish(k, p2, q2, t2);
     }
   }
   uint4* src = buf;
@@ -743,7 +751,7 @@ __global__ void __launch_bounds__(128) pcs_tail_kernel(const PcsInstance* __rest
     const uint32_t* c = I.challenges + 4 * (k - 1);
     const qm31 ch = {__ldcg(c), __ldcg(c + 1), __ldcg(c + 2), __ldcg(c + 3)};
     for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x) {
-      const uint4 p = __ldg(prev + 2 * i), q = __ldg(prev + 2 * i + 1);
+      const uint4 p = ld_written(prev + 2 * i), q = ld_written(prev + 2 * i + 1);
       const qm31 r = fri_fold_pair(qm31{p.x, p.y, p.z, p.w}, qm31{q.x, q.y, q.z, q.w}, __ldg(inv + i), ch);
       fl[i] = make_uint4(r.a, r.b, r.c, r.d);
     }

@@ -260,7 +260,7 @@ __device__ __forceinline__ void m31_tile(const FftJob& job, uint2 w, uint32_t* Y
 #pragma unroll
       for (int b = 0; b < 4; b++) {
         const uint64_t gi = p.gidx(LA | ((uint32_t)b << 8));
-        x[b] = gi < count ? __ldg(in_a + 4 * gi) : 0u;
+        x[b] = gi < count ? ld_written(in_a + 4 * gi) : 0u;
       }
 #pragma unroll
       for (int b = 0; b < 16; b++) v[b] = x[b & 3];
@@ -268,12 +268,12 @@ __device__ __forceinline__ void m31_tile(const FftJob& job, uint2 w, uint32_t* Y
 #pragma unroll
       for (int b = 0; b < 16; b++) {
         const uint64_t gi = p.gidx(LA | ((uint32_t)b << 8));
-        v[b] = gi < count ? __ldg(in_a + 4 * gi) : 0u;
+        v[b] = gi < count ? ld_written(in_a + 4 * gi) : 0u;
       }
     }
   } else {
 #pragma unroll
-    for (int b = 0; b < 16; b++) v[b] = __ldg(job.narrow + p.gidx(LA | ((uint32_t)b << 8)));
+    for (int b = 0; b < 16; b++) v[b] = ld_written(job.narrow + p.gidx(LA | ((uint32_t)b << 8)));
   }
   subpass<2>(v, w2, p, top_zero ? 1 : 3);
   if (p.c >= 8) {  // every stage among L bits 8-11 (a high-stage pass of at most 4 stages)
@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(kThreads, 2) fft_q_tile_kernel(const FftJob* _
         continue;
       }
       const uint64_t gi = p.gidx(LA | ((uint32_t)b << 8));
-      v[b] = gi < count ? to_q(__ldg(job.in + gi)) : qm31{0u, 0u, 0u, 0u};
+      v[b] = gi < count ? to_q(ld_written(job.in + gi)) : qm31{0u, 0u, 0u, 0u};
     }
   } else {
 #pragma unroll
@@ -416,6 +416,7 @@ __global__ void __launch_bounds__(kThreads, 4) fft_m31_low_tma_kernel(const FftJ
   if (item >= nwork) return;
   if (t == 0) {
     mbar_init(&bar, 1);
+    fence_proxy_async_global();  // the kernel ahead wrote the exchange buffer by ordinary stores
     fetch_low_tile(jobs, work[item], X, &bar);
   }
   __syncthreads();

@@ -45,7 +45,7 @@ __device__ __forceinline__ uint32_t warp_index() { return __shfl_sync(0xffffffff
 template <uint32_t KIND>
 __device__ __forceinline__ void leaf_digest(const TreeJob& job, uint64_t leaf, const uint32_t (&ch)[4], uint64_t (&d)[4]) {
   if constexpr (KIND == kLeafQM31) {
-    uint4 v = __ldg(job.layer + leaf);
+    uint4 v = ld_written(job.layer + leaf);
     sha3_16((uint64_t)v.x | ((uint64_t)v.y << 32), (uint64_t)v.z | ((uint64_t)v.w << 32), d);
   } else if constexpr (KIND == kLeafDigest) {
     ld_dig(reinterpret_cast<const uint64_t*>(job.raw) + 4 * leaf, d);
@@ -65,7 +65,7 @@ __device__ __forceinline__ void fold_challenge(const TreeJob& job, uint32_t (&ch
 // Value e of the layer that a fold kind produces.
 template <uint32_t KIND>
 __device__ __forceinline__ uint4 folded_value(const TreeJob& job, uint64_t e, const uint32_t (&ch)[4]) {
-  const uint4 p = __ldg(job.layer + 2 * e), q = __ldg(job.layer + 2 * e + 1);
+  const uint4 p = ld_written(job.layer + 2 * e), q = ld_written(job.layer + 2 * e + 1);
   const qm31 pos = {p.x, p.y, p.z, p.w}, neg = {q.x, q.y, q.z, q.w}, c = {ch[0], ch[1], ch[2], ch[3]};
   qm31 r;
   if constexpr (KIND == kLeafFoldQ) {
@@ -111,7 +111,7 @@ __device__ __forceinline__ uint32_t leaf_setup(const TreeJob& job, uint64_t leaf
       const uint64_t e = 4 * leaf + m;
       uint4 v;
       if constexpr (KIND == kLeafQM31x4) {
-        v = __ldg(job.layer + e);
+        v = ld_written(job.layer + e);
       } else {
         v = folded_value<KIND>(job, e, ch);
         job.out_layer[e] = v;
@@ -281,7 +281,7 @@ __device__ __noinline__ void value_subtree_phase(const TreeJob& job, uint32_t it
       } else {
         uint4 v;
         if constexpr (KIND == kLeafQM31) {
-          v = __ldg(job.layer + leaf);
+          v = ld_written(job.layer + leaf);
         } else {
           v = folded_value<KIND>(job, leaf, ch);
           job.out_layer[leaf] = v;
@@ -333,7 +333,7 @@ __device__ __forceinline__ uint4 pair_leaf(const TreeJob& job, uint64_t leaf, bo
     if constexpr (KIND == kLeafQM31 || KIND == kLeafFold || KIND == kLeafFoldQ) {
       uint4 v;
       if constexpr (KIND == kLeafQM31) {
-        v = __ldg(job.layer + leaf);
+        v = ld_written(job.layer + leaf);
       } else {
         v = folded_value<KIND>(job, leaf, ch);
         if (ok && q == 0) job.out_layer[leaf] = v;
@@ -348,7 +348,7 @@ __device__ __forceinline__ uint4 pair_leaf(const TreeJob& job, uint64_t leaf, bo
         const uint64_t e = 4 * leaf + 2 * q + m;
         uint4 v;
         if constexpr (KIND == kLeafQM31x4) {
-          v = __ldg(job.layer + e);
+          v = ld_written(job.layer + e);
         } else {
           v = folded_value<KIND>(job, e, ch);
           if (ok) job.out_layer[e] = v;

@@ -1049,6 +1049,7 @@ static void witness_run(azk_witness_plan* p, const uint4* x, uint64_t nx, const 
       p->roots_n = 0;
       p->roots.alloc(8 * n, "Witness.Roots");
       AZK_CU(launch_witness_roots(p->roots.as<uint2>(), ln, p->s));
+      sync_stream(p->s);  // the convolutions read it as read-only data
       p->roots_n = n;
     }
     a.roots = p->roots.as<uint2>();
