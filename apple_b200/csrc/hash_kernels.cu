@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(256) hash_batch(const uint8_t* __restrict__ in
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   uint64_t d[4];
-  hash_message(in + i * stride, LEN ? LEN : len, suffix, aligned8 != 0, d);
+  hash_message(in + i * stride, LEN ? LEN : len, suffix, aligned8 != 0, i == 0 || i + 1 == count, d);
   store_digest(out + i * out_stride, out_stride, d, out_align);
 }
 

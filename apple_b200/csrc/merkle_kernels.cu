@@ -42,6 +42,9 @@ __device__ __forceinline__ void ld_dig_cg(const uint64_t* p, uint64_t (&d)[4]) {
 // warp's lanes.
 __device__ __forceinline__ uint32_t warp_index() { return __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0); }
 
+// The first or the last leaf: nothing outside its bytes is read.
+__device__ __forceinline__ bool edge_leaf(const TreeJob& job, uint64_t leaf) { return leaf == 0 || leaf + 1 == 1ull << job.logn; }
+
 template <uint32_t KIND>
 __device__ __forceinline__ void leaf_digest(const TreeJob& job, uint64_t leaf, const uint32_t (&ch)[4], uint64_t (&d)[4]) {
   if constexpr (KIND == kLeafQM31) {
@@ -50,7 +53,7 @@ __device__ __forceinline__ void leaf_digest(const TreeJob& job, uint64_t leaf, c
   } else if constexpr (KIND == kLeafDigest) {
     ld_dig(reinterpret_cast<const uint64_t*>(job.raw) + 4 * leaf, d);
   } else {
-    hash_message(job.raw + leaf * job.stride, job.len, job.suffix, job.aligned8 != 0, d);
+    hash_message(job.raw + leaf * job.stride, job.len, job.suffix, job.aligned8 != 0, edge_leaf(job, leaf), d);
   }
 }
 
@@ -81,16 +84,20 @@ __device__ __forceinline__ uint4 folded_value(const TreeJob& job, uint64_t e, co
 // 17) of a zero state.  A compare, a select and an XOR for each lane of the rate took
 // 0.5 % of a tree of 2^22 64-byte leaves.
 template <uint32_t LANES>
-__device__ __forceinline__ void raw_setup(const TreeJob& job, const uint8_t* p, uint64_t (&a)[25]) {
+__device__ __forceinline__ void raw_setup(const TreeJob& job, uint64_t leaf, uint64_t (&a)[25]) {
+  const uint8_t* const p = job.raw + leaf * job.stride;
   const uint32_t full = job.len >> 3, rem = job.len & 7;
-  const UnalignedWords u(p);
   uint64_t tail = (uint64_t)job.suffix << (8 * rem);
-  if (rem) tail |= u.word(full, rem);
   if (job.aligned8) {
+    if (rem) tail |= aligned_tail(p + 8 * full, rem);
 #pragma unroll
     for (uint32_t i = 0; i < LANES; i++)
       if (i < full) a[i] = __ldg(reinterpret_cast<const uint64_t*>(p) + i);
   } else {
+    // the edge reader for every leaf: both readers in this loop's code cost unaligned
+    // trees 3 % (2^20 leaves of 99 bytes: 606 us, 618 with both, 598 without an edge)
+    const UnalignedWords<true> u(p, job.len);
+    if (rem) tail |= u.word(full, rem);
 #pragma unroll
     for (uint32_t i = 0; i < LANES; i++)
       if (i < full) a[i] = u.word(i, 8);
@@ -123,9 +130,8 @@ __device__ __forceinline__ uint32_t leaf_setup(const TreeJob& job, uint64_t leaf
     a[16] = kPadEnd;
     return 1;
   } else {
-    const uint8_t* const p = job.raw + leaf * job.stride;
-    if (job.len < 72) raw_setup<9>(job, p, a);
-    else raw_setup<17>(job, p, a);
+    if (job.len < 72) raw_setup<9>(job, leaf, a);
+    else raw_setup<17>(job, leaf, a);
     if (job.len == 136) return 2;
     a[16] ^= kPadEnd;
     return 1;
@@ -310,14 +316,15 @@ __device__ __noinline__ void value_subtree_phase(const TreeJob& job, uint32_t it
 __device__ __forceinline__ ulonglong2 pack_qm31(uint4 v) {
   return make_ulonglong2((uint64_t)v.x | ((uint64_t)v.y << 32), (uint64_t)v.z | ((uint64_t)v.w << 32));
 }
-// Word i (< 17) of a raw message of `len` bytes with its suffix (none at len 136).
-__device__ __forceinline__ uint64_t raw_message_word(const TreeJob& job, const uint8_t* p, uint32_t i) {
+// Word i of a raw message with its suffix (none at length 136); word(i, n): its n
+// bytes.
+template <class F>
+__device__ __forceinline__ uint64_t raw_message_word(const TreeJob& job, uint32_t i, F word) {
   const uint32_t full = job.len >> 3, rem = job.len & 7;
   if (i > full || i > 16) return 0;
-  if (i < full && job.aligned8) return __ldg(reinterpret_cast<const uint64_t*>(p) + i);
   const uint32_t n = i < full ? 8 : rem;
   const uint64_t v = i < full ? 0 : (uint64_t)job.suffix << (8 * rem);
-  return n ? v | UnalignedWords(p).word(i, n) : v;
+  return n ? v | word(i, n) : v;
 }
 
 // Digest of one leaf by a pair of lanes, in split form.  `ok`: the pair's leaf is
@@ -361,13 +368,22 @@ __device__ __forceinline__ uint4 pair_leaf(const TreeJob& job, uint64_t leaf, bo
     } else {
       // words 2m by thread 0, 2m + 1 by thread 1
       const uint8_t* p = job.raw + leaf * job.stride;
-      const uint32_t last = job.len >> 3;
+      auto words = [&](auto word) {
+        const uint32_t last = job.len >> 3;
 #pragma unroll
-      for (uint32_t m = 0; m < 9; m++) {
-        if (2 * m > last) continue;  // the same for the whole launch
-        uint32_t w1;
-        pair_split2(raw_message_word(job, p, 2 * m + q), q, a[2 * m], w1);
-        if (m < 8) a[2 * m + 1] = w1;
+        for (uint32_t m = 0; m < 9; m++) {
+          if (2 * m > last) continue;  // the same for the whole launch
+          uint32_t w1;
+          pair_split2(raw_message_word(job, 2 * m + q, word), q, a[2 * m], w1);
+          if (m < 8) a[2 * m + 1] = w1;
+        }
+      };
+      if (job.aligned8) {
+        words([&](uint32_t i, uint32_t n) { return n == 8 ? __ldg(reinterpret_cast<const uint64_t*>(p) + i) : aligned_tail(p + 8 * i, n); });
+      } else {
+        // the exchange between lanes needs the whole warp: one reader for all its leaves
+        const UnalignedWords<true> u(p, job.len);
+        words([&](uint32_t i, uint32_t n) { return u.word(i, n); });
       }
     }
     if (KIND == kLeafRaw && job.len == 136) {  // a full block, then the padding's own
