@@ -258,9 +258,9 @@ cudaError_t launch_gather_openings(const TreeJob* d_job, const uint64_t* d_idx, 
 cudaError_t launch_domain_tables(uint32_t logn, uint32_t* d_tw, uint32_t* d_inv, cudaStream_t s);
 cudaError_t launch_domain_points(uint32_t logn, uint32_t* d_xy, cudaStream_t s);
 cudaError_t launch_widen_m31(const uint32_t* d_in, uint4* d_out, uint64_t n, cudaStream_t s);
-// Witness columns -> FFT basis (witness_kernels.cu, witness_fft.cu): factorial
-// tables k!, 1/k!, 2^(1-k) k! of n entries (seg: ceil(n/1024) words of scratch).
-cudaError_t launch_witness_tables(uint64_t n, uint32_t* fact, uint32_t* seg, uint32_t* ifact, uint32_t* scale, cudaStream_t s);
+// Witness columns -> FFT basis (witness_kernels.cu, witness_fft.cu): tables k! and
+// 1/k! of n entries and 2^(1-k) k! of n_scale (seg: ceil(n/1024) words of scratch).
+cudaError_t launch_witness_tables(uint64_t n, uint64_t n_scale, uint32_t* fact, uint32_t* seg, uint32_t* ifact, uint32_t* scale, cudaStream_t s);
 // Chebyshev coefficients of two columns by the direct sum: count_x / count_y
 // monomial coefficients to n values each at cx, cy.  ax, ay: n QM31 of scratch each;
 // px, py: witness_partial_values(n) each.
@@ -275,14 +275,15 @@ struct WitnessConv {
   uint64_t count_x, count_y;
   const uint32_t *fact, *ifact;  // 2n entries
   const uint2* roots;            // n CM31 roots, bit-reversed
-  uint8_t *c, *c2, *c3;          // values between the convolutions (n, n / 2, n / 2 per column)
+  uint8_t* c;                    // values between the convolutions (n per column)
   uint64_t c_stride;             // bytes from one column's to the next's
   void* t;                       // 2n values per column
-  void* u[2];                    // the parity step's two products, likewise
+  void* u[2];                    // the parity step's two products, likewise (u[1] null: one after the other)
   uint64_t t_stride;
   const uint2* k[2];             // transforms of the fixed sequences
   uint8_t* o[2];                 // a convolution's outputs, o_stride bytes between columns
   uint64_t o_stride, outputs;
+  uint64_t odd;                  // bytes from the even values (n / 2 per column) in c to the odd ones
 };
 struct WitnessKernels {
   const uint2* k[3];  // transforms of 1/j!, 1/(2j)!, 1/(2j-1)!, 2n CM31 values each

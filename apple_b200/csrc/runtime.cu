@@ -2,7 +2,6 @@
 // Keccak-f batch, SHA3/Keccak batch hashing, raw/prehashed Merkle commitment,
 // Circle FFT codeword, single folds and fold chains.
 #include <algorithm>
-#include <map>
 #include <cstdlib>
 
 #include "azk_field.cuh"
@@ -975,34 +974,44 @@ void azk_codeword_plan_destroy(azk_codeword_plan* p) { delete p; }
 
 // ---- witness columns -> FFT basis (CircleWitnessToFFTBasisPlanV1) ----
 // Work is sized by the columns given: n = the power of two that holds the longer one
-// (at least kWitnessMinLog, or the capacity), not by the capacity.  Columns of at
-// least 2^kWitnessFftLog take the fast convolutions, shorter ones the direct sum.
-// Columns of at least 2^kWitnessFftLog take the fast convolutions, shorter ones the
-// direct sum (two full QM31 columns on B200, direct / convolutions: 2^12 74 / 100 us,
-// 2^13 160 / 111 us, 2^14 425 / 116 us, 2^19 175,900 / 828 us).
+// (at least 2^kWitnessMinLog, or the capacity), not by the capacity.  With n of at
+// least 2^kWitnessFftLog the fast convolutions run, below the direct sum (two full
+// QM31 columns on B200, direct / convolutions: 2^12 74 / 100 us, 2^13 160 / 111 us,
+// 2^14 425 / 116 us, 2^19 175,900 / 828 us).
 static constexpr uint32_t kWitnessMinLog = 11, kWitnessFftLog = 13;
 
+// Every buffer is made with the plan, for its longest columns, so a plan that exists
+// can run every call.  For a capacity of n coefficients (a 2n domain), in bytes:
+// factorials 16 n and roots 8 n; transforms of the fixed sequences for every size,
+// 96 n; `t` 64 n, `u` 64 n and `c` 32 n, the convolutions' values.  Host columns lie in
+// `u`, which is written only after the first convolution has read them, and the
+// result on its way to the host in `t`: 280 n, 587 MB at a 2^22 domain (`u` 128 n and
+// 344 n below that).
 struct azk_witness_plan {
   azk_ctx* ctx;
   std::mutex mu;
   cudaStream_t s = nullptr;
   uint32_t logn;
   uint64_t n;  // coefficient capacity = half the domain
-  DevBuf tables, flag;
+  DevBuf tables, flag, work;
   uint32_t *fact = nullptr, *ifact = nullptr, *scale = nullptr;  // in `tables`
-  DevBuf xin, yin, out;                  // host columns and result (made on first use)
-  DevBuf work;                           // scratch, sized for the largest call so far
-  DevBuf roots;                          // CM31 roots for convolutions of up to 2 * roots_n values
-  uint64_t roots_n = 0;
-  std::map<uint32_t, DevBuf> sequences;  // by lm: transforms of the three fixed sequences
+  uint2* roots = nullptr;                                        // CM31 roots for every size
+  uint8_t *t = nullptr, *u = nullptr, *c = nullptr;              // in `work`
+  uint64_t u_bytes = 0;
+  uint8_t* direct = nullptr;                                     // the direct sum's scratch
+  uint2* sequences = nullptr;
+  uint32_t built = 0;                                            // sizes (bit log2 n) whose sequences are there
   ~azk_witness_plan() {
     if (s) cudaStreamDestroy(s);
   }
-  void host_columns() {
-    if (xin.p) return;
-    out.alloc(32 * n, "Witness.Output");
-    yin.alloc(16 * n, "Witness.Columns");
-    xin.alloc(16 * n, "Witness.Columns");
+  uint4* host_x() const { return reinterpret_cast<uint4*>(u); }
+  uint4* host_y() const { return reinterpret_cast<uint4*>(u) + n; }
+  uint4* host_out() const { return reinterpret_cast<uint4*>(t); }
+  // Transforms for columns of 2^ln values: 6 * 2^ln CM31 values, sizes in ascending order.
+  WitnessKernels sequences_at(uint32_t ln) const {
+    const uint64_t m = 1ull << ln;
+    uint2* b = sequences + 6 * (m - (1ull << kWitnessFftLog));
+    return WitnessKernels{{b, b + 2 * m, b + 4 * m}};
   }
 };
 
@@ -1025,57 +1034,34 @@ static void witness_run(azk_witness_plan* p, const uint4* x, uint64_t nx, const 
   while ((1ull << ln) < std::max(nx, ny)) ln++;
   const uint64_t n = 1ull << ln;
   const bool direct = ln < kWitnessFftLog;
-  // scratch: one allocation, sliced for this call.  Values are QM31 in two columns,
-  // or (convolutions of lifted columns) CM31 in one.
+  // values are QM31 in two columns, or (convolutions of lifted columns) CM31 in one
   const uint64_t col = direct || !lifted ? 16 * n : 8 * n, cols = direct || !lifted ? 2 : 1;
-  const uint64_t partial = direct ? 16 * witness_partial_values(n) : 0;
-  const uint64_t need = direct ? cols * (2 * col + partial) : cols * (col + 3 * 2 * col + col);
-  if (p->work.bytes < need) p->work.alloc(need, "Witness.Work");
-  uint8_t* w = p->work.as<uint8_t>();
-  auto take = [&w](uint64_t bytes) {
-    uint8_t* r = w;
-    w += bytes;
-    return r;
-  };
   WitnessConv a{};
   a.lm = ln + 1;
   a.x = x, a.y = y;
   a.count_x = nx, a.count_y = ny;
   a.fact = p->fact, a.ifact = p->ifact;
-  a.c = take(cols * col);
+  a.c = p->c;
   a.c_stride = col;
-  if (!direct) {
-    if (p->roots_n < n) {
-      p->roots_n = 0;
-      p->roots.alloc(8 * n, "Witness.Roots");
-      AZK_CU(launch_witness_roots(p->roots.as<uint2>(), ln, p->s));
-      sync_stream(p->s);  // the convolutions read it as read-only data
-      p->roots_n = n;
-    }
-    a.roots = p->roots.as<uint2>();
-    a.t_stride = 2 * col;
-    a.t = take(cols * 2 * col);
-    a.u[0] = take(cols * 2 * col);
-    a.u[1] = take(cols * 2 * col);
-    a.c2 = take(cols * col / 2);
-    a.c3 = take(cols * col / 2);
-  }
+  a.roots = p->roots;
+  a.t_stride = 2 * col;
+  a.t = p->t;
+  a.u[0] = p->u;
+  // the parity step's second product, where there is room for both at once
+  a.u[1] = 2 * cols * 2 * col <= p->u_bytes ? p->u + cols * 2 * col : nullptr;
   GpuTimer g(p->s);
   if (direct) {
-    uint4* c = reinterpret_cast<uint4*>(a.c);
-    uint4 *ax = reinterpret_cast<uint4*>(take(col)), *ay = reinterpret_cast<uint4*>(take(col));
-    uint4 *px = reinterpret_cast<uint4*>(take(partial)), *py = reinterpret_cast<uint4*>(take(partial));
+    const uint64_t partial = witness_partial_values(n);
+    uint4 *ax = reinterpret_cast<uint4*>(p->direct), *ay = ax + n, *px = ay + n, *py = px + partial, *c = reinterpret_cast<uint4*>(a.c);
     AZK_CU(launch_witness_chebyshev(x, nx, y, ny, n, a.ifact, p->scale, ax, ay, px, py, c, c + n, p->s));
     AZK_CU(launch_witness_line(a, out, p->n, p->s));
   } else {
-    auto sequences = [n](const DevBuf& b) { return WitnessKernels{{b.as<uint2>(), b.as<uint2>() + 2 * n, b.as<uint2>() + 4 * n}}; };
-    auto seq = p->sequences.find(a.lm);
-    if (seq == p->sequences.end()) {
-      DevBuf b(3 * 16 * n, "Witness.Sequences");
-      AZK_CU(launch_witness_fft_tables(a, sequences(b), p->s));
-      seq = p->sequences.emplace(a.lm, std::move(b)).first;
+    const WitnessKernels seq = p->sequences_at(ln);
+    if (!(p->built >> ln & 1u)) {
+      AZK_CU(launch_witness_fft_tables(a, seq, p->s));
+      p->built |= 1u << ln;
     }
-    AZK_CU(launch_witness_fft(a, sequences(seq->second), lifted, out, p->n, p->s));
+    AZK_CU(launch_witness_fft(a, seq, lifted, out, p->n, p->s));
   }
   g.stop();
   fill_stats(st, t, 0, g.seconds());
@@ -1083,11 +1069,10 @@ static void witness_run(azk_witness_plan* p, const uint4* x, uint64_t nx, const 
 
 static void witness_columns_to_device(azk_witness_plan* w, const uint32_t* x, uint64_t nx, const uint32_t* y, uint64_t ny, void* dout) {
   std::lock_guard<std::mutex> lk(w->mu);
-  w->host_columns();
   Timer t;
-  if (nx) AZK_CU(cudaMemcpyAsync(w->xin.p, x, 16 * nx, cudaMemcpyHostToDevice, w->s));
-  if (ny) AZK_CU(cudaMemcpyAsync(w->yin.p, y, 16 * ny, cudaMemcpyHostToDevice, w->s));
-  witness_run(w, w->xin.as<uint4>(), nx, w->yin.as<uint4>(), ny, static_cast<uint4*>(dout), nullptr, t);
+  if (nx) AZK_CU(cudaMemcpyAsync(w->host_x(), x, 16 * nx, cudaMemcpyHostToDevice, w->s));
+  if (ny) AZK_CU(cudaMemcpyAsync(w->host_y(), y, 16 * ny, cudaMemcpyHostToDevice, w->s));
+  witness_run(w, w->host_x(), nx, w->host_y(), ny, static_cast<uint4*>(dout), nullptr, t);
   sync_stream(w->s);
 }
 
@@ -1103,15 +1088,31 @@ azk_status azk_witness_plan_create(azk_ctx* ctx, uint32_t log_size, azk_witness_
     p->n = 1ull << (log_size - 1);
     p->s = new_stream();
     const uint64_t n = p->n;
-    const uint64_t entries = n >> kWitnessFftLog ? 2 * n : n;  // the convolutions need k! for k < 2n
-    const uint64_t slice = align_up(4 * entries, 256);
-    p->tables.alloc(3 * slice + 4 * ((entries + 1023) / 1024), "Witness.Factorials");
+    const bool conv = n >> kWitnessFftLog != 0;
+    const uint64_t nd = std::min<uint64_t>(n, (1ull << kWitnessFftLog) / 2);  // most the direct sum takes
+    const uint64_t entries = conv ? 2 * n : n;                      // the convolutions need k! for k < 2n
+    const uint64_t slice = align_up(4 * entries, 256), scale = align_up(4 * nd, 256), roots = conv ? 8 * n : 0;
+    p->tables.alloc(2 * slice + scale + roots + 4 * ((entries + 1023) / 1024), "Witness.Factorials");
     p->fact = p->tables.as<uint32_t>();
     p->ifact = p->fact + slice / 4;
     p->scale = p->ifact + slice / 4;
-    uint32_t* seg = p->scale + slice / 4;
+    p->roots = reinterpret_cast<uint2*>(p->scale + scale / 4);
+    uint32_t* seg = reinterpret_cast<uint32_t*>(p->roots) + roots / 4;
+    const uint64_t t_bytes = align_up(conv ? 64 * n : 32 * n, 256), direct = 16 * 2 * (nd + witness_partial_values(nd));
+    // both products of the parity step at once up to 2^20 coefficients (one after the
+    // other, QM31 columns of 2^18 take 631 instead of 564 us, of 2^19 870 instead of
+    // 832); of 2^21 one alone fills the chip (3102 and 3077)
+    p->u_bytes = align_up(!conv ? 32 * n : n >> 21 ? 64 * n : 128 * n, 256);
+    const uint64_t c_bytes = align_up(32 * n, 256), seq = conv ? 48 * (2 * n - (1ull << kWitnessFftLog)) : 0;
+    p->work.alloc(t_bytes + p->u_bytes + c_bytes + align_up(direct, 256) + seq, "Witness.Work");
+    p->t = p->work.as<uint8_t>();
+    p->u = p->t + t_bytes;
+    p->c = p->u + p->u_bytes;
+    p->direct = p->c + c_bytes;
+    p->sequences = reinterpret_cast<uint2*>(p->direct + align_up(direct, 256));
     p->flag.alloc(32, "Witness.Flag");
-    AZK_CU(launch_witness_tables(entries, p->fact, seg, p->ifact, p->scale, p->s));
+    if (conv) AZK_CU(launch_witness_roots(p->roots, log_size - 1, p->s));
+    AZK_CU(launch_witness_tables(entries, nd, p->fact, seg, p->ifact, p->scale, p->s));
     sync_stream(p->s);
     *out = p.release();
   });
@@ -1126,12 +1127,11 @@ azk_status azk_witness_plan_execute(azk_witness_plan* p, const uint32_t* x, uint
     // CircleWitnessFFTBasis.swift:349-353
     layout(nx <= p->n && ny <= p->n && nx + ny > 0);
     std::lock_guard<std::mutex> lk(p->mu);
-    p->host_columns();
     Timer t;
-    if (nx) AZK_CU(cudaMemcpyAsync(p->xin.p, x, 16 * nx, cudaMemcpyHostToDevice, p->s));
-    if (ny) AZK_CU(cudaMemcpyAsync(p->yin.p, y, 16 * ny, cudaMemcpyHostToDevice, p->s));
-    witness_run(p, p->xin.as<uint4>(), nx, p->yin.as<uint4>(), ny, p->out.as<uint4>(), st, t);
-    AZK_CU(cudaMemcpyAsync(out, p->out.p, 32 * p->n, cudaMemcpyDeviceToHost, p->s));
+    if (nx) AZK_CU(cudaMemcpyAsync(p->host_x(), x, 16 * nx, cudaMemcpyHostToDevice, p->s));
+    if (ny) AZK_CU(cudaMemcpyAsync(p->host_y(), y, 16 * ny, cudaMemcpyHostToDevice, p->s));
+    witness_run(p, p->host_x(), nx, p->host_y(), ny, p->host_out(), st, t);
+    AZK_CU(cudaMemcpyAsync(out, p->host_out(), 32 * p->n, cudaMemcpyDeviceToHost, p->s));
     sync_stream(p->s);
   });
 }

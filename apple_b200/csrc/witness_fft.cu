@@ -245,7 +245,7 @@ __device__ __forceinline__ Val<W> conv_input(const WitnessConv& a, uint32_t colu
     const uint64_t k = D - i;  // r_k (-2)^k at y^(D + i), r_k = G_k / k!
     uint32_t w = m31_mul(m31_mul(a.ifact[k], a.fact[D + i]), pow2_m31(k + 31 - a.lm % 31));
     if (k & 1) w = m31_neg(w);
-    return vscale(ldv<W>((k & 1 ? a.c3 : a.c2) + column * (a.c_stride / 2), k >> 1), w);
+    return vscale(ldv<W>(a.c + (k & 1 ? a.odd : 0) + column * (a.c_stride / 2), k >> 1), w);
   }
 }
 
@@ -484,18 +484,21 @@ __global__ void __launch_bounds__(512) line_out_kernel(const WitnessConv a, uint
   }
 }
 
-template <int W, int STEP, uint32_t TL>
+// A convolution from conv_input (HIGH) or from the values that one left in `t`: `outs`
+// products at once.
+template <int W, int STEP, uint32_t TL, bool HIGH>
 cudaError_t run_conv_tiles(const WitnessConv& a, uint32_t columns, uint32_t outs, cudaStream_t s) {
   const uint32_t tiles = 1u << (a.lm - TL);
   const size_t smem = (size_t)4 * W << TL;
-  cudaError_t e = launch_dependent(conv_high_kernel<W, STEP, TL>, dim3(tiles, columns), dim3(kConvThreads<TL>), smem, s, a);
+  cudaError_t e = cudaSuccess;
+  if constexpr (HIGH) e = launch_dependent(conv_high_kernel<W, STEP, TL>, dim3(tiles, columns), dim3(kConvThreads<TL>), smem, s, a);
   if (e == cudaSuccess) e = launch_dependent(conv_low_kernel<W, TL>, dim3(tiles, columns, outs), dim3(kConvThreads<TL>), smem, s, a);
   if (e == cudaSuccess && STEP != kTable) e = launch_dependent(conv_out_kernel<W, TL>, dim3(tiles, columns, outs), dim3(kConvThreads<TL>), smem, s, a);
   return e;
 }
-template <int W, int STEP>
+template <int W, int STEP, bool HIGH = true>
 cudaError_t run_conv(const WitnessConv& a, uint32_t columns, uint32_t outs, cudaStream_t s) {
-  return a.lm <= kShortLog ? run_conv_tiles<W, STEP, kShortTile>(a, columns, outs, s) : run_conv_tiles<W, STEP, kLongTile>(a, columns, outs, s);
+  return a.lm <= kShortLog ? run_conv_tiles<W, STEP, kShortTile, HIGH>(a, columns, outs, s) : run_conv_tiles<W, STEP, kLongTile, HIGH>(a, columns, outs, s);
 }
 
 constexpr uint32_t kLineTileLog = 11;  // 2 columns x 2048 x 16 bytes of shared memory
@@ -537,12 +540,20 @@ cudaError_t transform(WitnessConv a, const WitnessKernels& kr, uint4* out, uint6
   if (e != cudaSuccess) return e;
   a.flip = 0;
   if ((e = run_conv<W, kShift2>(a, columns, 1, s)) != cudaSuccess) return e;
+  // the even and the odd values take the place of c, which only the first pass reads
   a.k[0] = kr.k[1], a.k[1] = kr.k[2];
   a.u[0] = u[0], a.u[1] = u[1];
-  a.o[0] = a.c2, a.o[1] = a.c3;
+  a.odd = columns * a.c_stride / 2;
+  a.o[0] = a.c, a.o[1] = a.c + a.odd;
   a.o_stride = a.c_stride / 2;
   a.outputs = n / 2;
-  if ((e = run_conv<W, kParity>(a, columns, 2, s)) != cudaSuccess) return e;
+  if ((e = run_conv<W, kParity>(a, columns, a.u[1] ? 2 : 1, s)) != cudaSuccess) return e;
+  if (!a.u[1]) {
+    a.k[0] = kr.k[2];
+    a.u[0] = a.t;
+    a.o[0] = a.o[1];
+    if ((e = run_conv<W, kParity, false>(a, columns, 1, s)) != cudaSuccess) return e;
+  }
   a.k[0] = kr.k[0];
   a.u[0] = a.t;
   a.o[0] = a.c;

@@ -63,14 +63,15 @@ __global__ void fact_seg_prefix_kernel(uint32_t* __restrict__ seg, uint32_t nseg
   }
 }
 
-// fact[k] *= prefix of its segment; ifact[k] = 1 / k!; scale[k] = 2^(1-k) k!.
+// fact[k] *= prefix of its segment; ifact[k] = 1 / k!; scale[k] = 2^(1-k) k! (k < n_scale).
 __global__ void fact_finish_kernel(uint32_t* __restrict__ fact, const uint32_t* __restrict__ seg, uint32_t* __restrict__ ifact,
-                                   uint32_t* __restrict__ scale, uint64_t n) {
+                                   uint32_t* __restrict__ scale, uint64_t n, uint64_t n_scale) {
   const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const uint32_t f = m31_mul(fact[k], seg[k >> 10]);
   fact[k] = f;
   ifact[k] = m31_inv(f);
+  if (k >= n_scale) return;
   // 2^(1-k) = 2^((1 - k) mod 31)
   const uint32_t e = (uint32_t)((1 + 31 * ((k / 31) + 1) - k) % 31);
   scale[k] = m31_mul(f, pow2_m31(e));
@@ -162,11 +163,11 @@ __global__ void chebyshev_sum_kernel(const uint4* __restrict__ px, const uint4* 
   cy[m] = make_uint4(sy.a, sy.b, sy.c, sy.d);
 }
 
-cudaError_t launch_witness_tables(uint64_t n, uint32_t* fact, uint32_t* seg, uint32_t* ifact, uint32_t* scale, cudaStream_t s) {
+cudaError_t launch_witness_tables(uint64_t n, uint64_t n_scale, uint32_t* fact, uint32_t* seg, uint32_t* ifact, uint32_t* scale, cudaStream_t s) {
   const uint32_t nseg = (uint32_t)((n + 1023) / 1024);
   fact_segments_kernel<<<nseg, 1024, 0, s>>>(fact, seg, n);
   fact_seg_prefix_kernel<<<1, 32, 0, s>>>(seg, nseg);
-  fact_finish_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(fact, seg, ifact, scale, n);
+  fact_finish_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(fact, seg, ifact, scale, n, n_scale);
   return cudaGetLastError();
 }
 
