@@ -16,6 +16,7 @@
 
 #include "../../include/azk_cuda.h"
 #include "azk_internal.h"
+#include "azk_wait.h"
 
 struct azk_ctx {
   int device = 0;
@@ -165,27 +166,18 @@ struct Timer {
 // lane threads) set this for themselves; their waits then sleep early.
 inline thread_local bool t_shared_host = false;
 
-// Wait for an event by polling it.  A caller's own thread spins for up to 5 ms, as
-// CUDA's own synchronisation does (a sleep of 20 us lasts about 75 with the kernel's
-// timer slack: 25 to 100 us on calls whose device time is 30 to 250), and sleeps
-// between polls after that.  A server thread spins for a few polls, then sleeps
-// growing from 20 to 160 us, so a waiting thread takes little of a host core.
+// Wait for an event by polling it (azk_wait.h).
 // Not cudaEventSynchronize on a blocking-sync event, which sleeps until the
 // driver's completion interrupt: with the server's 32 workers waiting that way at
 // once, the device stopped starting work for 40-80 ms about every 2 s.
 inline void wait_event(cudaEvent_t e) {
-  const auto t0 = std::chrono::steady_clock::now();
-  for (int k = 0;; k++) {
-    const cudaError_t q = cudaEventQuery(e);
-    if (q == cudaSuccess) return;
-    if (q != cudaErrorNotReady) AZK_CU(q);
-    if (t_shared_host) {
-      if (k < 8) continue;
-      std::this_thread::sleep_for(std::chrono::microseconds(k < 24 ? 20 : k < 48 ? 50 : 160));
-    } else if (std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(5)) {
-      std::this_thread::sleep_for(std::chrono::microseconds(20));
-    }
-  }
+  poll_until(
+      [e] {
+        const cudaError_t q = cudaEventQuery(e);
+        if (q != cudaErrorNotReady) AZK_CU(q);
+        return q == cudaSuccess;
+      },
+      [](uint32_t us) { std::this_thread::sleep_for(std::chrono::microseconds(us)); }, t_shared_host, SpinPlaces::process());
 }
 
 // Wait for everything queued on a stream (wait_event on a per-thread event).
