@@ -531,8 +531,7 @@ struct Engine {
       AZK_CU(cudaMemsetAsync(found.p, 0xFF, 8, s));
       AZK_CU(launch_pcs_grind(d_inst(), i, start, chunk, found.as<unsigned long long>(), s));
       uint64_t nonce = ~0ull;
-      AZK_CU(cudaMemcpyAsync(&nonce, found.p, 8, cudaMemcpyDeviceToHost, s));
-      sync_stream(s);
+      read_back(s, {{&nonce, found.p, 8}});
       if (nonce != ~0ull) {
         h_inst[i].nonce = nonce;
         h_inst[i].has_nonce = 1;
@@ -613,12 +612,10 @@ struct Engine {
 
   void trace(uint32_t i, uint8_t* cm, uint32_t* ch, uint32_t* fl, uint32_t* qp) {
     const auto& c2 = cfg[i];
-    if (cm) AZK_CU(cudaMemcpyAsync(cm, arena.at<uint8_t>(off_cm[i]), 32ull * c2.rounds, cudaMemcpyDeviceToHost, s));
-    if (ch) AZK_CU(cudaMemcpyAsync(ch, arena.at<uint8_t>(off_ch[i]), 16ull * c2.rounds, cudaMemcpyDeviceToHost, s));
-    if (fl)
-      AZK_CU(cudaMemcpyAsync(fl, h_inst[i].layers + layer_offset(c2.logn, c2.rounds), 16ull << (c2.logn - c2.rounds), cudaMemcpyDeviceToHost, s));
-    if (qp) AZK_CU(cudaMemcpyAsync(qp, arena.at<uint8_t>(off_qp[i]), 4ull * c2.queries, cudaMemcpyDeviceToHost, s));
-    sync_stream(s);
+    read_back(s, {{cm, arena.at<uint8_t>(off_cm[i]), 32ull * c2.rounds},
+                  {ch, arena.at<uint8_t>(off_ch[i]), 16ull * c2.rounds},
+                  {fl, h_inst[i].layers + layer_offset(c2.logn, c2.rounds), 16ull << (c2.logn - c2.rounds)},
+                  {qp, arena.at<uint8_t>(off_qp[i]), 4ull * c2.queries}});
   }
 };
 
@@ -697,9 +694,15 @@ static void pcs_prove_common(azk_pcs_prover* p, bool coeffs, const uint8_t pub[3
   e.set_publics(pub);
   uint64_t sub = 0;
   e.run(coeffs, true, &sub, t);
-  AZK_CU(cudaMemcpyAsync(proof_out, e.h_inst[0].proof, len, proof_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, e.s));
-  sync_stream(e.s);
-  const double gs = e.finish_run();
+  double gs = 0;
+  if (proof_on_device) {
+    AZK_CU(cudaMemcpyAsync(proof_out, e.h_inst[0].proof, len, cudaMemcpyDeviceToDevice, e.s));
+    sync_stream(e.s);
+    gs = e.finish_run();
+  } else {
+    const HostResult proof = {proof_out, e.h_inst[0].proof, len};
+    read_back(e.s, &proof, 1, [&] { gs = e.finish_run(); });
+  }
   *proof_len = len;
   fill_stats(st, t, sub, gs);
 }
@@ -944,12 +947,13 @@ azk_status azk_batch_download_proofs(azk_batch* b, uint8_t* out, uint64_t cap) {
     Engine& e = b->eng;
     layout(e.has_proofs(), "a 64-byte-leaf batch produces commitments, challenges and final layers (azk_batch_trace), not proof bytes");
     uint64_t pos = 0;
+    std::vector<HostResult> proofs;
     for (size_t i = 0; i < e.cfg.size(); i++) {
       layout(pos + e.proof_len[i] <= cap, "proof buffer too small");
-      AZK_CU(cudaMemcpyAsync(out + pos, e.h_inst[i].proof, e.proof_len[i], cudaMemcpyDeviceToHost, e.s));
+      proofs.push_back({out + pos, e.h_inst[i].proof, e.proof_len[i]});
       pos += e.proof_len[i];
     }
-    sync_stream(e.s);
+    read_back(e.s, proofs.data(), proofs.size(), [] {});
   });
 }
 
@@ -983,10 +987,9 @@ azk_status azk_batch_download_each(azk_batch* b, void* const* outs) {
     layout(e.has_proofs(), "a 64-byte-leaf batch produces commitments, challenges and final layers (azk_batch_trace), not proof bytes");
     for (size_t i = 0; i < e.cfg.size(); i++) layout(outs[i] != nullptr);
     touch_pages(outs, e.proof_len);
-    for (size_t i = 0; i < e.cfg.size(); i++) {
-      AZK_CU(cudaMemcpyAsync(outs[i], e.h_inst[i].proof, e.proof_len[i], cudaMemcpyDeviceToHost, e.s));
-    }
-    sync_stream(e.s);
+    std::vector<HostResult> proofs;
+    for (size_t i = 0; i < e.cfg.size(); i++) proofs.push_back({outs[i], e.h_inst[i].proof, e.proof_len[i]});
+    read_back(e.s, proofs.data(), proofs.size(), [] {});
   });
 }
 
