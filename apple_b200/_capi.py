@@ -181,7 +181,7 @@ PROTOTYPES = {
     "azk_batch_prove": (I32, [P, P, I32, STATS]),
     "azk_batch_proof_sizes": (I32, [P, P, U64P]),
     "azk_batch_download_proofs": (I32, [P, P, U64]),
-    "azk_batch_download_each": (I32, [P, P]),
+    "azk_batch_download_each": (I32, [P, P, U64P]),
     "azk_batch_trace": (I32, [P, U32, P, P, P, P]),
     "azk_batch_set_profiling": (I32, [P, I32]),
     "azk_batch_profile": (I32, [P, P]),

@@ -979,13 +979,13 @@ static void touch_pages(void* const* outs, const std::vector<uint64_t>& bytes) {
   for (auto& t : pool) t.join();
 }
 
-azk_status azk_batch_download_each(azk_batch* b, void* const* outs) {
+azk_status azk_batch_download_each(azk_batch* b, void* const* outs, const uint64_t* capacities) {
   return guarded(b ? b->ctx : nullptr, [&] {
-    layout(b && outs);
+    layout(b && outs && capacities);
     std::lock_guard<std::mutex> lk(b->mu);
     Engine& e = b->eng;
     layout(e.has_proofs(), "a 64-byte-leaf batch produces commitments, challenges and final layers (azk_batch_trace), not proof bytes");
-    for (size_t i = 0; i < e.cfg.size(); i++) layout(outs[i] != nullptr);
+    for (size_t i = 0; i < e.cfg.size(); i++) layout(outs[i] && capacities[i] >= e.proof_len[i], "proof buffer too small");
     touch_pages(outs, e.proof_len);
     std::vector<HostResult> proofs;
     for (size_t i = 0; i < e.cfg.size(); i++) proofs.push_back({outs[i], e.h_inst[i].proof, e.proof_len[i]});

@@ -883,7 +883,8 @@ class BatchProver(_Plan):
             self._check(lib().azk_batch_download_proofs(self._h, _ptr(np.empty(1, np.uint8)), 0))
             return [b""] * len(self.proof_sizes)
         fresh = [_fresh_bytes(n) for n in self.proof_sizes]
-        self._check(lib().azk_batch_download_each(self._h, (_vp * len(fresh))(*[at for _, at in fresh])))
+        n = len(fresh)
+        self._check(lib().azk_batch_download_each(self._h, (_vp * n)(*[at for _, at in fresh]), (ctypes.c_uint64 * n)(*self.proof_sizes)))
         return [b for b, _ in fresh]
 
     def set_profiling(self, enabled: bool = True):

@@ -441,8 +441,9 @@ azk_status azk_batch_prove(azk_batch* b, const uint8_t* public_digests, int plai
 azk_status azk_batch_proof_sizes(azk_batch* b, uint64_t* sizes, uint64_t* total);
 /* Proof bytes of all instances, concatenated in instance order. */
 azk_status azk_batch_download_proofs(azk_batch* b, uint8_t* out, uint64_t capacity);
-/* The same into one buffer per instance (azk_batch_proof_sizes bytes each). */
-azk_status azk_batch_download_each(azk_batch* b, void* const* outs);
+/* The same into one buffer per instance, of capacities[i] bytes: azk_batch_proof_sizes
+ * at least, else nothing is written and AZK_ERR_INVALID_INPUT_LAYOUT is returned. */
+azk_status azk_batch_download_each(azk_batch* b, void* const* outs, const uint64_t* capacities);
 azk_status azk_batch_trace(azk_batch* b, uint32_t index, uint8_t* commitments, uint32_t* challenges, uint32_t* final_layer, uint32_t* query_pairs);
 /* Per-stage CUDA-event timing of the next proves (event pairs on the batch's own
  * stream around each stage; profiled proves launch the graph's kernel sequence
