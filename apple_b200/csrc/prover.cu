@@ -14,13 +14,13 @@
 #include <condition_variable>
 #include <deque>
 #include <set>
-#include <system_error>
 #include <thread>
 #include <tuple>
 #include <unordered_map>
 
 #include "azk_field.cuh"
 #include "azk_runtime.h"
+#include "azk_touch.h"
 #include "azk_tuned.h"
 
 using namespace azk;
@@ -955,28 +955,6 @@ azk_status azk_batch_download_proofs(azk_batch* b, uint8_t* out, uint64_t cap) {
     }
     read_back(e.s, proofs.data(), proofs.size(), [] {});
   });
-}
-
-// First touch of large fresh result buffers by several threads: a copy into them
-// otherwise takes its page faults one after another on the calling thread (61 MB of
-// proofs in fresh pages: 30 ms, 6 ms into touched ones).
-static void touch_pages(void* const* outs, const std::vector<uint64_t>& bytes) {
-  uint64_t total = 0;
-  for (uint64_t n : bytes) total += n;
-  const unsigned threads = std::min(8u, std::max(1u, std::thread::hardware_concurrency() / 2));
-  if (total < (4ull << 20) || threads < 2) return;
-  auto touch = [&](unsigned t) {
-    for (size_t i = t; i < bytes.size(); i += threads)
-      for (uint64_t k = 0; k < bytes[i]; k += 4096) static_cast<volatile uint8_t*>(outs[i])[k] = 0;
-  };
-  std::vector<std::thread> pool;
-  try {
-    for (unsigned t = 1; t < threads; t++) pool.emplace_back(touch, t);
-  } catch (const std::system_error&) {
-    // fewer threads: the copy faults in what is left
-  }
-  touch(0);
-  for (auto& t : pool) t.join();
 }
 
 azk_status azk_batch_download_each(azk_batch* b, void* const* outs, const uint64_t* capacities) {
