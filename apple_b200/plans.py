@@ -27,9 +27,9 @@ def _u8(data) -> np.ndarray:
     return np.frombuffer(bytes(data), dtype=np.uint8)
 
 
-_new_bytes = ctypes.pythonapi.PyBytes_FromStringAndSize
-_new_bytes.restype = ctypes.py_object
-_new_bytes.argtypes = [ctypes.c_void_p, ctypes.c_ssize_t]
+# A prototype of this module's own: ctypes.pythonapi's function objects are shared by
+# every package of the process.
+_new_bytes = ctypes.PYFUNCTYPE(ctypes.py_object, ctypes.c_void_p, ctypes.c_ssize_t)(("PyBytes_FromStringAndSize", ctypes.pythonapi))
 
 
 def _fresh_bytes(n: int):
