@@ -20,12 +20,6 @@ __host__ __device__ __forceinline__ uint32_t m31_reduce_once(uint32_t s) {
   const uint32_t t = s - kP;
   return t < s ? t : s;
 }
-__host__ __device__ __forceinline__ uint32_t m31_fold64(uint64_t v) {
-  // v < 2^62: two Mersenne folds then one conditional subtraction
-  uint64_t r = (v & kP) + (v >> 31);
-  uint32_t s = (uint32_t)((r & kP) + (r >> 31));
-  return s >= kP ? s - kP : s;
-}
 // Inputs are at most p (canonical values, or p itself as a redundant zero).
 __host__ __device__ __forceinline__ uint32_t m31_add(uint32_t a, uint32_t b) { return m31_reduce_once(a + b); }
 // a + (p - b) lies in [0, 2p): one reduction, no branch on a >= b.

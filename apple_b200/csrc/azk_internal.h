@@ -191,11 +191,6 @@ __host__ __device__ inline uint64_t proof_total_bytes(uint32_t logn, uint32_t ro
 // ---------------------------------------------------------------------------
 // Launchers (defined in the .cu files)
 // ---------------------------------------------------------------------------
-struct LaunchCfg {
-  uint32_t threads = 256;  // threads per CTA
-  uint32_t grid_cap = 0;   // 0: one CTA per work item
-};
-
 // Dependent launches: the kernel may be set up while the kernel ahead of it in the
 // stream ends, so a chain of short kernels does not pay the launch latency between
 // them.  Such a kernel calls dependent_begin() before it touches anything that an

@@ -98,21 +98,29 @@ __host__ __device__ __forceinline__ void rho_pi_all(const uint64_t (&a)[25], con
 // 0xD2 = a ^ (~b & c).  Written out so that theta's column terms are folded into
 // each lane's XOR (one LOP3 per half) instead of being combined first and XORed
 // in afterwards (two), which is the 180-operation round the roofline counts.
-__device__ __forceinline__ uint32_t lop3_xor3(uint32_t a, uint32_t b, uint32_t c) {
+__host__ __device__ __forceinline__ uint32_t lop3_xor3(uint32_t a, uint32_t b, uint32_t c) {
+#if defined(__CUDA_ARCH__)
   uint32_t r;
   asm("lop3.b32 %0, %1, %2, %3, 0x96;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
   return r;
+#else
+  return a ^ b ^ c;
+#endif
 }
-__device__ __forceinline__ uint32_t lop3_chi(uint32_t a, uint32_t b, uint32_t c) {
+__host__ __device__ __forceinline__ uint32_t lop3_chi(uint32_t a, uint32_t b, uint32_t c) {
+#if defined(__CUDA_ARCH__)
   uint32_t r;
   asm("lop3.b32 %0, %1, %2, %3, 0xD2;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
   return r;
+#else
+  return a ^ (~b & c);
+#endif
 }
-__device__ __forceinline__ uint64_t xor3_64(uint64_t a, uint64_t b, uint64_t c) {
+__host__ __device__ __forceinline__ uint64_t xor3_64(uint64_t a, uint64_t b, uint64_t c) {
   return ((uint64_t)lop3_xor3((uint32_t)(a >> 32), (uint32_t)(b >> 32), (uint32_t)(c >> 32)) << 32) |
          lop3_xor3((uint32_t)a, (uint32_t)b, (uint32_t)c);
 }
-__device__ __forceinline__ uint64_t chi_64(uint64_t a, uint64_t b, uint64_t c) {
+__host__ __device__ __forceinline__ uint64_t chi_64(uint64_t a, uint64_t b, uint64_t c) {
   return ((uint64_t)lop3_chi((uint32_t)(a >> 32), (uint32_t)(b >> 32), (uint32_t)(c >> 32)) << 32) |
          lop3_chi((uint32_t)a, (uint32_t)b, (uint32_t)c);
 }
@@ -173,7 +181,6 @@ __host__ __device__ __forceinline__ void keccak_f1600(uint64_t (&a)[25]) {
 #endif
 }
 
-#if defined(__CUDACC__)
 // ---------------------------------------------------------------------------
 // A one-block digest: lanes outside NZ (a bit per lane) are zero before the
 // permutation and only lanes 0..3 are wanted after it, so the first round XORs what
@@ -252,7 +259,6 @@ __device__ __forceinline__ void keccak_digest(uint64_t (&a)[25], uint64_t (&out)
   keccak_first_round<NZ>(a, kKeccakRC[0]);
   keccak_digest_rest(a, out);
 }
-#endif
 
 // Sponge padding constants for one 136-byte block (rate of SHA3-256).
 static constexpr int kRateLanes = 17;

@@ -26,7 +26,9 @@ namespace azk {
 // word) and (r - 1) / 2 (the new odd word).
 // ---------------------------------------------------------------------------
 // Even bits of each 16-bit half of x to its low byte, odd bits to its high byte (and
-// back); the bytes of both words of a lane then move in two permutes.
+// back), by exchanging neighbouring fields of doubling width (the unshuffle of H. S.
+// Warren, Hacker's Delight, 7-2); the bytes of both words of a lane then move in two
+// permutes.
 __host__ __device__ __forceinline__ uint32_t unshuffle16(uint32_t x) {
   uint32_t t;
   t = (x ^ (x >> 1)) & 0x22222222u; x ^= t ^ (t << 1);

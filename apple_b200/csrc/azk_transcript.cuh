@@ -96,16 +96,6 @@ __host__ __device__ inline void circle_frame(FrameBuf& f, uint8_t type) {
   fb_u32(f, 1);
   fb_u8(f, type);
 }
-// QM31 fold-chain base frame: u32 len || "AppleZKProver.QM31FRI.FoldChain" || u32 1 || u8 type
-__host__ __device__ inline void qm31_frame(FrameBuf& f, uint8_t type) {
-  const char dom[] = "AppleZKProver.QM31FRI.FoldChain";
-  f.n = 0;
-  fb_u32(f, 31);
-  fb_str(f, dom, 31);
-  fb_u32(f, 1);
-  fb_u8(f, type);
-}
-
 // Circle V1 round: commitment frame, root, challenge frame, squeeze 4 limbs.
 __host__ __device__ inline void circle_round(Transcript& t, uint32_t round, const uint64_t (&root)[4], uint32_t (&ch)[4]) {
   FrameBuf f;
@@ -115,24 +105,6 @@ __host__ __device__ inline void circle_round(Transcript& t, uint32_t round, cons
   tr_absorb(t, f.b, f.n);
   tr_absorb_digest(t, root);
   circle_frame(f, 4);
-  fb_u32(f, round);
-  fb_u32(f, 2147483647u);
-  fb_u32(f, 4);
-  tr_absorb(t, f.b, f.n);
-  tr_squeeze_u32(t, 4, 2147483647u, ch);
-}
-
-// QM31 fold-chain round (QM31FRIFold.swift:203-213).
-__host__ __device__ inline void qm31_round(Transcript& t, uint32_t round, uint64_t inCount, const uint64_t (&root)[4], uint32_t (&ch)[4]) {
-  FrameBuf f;
-  qm31_frame(f, 1);
-  fb_u32(f, round);
-  fb_u64(f, inCount);
-  fb_u64(f, inCount / 2);
-  fb_u32(f, 32);
-  tr_absorb(t, f.b, f.n);
-  tr_absorb_digest(t, root);
-  qm31_frame(f, 2);
   fb_u32(f, round);
   fb_u32(f, 2147483647u);
   fb_u32(f, 4);

@@ -86,20 +86,6 @@ struct WarpSponge {
   }
   // Word `lane` of a padded 32-byte message.
   __device__ __forceinline__ uint64_t digest_word(const uint64_t* d) const { return lane < 4 ? d[lane] : lane == 4 ? 0x06ull : lane == 16 ? kPadEnd : 0ull; }
-  // A message of `bytes` bytes (a multiple of 8) in global memory.
-  __device__ __forceinline__ void absorb_words(const uint64_t* p, uint64_t bytes) {
-    const uint64_t n = bytes / 8;
-    for (uint64_t k = 0; k <= n; k += 17) {  // the last block holds fewer than 17 words, and the padding
-      const uint64_t left = n - k;
-      uint64_t w = 0;
-      if (lane < 17 && lane < left) w = p[k + lane];
-      if (left < 17) {
-        if (lane == left) w = 0x06;
-        if (lane == 16) w ^= kPadEnd;
-      }
-      absorb(w);
-    }
-  }
   // Four field elements (challenge limbs), in every lane; the state is unchanged.
   __device__ __forceinline__ void squeeze4_m31(uint32_t (&out)[4]) {
     const uint64_t w0 = __shfl_sync(0xffffffffu, a, 0), w1 = __shfl_sync(0xffffffffu, a, 1);

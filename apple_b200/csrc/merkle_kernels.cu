@@ -19,10 +19,6 @@
 
 namespace azk {
 
-struct Dig {
-  uint64_t w[4];
-};
-
 __device__ __forceinline__ void st_dig(uint64_t* p, const uint64_t (&d)[4]) {
   reinterpret_cast<ulonglong2*>(p)[0] = make_ulonglong2(d[0], d[1]);
   reinterpret_cast<ulonglong2*>(p)[1] = make_ulonglong2(d[2], d[3]);
@@ -467,18 +463,6 @@ __device__ __noinline__ void pair_levels(uint64_t* a, uint64_t* b, uint64_t* top
       src = dst;
       dst = t;
     }
-  }
-}
-
-// A parent node by one warp: children at src (8 lanes), the digest to dst (shared)
-// and node (global).
-__device__ __forceinline__ void warp_parent(const WarpKeccak& kf, const uint64_t* src, uint64_t* dst, uint64_t* node) {
-  const uint32_t lane = threadIdx.x & 31;
-  uint64_t a = lane < 8 ? src[lane] : lane == 8 ? 0x06ull : lane == 16 ? kPadEnd : 0ull;
-  kf.permute_small(a);
-  if (lane < 4) {
-    dst[lane] = a;
-    node[lane] = a;
   }
 }
 
