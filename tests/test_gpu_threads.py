@@ -46,7 +46,13 @@ def _codeword(ctx, seed):
     return lambda: p.execute_coefficients(x).tobytes()
 
 
-@pytest.mark.parametrize("make", [_prove, _prove_evaluations, _hash, _commit, _codeword])
+def _large_codeword(ctx, seed):
+    p = azk.CircleCodewordPlan(ctx, 18)
+    x = np.random.default_rng(seed).integers(0, G.P, (1 << 18, 4), dtype=np.uint32)
+    return lambda: p.execute_coefficients(x)[::64].tobytes()
+
+
+@pytest.mark.parametrize("make", [_prove, _prove_evaluations, _hash, _commit, _codeword, _large_codeword])
 def test_every_thread_gets_its_calls_through(ctx, make):
     calls = [make(ctx, seed) for seed in range(THREADS)]
     want = [hashlib.sha256(call()).digest() for call in calls]
@@ -69,8 +75,8 @@ def test_every_thread_gets_its_calls_through(ctx, make):
 
 
 def test_results_larger_than_a_threads_landing(ctx, oracle):
-    """Results that cross in one copy to the caller's memory instead (4 MB of digests, a
-    4 MB codeword), small and large ones from one thread in turn."""
+    """Results that cross in pieces (4 MB of digests, a 4 MB codeword, batches of proofs whose
+    sizes are no multiple of a piece), small and large ones from one thread in turn."""
     rng = np.random.default_rng(3)
     for count in (1 << 10, 1 << 17, 3):
         m = rng.integers(0, 256, (count, 32), dtype=np.uint8)
@@ -79,3 +85,14 @@ def test_results_larger_than_a_threads_landing(ctx, oracle):
             assert got[i].tobytes() == hashlib.sha3_256(m[i].tobytes()).digest()
     x = rng.integers(0, G.P, (1 << 18, 4), dtype=np.uint32)
     assert np.array_equal(azk.CircleCodewordPlan(ctx, 18).execute_coefficients(x), oracle.fft_evaluate(18, x))
+    logs = [16] * 24
+    counts = [(1 << lg) >> 2 for lg in logs]
+    c = rng.integers(0, G.P, (sum(counts), 4), dtype=np.uint32)
+    b = azk.BatchProver(ctx, logs, [10] * len(logs), 2, 16)
+    b.upload(c, list(np.cumsum([0] + counts[:-1])), counts)
+    b.prove(PUB * len(logs))
+    assert sum(b.proof_sizes) > 2 << 20  # more than a thread's landing
+    p = azk.CirclePCSFRIProver(ctx, 16, 2, 16, 10)
+    proofs = b.proofs()
+    for i in (0, 7, 23):
+        assert proofs[i] == p.prove_coefficients(c[i << 14:(i + 1) << 14], PUB)
