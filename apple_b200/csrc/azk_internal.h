@@ -333,6 +333,7 @@ cudaError_t launch_scan_inputs(const ScanJob* d_jobs, uint32_t njobs, uint64_t m
 cudaError_t launch_fold_jobs(const FoldJob* d_jobs, const uint2* d_work, uint32_t nwork, cudaStream_t s);
 cudaError_t launch_fold_qm31_inv(const uint4* prev, const uint4* inv, const uint32_t* ch, uint4* out, uint64_t n_out, cudaStream_t s);
 static constexpr uint32_t kFoldTile = 2048, kFoldTileRounds = 11;
+// scratch: n / 16 values hold every layer between launches.
 cudaError_t launch_fold_chain(const uint4* prev, uint64_t n, const uint4* inv, const uint32_t* m31_inv, const uint32_t* ch, uint32_t rounds, uint4* scratch,
                               uint4* out, cudaStream_t s);
 cudaError_t launch_pcs_base(const PcsInstance* d_inst, uint32_t ninst, cudaStream_t s);

@@ -37,7 +37,7 @@ struct azk_ctx {
     uint32_t* inv = nullptr;
   };
   std::map<uint32_t, Domain> domains;
-  // Scratch of azk_sumcheck_prove for tables of at most 2^kSumcheckKeptLog words (12.6
+  // Scratch of azk_sumcheck_prove for tables of at most 2^kSumcheckKeptLog words (8.4
   // MB on the device, 4.2 MB page-locked), used under `mu`, freed with the context;
   // larger tables take their own for the call.
   static constexpr uint32_t kSumcheckKeptLog = 20;

@@ -7,7 +7,8 @@
 // CircleFRITranscriptV1 (CircleProofFormat.swift:906-975) and
 // QM31FRIFoldTranscriptFraming (QM31FRIFold.swift:769-862).
 //
-// Transcript work is a handful of permutations per round, run by one thread.
+// A handful of permutations per round.  This is the one-thread form (nonce search, rare
+// rejections, host checks); azk_transcript_warp.cuh has the warp form that proofs run.
 #pragma once
 #include <stdint.h>
 #include "azk_keccak.cuh"
@@ -96,7 +97,8 @@ __host__ __device__ inline void circle_frame(FrameBuf& f, uint8_t type) {
   fb_u32(f, 1);
   fb_u8(f, type);
 }
-// Circle V1 round: commitment frame, root, challenge frame, squeeze 4 limbs.
+// Circle V1 round: commitment frame, root, challenge frame, squeeze 4 limbs.  The
+// one-thread form that the host check runs; the kernels' is azk_transcript_warp.cuh's.
 __host__ __device__ inline void circle_round(Transcript& t, uint32_t round, const uint64_t (&root)[4], uint32_t (&ch)[4]) {
   FrameBuf f;
   circle_frame(f, 3);

@@ -557,8 +557,8 @@ cudaError_t launch_fold_qm31_inv(const uint4* prev, const uint4* inv, const uint
 // all rounds are one factor 2^-rounds on the outputs.  The first rounds are bound by
 // integer issue (about 85 instructions per fold), the last by latency.  A launch per
 // round with 16-byte inverses read and wrote every layer and left all but the first
-// few rounds to launch latency: 16 rounds of 2^22 values took 120 us, 49 us so; 10
-// rounds of 2^16 45 and 15 us.
+// few rounds to launch latency: 16 rounds of 2^22 values took 120 us, 45 us so; 10
+// rounds of 2^16 45 and 13 us.
 template <bool Q>
 struct FoldInv {
   using type = uint32_t;
@@ -646,12 +646,14 @@ __global__ void __launch_bounds__(256, 4) fold_chain_kernel(const uint4* prev, u
   }
 }
 
-// All `rounds` folds of n values: kFoldTileRounds a launch, the values between two
-// launches in `scratch` (n >> kFoldTileRounds of them).  `m31_inv`: inverse layers of
-// M31 words, else `inv` of QM31 values.  ch: 4 limbs per round on the device.
+// All `rounds` folds of n values, up to kFoldTileRounds a launch.  `scratch`: the values
+// between launches, one layer behind the other (the sum of the layers written between
+// launches: less than n / 16 values in all).  `m31_inv`: inverse layers of M31 words, else
+// `inv` of QM31 values.  ch: 4 limbs per round on the device.
 // A long input is bound by its first rounds, and a CTA's last rounds are a chain with
 // a few threads busy: from kFoldLong values on a launch stops after kFoldLongRounds
-// (2^22 values, 16 rounds: 11 + 5 rounds 52 us, 5 + 11 rounds 47 us).
+// (16 rounds between events: 2^24 values 174 us in launches of 11 and 5 rounds, 135 in
+// 5, 5 and 6; 2^22 51 and 45; 2^20, one long launch, 22.7 and 23.9).
 static constexpr uint64_t kFoldLong = 1ull << 19;
 static constexpr uint32_t kFoldLongRounds = 5;
 cudaError_t launch_fold_chain(const uint4* prev, uint64_t n, const uint4* inv, const uint32_t* m31_inv, const uint32_t* ch, uint32_t rounds, uint4* scratch,

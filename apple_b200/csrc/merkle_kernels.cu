@@ -747,7 +747,7 @@ cudaError_t launch_tree_jobs(const TreeJob* d_jobs, const uint2* d_work, uint32_
 }
 
 // One raw-leaf tree, job by value, 256 threads, treelets of at most 2^9 leaves
-// (24 KiB of dynamic shared memory: under the default limit, no opt-in needed).
+// (12 KiB of dynamic shared memory: under the default limit, no opt-in needed).
 cudaError_t launch_tree_direct_raw(const TreeJob& job, cudaStream_t s) {
   if (job.tile_log > 9 || (job.logn > 0 && job.tile_log == 0)) return cudaErrorInvalidValue;
   uint32_t tl = job.tile_log < job.logn ? job.tile_log : job.logn;

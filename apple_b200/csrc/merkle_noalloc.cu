@@ -24,7 +24,7 @@
 namespace azk {
 
 static constexpr uint64_t kNoAllocMaxLeaves = 1ull << 16;
-static constexpr uint32_t kNoAllocTileLog = 9;  // 24 KiB of shared memory: under the default limit
+static constexpr uint32_t kNoAllocTileLog = 9;  // 12 KiB of dynamic shared memory: under the default limit
 // Arrival counters: with treelets of min(logn, 9) levels a tree of at most 2^16
 // leaves has at most 128 treelets, and tree_counter_count() bounds the counters
 // (treelets + 64); inner nodes: at most 2^16 - 1 digests.

@@ -153,7 +153,7 @@ __device__ __forceinline__ uint32_t group_sum_m31(const G& grp, uint32_t v, uint
 // One table on one group.  The group's first warp computes the statement's word
 // digest while its other warps sum the table's even and odd entries (round 0's
 // two sums; together the claimed sum), which need no challenge.  Then each round
-// is a transcript round by the group's thread 0 (round frame, challenge frame,
+// is a transcript round by the group's first warp (round frame, challenge frame,
 // squeeze one word mod p) and one pass over the table that folds it,
 // t'[i] = (1 - r) t[2i] + r t[2i+1], and sums the folded table's even and odd
 // entries for the next round, so after the digest the table is read once per
