@@ -15,6 +15,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <optional>
 #include <stdexcept>
 #include <string>
 #include <thread>
@@ -23,6 +24,22 @@
 #include "../../include/azk_cuda.h"
 #include "azk_internal.h"
 #include "azk_wait.h"
+
+// Page-locked memory that results cross to the host through, and an event for each half
+// of it.
+struct azk_landing {
+  void* p = nullptr;
+  uint64_t n = 0;
+  cudaEvent_t half[2] = {nullptr, nullptr};
+  azk_landing() = default;
+  azk_landing(const azk_landing&) = delete;
+  azk_landing& operator=(const azk_landing&) = delete;
+  ~azk_landing() {
+    if (p) cudaFreeHost(p);
+    for (auto& e : half)
+      if (e) cudaEventDestroy(e);
+  }
+};
 
 struct azk_ctx {
   int device = 0;
@@ -44,6 +61,11 @@ struct azk_ctx {
   void* sumcheck_dev = nullptr;
   void* sumcheck_pin = nullptr;
   uint64_t sumcheck_dev_bytes = 0, sumcheck_pin_bytes = 0;
+  // Landings that no call is using, at most kLandingsKept (of at most 2 MB each), freed
+  // with the context.
+  static constexpr size_t kLandingsKept = 32;
+  std::mutex landing_mu;
+  std::vector<std::unique_ptr<azk_landing>> landings;
 };
 
 namespace azk {
@@ -318,10 +340,10 @@ struct HostPinned {
 
 // Results on their way to a caller's memory: the copies are queued on `s`, the stream
 // is waited for, check() may refuse the results, and `dst` (null: skipped) is written.
-// They cross through page-locked memory of the calling thread, at once where they fit,
-// in pieces where they do not.  A copy to pageable memory holds a lock of the
-// driver while it waits, and the driver does not hand that lock out in turn: with a
-// dozen threads in calls that end in such copies, some threads got no call through until
+// They cross through page-locked memory that the context keeps, at once up to
+// kLandingPiece, in pieces above.  A copy to pageable memory holds a lock
+// of the driver while it waits, and the driver does not hand that lock out in turn: with
+// a dozen threads in calls that end in such copies, some threads got no call through until
 // the others stopped (32 threads with a 2^14 prover each: all but six, 7,900 proofs/s in
 // all against 19,700 so).
 struct HostResult {
@@ -329,51 +351,66 @@ struct HostResult {
   const void* src;
   uint64_t bytes;
 };
-static constexpr uint64_t kThreadLanding = 2ull << 20, kLandingPiece = 1ull << 20;
-struct ThreadLanding {
-  void* p = nullptr;
-  uint64_t n = 0;
-  cudaEvent_t half[2] = {nullptr, nullptr};
-  int dev = -1;
-  ~ThreadLanding() {
-    if (p) cudaFreeHost(p);
-    drop_events();
-  }
-  void drop_events() {
-    for (auto& e : half) {
-      if (e) cudaEventDestroy(e);
-      e = nullptr;
-    }
-  }
-  // At least `bytes` page-locked bytes, or null.
-  uint8_t* ensure(uint64_t bytes) {
-    if (bytes > n) {
-      uint64_t m = 16384;
-      while (m < bytes) m *= 2;
-      if (p) cudaFreeHost(p);
-      p = nullptr;
-      n = 0;
-      if (cudaHostAlloc(&p, m, cudaHostAllocPortable) != cudaSuccess) {
-        cudaGetLastError();
-        p = nullptr;
-        return nullptr;
+static constexpr uint64_t kLandingBytes = 2ull << 20, kLandingPiece = kLandingBytes / 2;
+// One of the context's landings, for the duration of a call.
+struct LandingLease {
+  azk_ctx* ctx;
+  std::unique_ptr<azk_landing> l;
+  LandingLease(azk_ctx* c, uint64_t bytes) : ctx(c) {
+    {
+      // the smallest one that is large enough, else the largest
+      std::lock_guard<std::mutex> lk(c->landing_mu);
+      auto& v = c->landings;
+      size_t best = v.size();
+      for (size_t i = 0; i < v.size(); i++) {
+        const bool fits = v[i]->n >= bytes;
+        if (best == v.size() || (fits ? v[best]->n < bytes || v[i]->n < v[best]->n : v[best]->n < bytes && v[i]->n > v[best]->n)) best = i;
       }
-      n = m;
+      if (best < v.size()) {
+        l = std::move(v[best]);
+        v[best] = std::move(v.back());
+        v.pop_back();
+      }
     }
-    return static_cast<uint8_t*>(p);
+    if (!l) l = std::make_unique<azk_landing>();
+    if (l->n >= bytes) return;
+    uint64_t m = 16384;
+    while (m < bytes) m *= 2;
+    if (l->p) cudaFreeHost(l->p);
+    l->p = nullptr;
+    l->n = 0;
+    if (cudaHostAlloc(&l->p, m, cudaHostAllocDefault) != cudaSuccess) {
+      cudaGetLastError();
+      l->p = nullptr;
+    } else {
+      l->n = m;
+    }
   }
-  void ensure_events() {
-    int d = 0;
-    AZK_CU(cudaGetDevice(&d));
-    if (half[1] && dev == d) return;
-    drop_events();
-    for (auto& e : half) AZK_CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    dev = d;
+  ~LandingLease() {
+    std::lock_guard<std::mutex> lk(ctx->landing_mu);
+    if (l->p && ctx->landings.size() < azk_ctx::kLandingsKept) ctx->landings.push_back(std::move(l));  // reserved by azk_ctx_create
   }
-  static ThreadLanding& mine() {
-    thread_local ThreadLanding l;
-    return l;
+  LandingLease(const LandingLease&) = delete;
+  LandingLease& operator=(const LandingLease&) = delete;
+  // Page-locked bytes, or null where there are none to be had.
+  uint8_t* bytes() const { return static_cast<uint8_t*>(l->p); }
+  cudaEvent_t* halves() const {
+    for (auto& e : l->half)
+      if (!e) AZK_CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    return l->half;
   }
+};
+// Waits for the stream unless told that it is idle: an error must not leave copies in
+// flight into a landing that the next call takes.
+struct SettleStream {
+  cudaStream_t s;
+  bool idle = false;
+  explicit SettleStream(cudaStream_t st) : s(st) {}
+  ~SettleStream() {
+    if (!idle) cudaStreamSynchronize(s);
+  }
+  SettleStream(const SettleStream&) = delete;
+  SettleStream& operator=(const SettleStream&) = delete;
 };
 // memcpy of a piece of a large result, past the caches where the host has such stores:
 // lines of the destination are not read first (a 2^20 codeword of 16 MB to the host: 2.66
@@ -398,40 +435,71 @@ inline void copy_past_caches(uint8_t* dst, const uint8_t* src, uint64_t n) {
   std::memcpy(dst, src, n);
 #endif
 }
+// Host memory that a copy reaches without the driver's staging.
+inline bool page_locked(const void* p) {
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type != cudaMemoryTypeUnregistered;
+}
+static constexpr uint64_t kLandingSmall = 32ull << 10;  // results up to here are not worth the question
 template <class Check>
-void read_back(cudaStream_t s, const HostResult* r, size_t n, Check check) {
+void read_back(azk_ctx* ctx, cudaStream_t s, const HostResult* results, size_t count, Check check) {
+  // results that need a landing, and those for page-locked memory of the caller's, which
+  // are copied straight to it once check() has passed (it may run twice then)
+  std::optional<LandingLease> lease;  // given back after `settle`
+  SettleStream settle(s);
+  std::vector<HostResult> r, straight;
   uint64_t total = 0;
-  for (size_t i = 0; i < n; i++) total += r[i].dst ? align_up(r[i].bytes, 16) : 0;
-  ThreadLanding& l = ThreadLanding::mine();
-  uint8_t* const landing = l.ensure(total <= kThreadLanding ? total : kThreadLanding);
-  if (landing && total <= kThreadLanding) {
+  for (size_t i = 0; i < count; i++) {
+    if (!results[i].dst || !results[i].bytes) continue;
+    const bool locked = results[i].bytes > kLandingSmall && page_locked(results[i].dst);
+    (locked ? straight : r).push_back(results[i]);
+    if (!locked) total += align_up(results[i].bytes, 16);
+  }
+  const size_t n = r.size();
+  if (!straight.empty() || n == 0) {
+    sync_stream(s);
+    check();
+    for (const HostResult& h : straight) AZK_CU(cudaMemcpyAsync(h.dst, h.src, h.bytes, cudaMemcpyDeviceToHost, s));
+    if (n == 0) {
+      if (!straight.empty()) sync_stream(s);
+      settle.idle = true;
+      return;
+    }
+  }
+  lease.emplace(ctx, total <= kLandingPiece ? total : kLandingBytes);
+  uint8_t* const landing = lease->bytes();
+  if (landing && total <= kLandingPiece) {
     uint64_t at = 0;
     for (size_t i = 0; i < n; i++) {
-      if (!r[i].dst || !r[i].bytes) continue;
       AZK_CU(cudaMemcpyAsync(landing + at, r[i].src, r[i].bytes, cudaMemcpyDeviceToHost, s));
       at += align_up(r[i].bytes, 16);
     }
     sync_stream(s);
+    settle.idle = true;
     check();
     at = 0;
     for (size_t i = 0; i < n; i++) {
-      if (!r[i].dst || !r[i].bytes) continue;
       std::memcpy(r[i].dst, landing + at, r[i].bytes);
       at += align_up(r[i].bytes, 16);
     }
     return;
   }
-  if (!landing) {  // no page-locked memory to be had
+  if (!landing) {
     sync_stream(s);
     check();
-    for (size_t i = 0; i < n; i++)
-      if (r[i].dst && r[i].bytes) AZK_CU(cudaMemcpyAsync(r[i].dst, r[i].src, r[i].bytes, cudaMemcpyDeviceToHost, s));
+    for (const HostResult& h : r) AZK_CU(cudaMemcpyAsync(h.dst, h.src, h.bytes, cudaMemcpyDeviceToHost, s));
     sync_stream(s);
+    settle.idle = true;
     return;
   }
-  // In pieces, one copied out while the next one is in flight.
-  l.ensure_events();
-  constexpr uint64_t kHalf = kLandingPiece;
+  // In pieces, one copied out while the next one is in flight; small ones where the
+  // first one's way and the last one's copying would otherwise be most of the time.
+  const uint64_t most = total >= 4 * kLandingPiece ? kLandingPiece : kLandingPiece / 4;
+  cudaEvent_t* const half = lease->halves();
   struct Piece {
     uint8_t* dst = nullptr;
     uint64_t bytes = 0;
@@ -440,29 +508,26 @@ void read_back(cudaStream_t s, const HostResult* r, size_t n, Check check) {
   uint32_t k = 0;
   auto finish = [&](uint32_t h) {
     if (!piece[h].dst) return;
-    wait_event(l.half[h]);
+    wait_event(half[h]);
     if (!checked) check();
     checked = true;
-    copy_past_caches(piece[h].dst, landing + h * kHalf, piece[h].bytes);
+    copy_past_caches(piece[h].dst, landing + h * kLandingPiece, piece[h].bytes);
     piece[h].dst = nullptr;
   };
   for (size_t i = 0; i < n; i++) {
-    if (!r[i].dst) continue;
-    for (uint64_t at = 0; at < r[i].bytes; at += kHalf, k++) {
+    for (uint64_t at = 0; at < r[i].bytes; at += most, k++) {
       const uint32_t h = k & 1;
       finish(h);
-      piece[h] = {static_cast<uint8_t*>(r[i].dst) + at, r[i].bytes - at < kHalf ? r[i].bytes - at : kHalf};
-      AZK_CU(cudaMemcpyAsync(landing + h * kHalf, static_cast<const uint8_t*>(r[i].src) + at, piece[h].bytes, cudaMemcpyDeviceToHost, s));
-      AZK_CU(cudaEventRecord(l.half[h], s));
+      piece[h] = {static_cast<uint8_t*>(r[i].dst) + at, std::min(r[i].bytes - at, most)};
+      AZK_CU(cudaMemcpyAsync(landing + h * kLandingPiece, static_cast<const uint8_t*>(r[i].src) + at, piece[h].bytes, cudaMemcpyDeviceToHost, s));
+      AZK_CU(cudaEventRecord(half[h], s));
     }
   }
   finish(k & 1);
   finish((k + 1) & 1);
-  sync_stream(s);
+  settle.idle = true;  // every piece was waited for
 }
-inline void read_back(cudaStream_t s, std::initializer_list<HostResult> r) {
-  read_back(s, r.begin(), r.size(), [] {});
-}
+inline void read_back(azk_ctx* ctx, cudaStream_t s, std::initializer_list<HostResult> r) { read_back(ctx, s, r.begin(), r.size(), [] {}); }
 
 inline void fill_stats(azk_stats* st, const Timer& t, uint64_t submit_ns, double gpu_s) {
   if (!st) return;

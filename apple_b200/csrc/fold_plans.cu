@@ -98,7 +98,7 @@ azk_status azk_qm31_fold_plan_execute(azk_qm31_fold_plan* p, const uint32_t* eva
     AZK_CU(cudaMemcpyAsync(p->ev.p, evaluations, kQ * p->n_in, cudaMemcpyHostToDevice, p->s));
     AZK_CU(cudaMemcpyAsync(p->inv.p, inverse_points, kQ * p->n_out, cudaMemcpyHostToDevice, p->s));
     double gs = qm31_fold_run(p, p->ev.as<uint4>(), p->inv.as<uint4>(), p->out.as<uint4>(), challenge);
-    read_back(p->s, {{out, p->out.p, kQ * p->n_out}});
+    read_back(p->ctx, p->s, {{out, p->out.p, kQ * p->n_out}});
     fill_stats(st, t, 0, gs);
   });
 }
@@ -363,7 +363,7 @@ azk_status azk_fold_chain_plan_execute(azk_fold_chain_plan* p, const uint32_t* e
     GpuTimer g(p->s);
     chain_fold_all(p, p->ev.as<uint4>(), p->inv.as<uint4>(), p->out.as<uint4>());
     g.stop();
-    read_back(p->s, {{final_out, p->out.p, kQ * p->n_out}});
+    read_back(p->ctx, p->s, {{final_out, p->out.p, kQ * p->n_out}});
     fill_stats(st, t, 0, g.seconds());
   });
 }
@@ -405,7 +405,7 @@ azk_status azk_fold_chain_plan_execute_transcript(azk_fold_chain_plan* p, const 
     AZK_CU(launch_transcript_rounds_given(p->tr.as<Transcript>(), kRootQM31Round, p->cm.as<uint64_t>(), p->rounds, p->n_in, p->ch.as<uint32_t>(), p->s));
     chain_fold_all(p, p->ev.as<uint4>(), p->inv.as<uint4>(), p->out.as<uint4>());
     g.stop();
-    read_back(p->s, {{final_out, p->out.p, kQ * p->n_out}, {challenges_out, p->ch.p, 16ull * p->rounds}});
+    read_back(p->ctx, p->s, {{final_out, p->out.p, kQ * p->n_out}, {challenges_out, p->ch.p, 16ull * p->rounds}});
     fill_stats(st, t, 0, g.seconds());
   });
 }
@@ -451,7 +451,7 @@ azk_status azk_fold_chain_plan_execute_merkle(azk_fold_chain_plan* p, const uint
     GpuTimer g(p->s);
     chain_merkle(p, p->ev.as<uint4>(), p->inv.as<uint4>(), p->layers.as<uint4>(), false, p->out.as<uint4>(), nullptr);
     g.stop();
-    read_back(p->s, {{final_out, p->out.p, kQ * p->n_out},
+    read_back(p->ctx, p->s, {{final_out, p->out.p, kQ * p->n_out},
                      {commitments_out, p->cm.p, 32ull * p->rounds},
                      {challenges_out, p->ch.p, 16ull * p->rounds}});
     fill_stats(st, t, 0, g.seconds());
@@ -472,7 +472,7 @@ azk_status azk_fold_chain_plan_execute_merkle_readback(azk_fold_chain_plan* p, c
     chain_merkle(p, dev_q(dev_evaluations, evaluations_offset), dev_q(dev_inverse_layers, inverse_offset), p->layers.as<uint4>(), false,
                  p->out.as<uint4>(), nullptr);
     g.stop();
-    read_back(p->s, {{final_out, p->out.p, kQ * p->n_out},
+    read_back(p->ctx, p->s, {{final_out, p->out.p, kQ * p->n_out},
                      {commitments_out, p->cm.p, 32ull * p->rounds},
                      {challenges_out, p->ch.p, 16ull * p->rounds}});
     fill_stats(st, t, 0, g.seconds());
@@ -538,7 +538,7 @@ azk_status azk_fold_chain_plan_challenges(azk_fold_chain_plan* p, uint32_t* chal
   return guarded(p ? p->ctx : nullptr, [&] {
     layout(p && challenges_out);
     std::lock_guard<std::mutex> lk(p->mu);
-    read_back(p->s, {{challenges_out, p->ch.p, 16ull * p->rounds}});
+    read_back(p->ctx, p->s, {{challenges_out, p->ch.p, 16ull * p->rounds}});
   });
 }
 
@@ -673,11 +673,11 @@ azk_status azk_query_extractor_extract(azk_query_extractor* x, const void* dev_l
     AZK_CU(launch_query_extract(x->inst.as<PcsInstance>(), x->pairs.as<uint32_t>(), (uint32_t)count, x->out.as<uint8_t>(), x->s));
     g.stop();
     std::vector<uint8_t> roots(32ull * x->rounds);
-    read_back(x->s, {{roots.data(), x->roots.p, roots.size()}});
+    read_back(x->ctx, x->s, {{roots.data(), x->roots.p, roots.size()}});
     // each layer's root must be the committed one (extractOpening, :1161-1167)
     require(std::equal(roots.begin(), roots.end(), commitments), AZK_ERR_CORRECTNESS_VALIDATION_FAILED,
             "Resident Circle FRI query opening root did not match the committed layer root.");
-    read_back(x->s, {{queries_out, x->out.p, need}});
+    read_back(x->ctx, x->s, {{queries_out, x->out.p, need}});
     *out_len = need;
     fill_stats(st, t, 0, g.seconds());
   });
@@ -800,7 +800,7 @@ static void domain_read(azk_domain_plan* p, const DevBuf& b, bool present, void*
   require(present, AZK_ERR_INVALID_INPUT_LAYOUT, "the plan did not materialise this table");
   std::lock_guard<std::mutex> lk(p->mu);
   AZK_CU(cudaSetDevice(p->ctx->device));
-  read_back(p->s, {{out, b.p, bytes}});
+  read_back(p->ctx, p->s, {{out, b.p, bytes}});
 }
 
 azk_status azk_domain_plan_read_points(azk_domain_plan* p, uint32_t* xy_out) {
@@ -877,7 +877,7 @@ azk_status azk_circle_fold_plan_execute(azk_circle_fold_plan* p, const uint32_t*
     AZK_CU(cudaMemcpyAsync(f->ev.p, evaluations, kQ * n, cudaMemcpyHostToDevice, f->s));
     azk_stats inner{};
     forward(p->ctx, azk_qm31_fold_plan_execute_resident(f, f->ev.p, 0, p->dom->inv.p, 0, f->out.p, 0, challenge, &inner));
-    read_back(f->s, {{out, f->out.p, kQ * (n / 2)}});
+    read_back(f->ctx, f->s, {{out, f->out.p, kQ * (n / 2)}});
     fill_stats(st, t, 0, inner.gpu_s);
   });
 }
@@ -933,7 +933,7 @@ azk_status azk_circle_fold_chain_plan_execute(azk_circle_fold_chain_plan* p, con
     AZK_CU(cudaMemcpyAsync(c->ev.p, evaluations, kQ * c->n_in, cudaMemcpyHostToDevice, c->s));
     azk_stats inner{};
     forward(p->ctx, azk_fold_chain_plan_execute_resident(c, c->ev.p, 0, p->dom->inv.p, 0, c->out.p, 0, challenges, &inner));
-    read_back(c->s, {{final_out, c->out.p, kQ * c->n_out}});
+    read_back(c->ctx, c->s, {{final_out, c->out.p, kQ * c->n_out}});
     fill_stats(st, t, 0, inner.gpu_s);
   });
 }

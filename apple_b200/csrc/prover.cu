@@ -531,7 +531,7 @@ struct Engine {
       AZK_CU(cudaMemsetAsync(found.p, 0xFF, 8, s));
       AZK_CU(launch_pcs_grind(d_inst(), i, start, chunk, found.as<unsigned long long>(), s));
       uint64_t nonce = ~0ull;
-      read_back(s, {{&nonce, found.p, 8}});
+      read_back(ctx, s, {{&nonce, found.p, 8}});
       if (nonce != ~0ull) {
         h_inst[i].nonce = nonce;
         h_inst[i].has_nonce = 1;
@@ -612,7 +612,7 @@ struct Engine {
 
   void trace(uint32_t i, uint8_t* cm, uint32_t* ch, uint32_t* fl, uint32_t* qp) {
     const auto& c2 = cfg[i];
-    read_back(s, {{cm, arena.at<uint8_t>(off_cm[i]), 32ull * c2.rounds},
+    read_back(ctx, s, {{cm, arena.at<uint8_t>(off_cm[i]), 32ull * c2.rounds},
                   {ch, arena.at<uint8_t>(off_ch[i]), 16ull * c2.rounds},
                   {fl, h_inst[i].layers + layer_offset(c2.logn, c2.rounds), 16ull << (c2.logn - c2.rounds)},
                   {qp, arena.at<uint8_t>(off_qp[i]), 4ull * c2.queries}});
@@ -701,7 +701,7 @@ static void pcs_prove_common(azk_pcs_prover* p, bool coeffs, const uint8_t pub[3
     gs = e.finish_run();
   } else {
     const HostResult proof = {proof_out, e.h_inst[0].proof, len};
-    read_back(e.s, &proof, 1, [&] { gs = e.finish_run(); });
+    read_back(e.ctx, e.s, &proof, 1, [&] { gs = e.finish_run(); });
   }
   *proof_len = len;
   fill_stats(st, t, sub, gs);
@@ -953,7 +953,7 @@ azk_status azk_batch_download_proofs(azk_batch* b, uint8_t* out, uint64_t cap) {
       proofs.push_back({out + pos, e.h_inst[i].proof, e.proof_len[i]});
       pos += e.proof_len[i];
     }
-    read_back(e.s, proofs.data(), proofs.size(), [] {});
+    read_back(e.ctx, e.s, proofs.data(), proofs.size(), [] {});
   });
 }
 
@@ -967,7 +967,7 @@ azk_status azk_batch_download_each(azk_batch* b, void* const* outs, const uint64
     touch_pages(outs, e.proof_len);
     std::vector<HostResult> proofs;
     for (size_t i = 0; i < e.cfg.size(); i++) proofs.push_back({outs[i], e.h_inst[i].proof, e.proof_len[i]});
-    read_back(e.s, proofs.data(), proofs.size(), [] {});
+    read_back(e.ctx, e.s, proofs.data(), proofs.size(), [] {});
   });
 }
 

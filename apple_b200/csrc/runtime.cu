@@ -275,6 +275,7 @@ azk_status azk_ctx_create(int device, azk_ctx** out) {
     c->cc_major = prop.major;
     c->cc_minor = prop.minor;
     c->total_mem = prop.totalGlobalMem;
+    c->landings.reserve(azk_ctx::kLandingsKept);
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) {
       delete c;
       fail(AZK_ERR_COMMAND_EXECUTION_FAILED, "failed to create a CUDA stream");
@@ -291,6 +292,7 @@ void azk_ctx_destroy(azk_ctx* ctx) {
     cudaFree(kv.second.tw);
     cudaFree(kv.second.inv);
   }
+  ctx->landings.clear();
   if (ctx->sumcheck_dev) cudaFree(ctx->sumcheck_dev);
   if (ctx->sumcheck_pin) cudaFreeHost(ctx->sumcheck_pin);
   cudaStreamDestroy(ctx->stream);
@@ -474,7 +476,7 @@ azk_status azk_keccakf_plan_permute(azk_keccakf_plan* p, const void* host_states
     Timer t;
     AZK_CU(cudaMemcpyAsync(p->in.p, host_states, p->count * p->in_stride, cudaMemcpyHostToDevice, p->s));
     keccakf_run(p, p->in.as<uint8_t>(), p->out.as<uint8_t>(), nullptr, t);
-    read_back(p->s, {{host_out, p->out.p, p->count * p->out_stride}});
+    read_back(p->ctx, p->s, {{host_out, p->out.p, p->count * p->out_stride}});
     if (st) { st->cpu_wall_s = t.seconds(); st->gpu_s = 0; st->cpu_submit_ns = 0; }
   });
 }
@@ -536,7 +538,7 @@ azk_status azk_hash_plan_hash(azk_hash_plan* p, const void* msgs, void* digests,
     AZK_CU(launch_hash_batch(p->in.as<uint8_t>(), p->stride, (uint32_t)p->length, p->suffix, p->out.as<uint8_t>(), p->out_stride, p->count,
                              p->threads, p->s));
     uint64_t sub = t.ns();
-    read_back(p->s, {{digests, p->out.p, p->count * p->out_stride}});
+    read_back(p->ctx, p->s, {{digests, p->out.p, p->count * p->out_stride}});
     fill_stats(st, t, sub, 0);
   });
 }
@@ -629,7 +631,7 @@ static void merkle_commit_dev(azk_merkle_plan* p, const uint8_t* dleaves, uint8_
   AZK_CU(launch_tree_jobs(p->job.as<TreeJob>(), p->work.as<uint2>(), (uint32_t)p->h_work.size(), p->tile_log, kLeafRaw, p->threads, p->s));
   uint64_t sub = t.ns();
   g.stop();
-  read_back(p->s, {{root_out, p->root.p, 32}});
+  read_back(p->ctx, p->s, {{root_out, p->root.p, 32}});
   p->committed = true;
   fill_stats(st, t, sub, g.seconds());
 }
@@ -659,7 +661,7 @@ static void merkle_gather(azk_merkle_plan* p, const uint64_t* idx, uint64_t n, u
   p->paths.alloc(n * p->logn * 32, "Merkle.OpenPaths");
   AZK_CU(cudaMemcpyAsync(p->idx.p, idx, n * 8, cudaMemcpyHostToDevice, p->s));
   AZK_CU(launch_gather_openings(p->job.as<TreeJob>(), p->idx.as<uint64_t>(), (uint32_t)n, p->paths.as<uint64_t>(), p->s));
-  read_back(p->s, {{out, p->paths.p, n * p->logn * 32}});
+  read_back(p->ctx, p->s, {{out, p->paths.p, n * p->logn * 32}});
 }
 
 azk_status azk_merkle_plan_open(azk_merkle_plan* p, const void* leaves, uint64_t index, uint8_t* leaf_out, uint8_t* sib_out, uint8_t root[32],
@@ -745,7 +747,7 @@ azk_status azk_merkle_commit_prehashed(azk_ctx* ctx, const void* digests, uint64
     GpuTimer g(s);
     AZK_CU(launch_tree_jobs(jb.as<TreeJob>(), dw.as<uint2>(), (uint32_t)tiles, tl, kLeafDigest, 256, s));
     g.stop();
-    read_back(s, {{root, r.p, 32}});
+    read_back(ctx, s, {{root, r.p, 32}});
     fill_stats(st, t, 0, g.seconds());
   });
 }
@@ -795,7 +797,7 @@ static void prehashed_commit(azk_merkle_prehashed_plan* p, const uint8_t* leaves
   GpuTimer g(p->s);
   AZK_CU(launch_tree_jobs(p->job.as<TreeJob>(), p->work.as<uint2>(), (uint32_t)(1ull << (p->logn - p->tile_log)), p->tile_log, kLeafDigest, 256, p->s));
   g.stop();
-  read_back(p->s, {{root, p->root.p, 32}});
+  read_back(p->ctx, p->s, {{root, p->root.p, 32}});
   fill_stats(st, t, 0, g.seconds());
 }
 
@@ -834,7 +836,7 @@ azk_status azk_circle_domain_points(azk_ctx* ctx, uint32_t logn, uint32_t* xy) {
     uint64_t n = 1ull << logn;
     DevBuf d(8 * n, "CircleDomain.Points");
     AZK_CU(launch_domain_points(logn, d.as<uint32_t>(), ctx->stream));
-    read_back(ctx->stream, {{xy, d.p, 8 * n}});
+    read_back(ctx, ctx->stream, {{xy, d.p, 8 * n}});
   });
 }
 
@@ -906,7 +908,7 @@ azk_status azk_codeword_plan_execute(azk_codeword_plan* p, const uint32_t* coeff
     if (count) AZK_CU(cudaMemcpyAsync(p->coeff.p, coeffs, 16 * count, cudaMemcpyHostToDevice, p->s));
     if (count < n) AZK_CU(cudaMemsetAsync(p->coeff.as<uint4>() + count, 0, 16 * (n - count), p->s));
     codeword_run(p, p->coeff.as<uint4>(), p->out.as<uint4>(), nullptr, t);
-    read_back(p->s, {{codeword, p->out.p, 16 * n}});
+    read_back(p->ctx, p->s, {{codeword, p->out.p, 16 * n}});
     fill_stats(st, t, 0, 0);
   });
 }
@@ -938,7 +940,7 @@ azk_status azk_codeword_plan_execute_polynomial(azk_codeword_plan* p, const uint
     }
     witness_columns_to_device(p->wit, x, nx, y, ny, p->coeff.p);
     codeword_run(p, p->coeff.as<uint4>(), p->out.as<uint4>(), st, t);
-    read_back(p->s, {{codeword, p->out.p, 16ull << p->logn}});
+    read_back(p->ctx, p->s, {{codeword, p->out.p, 16ull << p->logn}});
   });
 }
 
@@ -1016,7 +1018,7 @@ static void witness_run(azk_witness_plan* p, const uint4* x, uint64_t nx, const 
   if (nx) AZK_CU(launch_scan_input(x, nx, bad, info, p->s));
   if (ny) AZK_CU(launch_scan_input(y, ny, bad, info, p->s));
   uint32_t found[8];
-  read_back(p->s, {{found, bad, sizeof(found)}});
+  read_back(p->ctx, p->s, {{found, bad, sizeof(found)}});
   layout(found[0] == 0, "witness coefficients contain a non-canonical field element");
   const bool lifted = found[4] != 0;
 
@@ -1121,7 +1123,7 @@ azk_status azk_witness_plan_execute(azk_witness_plan* p, const uint32_t* x, uint
     if (nx) AZK_CU(cudaMemcpyAsync(p->host_x(), x, 16 * nx, cudaMemcpyHostToDevice, p->s));
     if (ny) AZK_CU(cudaMemcpyAsync(p->host_y(), y, 16 * ny, cudaMemcpyHostToDevice, p->s));
     witness_run(p, p->host_x(), nx, p->host_y(), ny, p->host_out(), st, t);
-    read_back(p->s, {{out, p->host_out(), 32 * p->n}});
+    read_back(p->ctx, p->s, {{out, p->host_out(), 32 * p->n}});
   });
 }
 
@@ -1172,7 +1174,7 @@ azk_status azk_qm31_fold(azk_ctx* ctx, const uint32_t* ev, uint64_t n, const uin
     GpuTimer g(s);
     AZK_CU(launch_fold_qm31_inv(de.as<uint4>(), di.as<uint4>(), dc.as<uint32_t>(), dout.as<uint4>(), n / 2, s));
     g.stop();
-    read_back(s, {{out, dout.p, 8 * n}});
+    read_back(ctx, s, {{out, dout.p, 8 * n}});
     fill_stats(st, t, 0, g.seconds());
   });
 }
@@ -1211,7 +1213,7 @@ azk_status azk_circle_fold_chain(azk_ctx* ctx, uint32_t logn, const uint32_t* ev
     for (uint32_t r = 0; r < rounds; r++)
       AZK_CU(launch_fold_jobs(djobs.as<FoldJob>(), dwork.as<uint2>() + ranges[r].first, (uint32_t)ranges[r].second, s));
     g.stop();
-    read_back(s, {{out, layers.as<uint4>() + layer_offset(logn, rounds), 16 * (n >> rounds)}});
+    read_back(ctx, s, {{out, layers.as<uint4>() + layer_offset(logn, rounds), 16 * (n >> rounds)}});
     fill_stats(st, t, 0, g.seconds());
   });
 }
@@ -1276,7 +1278,7 @@ azk_status azk_qm31_merkle_fold_chain(azk_ctx* ctx, const uint32_t* ev, uint64_t
       inv_off += m;
     }
     g.stop();
-    read_back(s, {{final_out, layers.as<uint4>() + layer_offset(logn, rounds), 16 * (n >> rounds)},
+    read_back(ctx, s, {{final_out, layers.as<uint4>() + layer_offset(logn, rounds), 16 * (n >> rounds)},
                   {commitments_out, dcm.p, 32ull * rounds},
                   {ch_out, dch.p, 16ull * rounds}});
     fill_stats(st, t, 0, g.seconds());
@@ -1298,7 +1300,7 @@ azk_status azk_qm31_transcript_challenges(azk_ctx* ctx, uint64_t input_count, co
     AZK_CU(cudaMemcpyAsync(roots.p, commitments, 32ull * rounds, cudaMemcpyHostToDevice, s));
     AZK_CU(launch_qm31_transcript_prefix(tr.as<Transcript>(), input_count, rounds, s));
     AZK_CU(launch_transcript_rounds_given(tr.as<Transcript>(), kRootQM31Round, roots.as<uint64_t>(), rounds, input_count, dch.as<uint32_t>(), s));
-    read_back(s, {{ch_out, dch.p, 16ull * rounds}});
+    read_back(ctx, s, {{ch_out, dch.p, 16ull * rounds}});
   });
 }
 
@@ -1331,7 +1333,7 @@ azk_status azk_check_canonical(azk_ctx* ctx, const void* dwords, uint64_t nwords
     DevBuf f(4, "Canonical.Flag");
     AZK_CU(cudaMemsetAsync(f.p, 0, 4, s));
     AZK_CU(launch_check_canonical(static_cast<const uint32_t*>(dwords), nwords, f.as<uint32_t>(), s));
-    read_back(s, {{flag_out, f.p, 4}});
+    read_back(ctx, s, {{flag_out, f.p, 4}});
   });
 }
 
