@@ -11,7 +11,9 @@
 
 #include <atomic>
 #include <chrono>
+#include <condition_variable>
 #include <cstdint>
+#include <mutex>
 #include <thread>
 
 namespace azk {
@@ -64,5 +66,28 @@ void poll_until(Done done, Sleep sleep, bool shared_host, SpinPlaces& places) {
     }
   }
 }
+
+// One thread at a time, in the order they came (a std::mutex lets a thread that returns
+// at once pass those that wait).
+struct Turns {
+  struct Turn {
+    Turns& of;
+    explicit Turn(Turns& t) : of(t) {
+      std::unique_lock<std::mutex> lk(of.mu);
+      const uint64_t mine = of.next++;
+      of.moved.wait(lk, [&] { return of.now == mine; });
+    }
+    ~Turn() {
+      std::lock_guard<std::mutex> lk(of.mu);
+      of.now++;
+      if (of.now != of.next) of.moved.notify_all();
+    }
+    Turn(const Turn&) = delete;
+    Turn& operator=(const Turn&) = delete;
+  };
+  std::mutex mu;
+  std::condition_variable moved;
+  uint64_t next = 0, now = 0;
+};
 
 }  // namespace azk

@@ -95,8 +95,8 @@ azk_status azk_qm31_fold_plan_execute(azk_qm31_fold_plan* p, const uint32_t* eva
     std::lock_guard<std::mutex> lk(p->mu);
     AZK_CU(cudaSetDevice(p->ctx->device));
     Timer t;
-    AZK_CU(cudaMemcpyAsync(p->ev.p, evaluations, kQ * p->n_in, cudaMemcpyHostToDevice, p->s));
-    AZK_CU(cudaMemcpyAsync(p->inv.p, inverse_points, kQ * p->n_out, cudaMemcpyHostToDevice, p->s));
+    upload(p->ctx, p->s, p->ev.p, evaluations, kQ * p->n_in);
+    upload(p->ctx, p->s, p->inv.p, inverse_points, kQ * p->n_out);
     double gs = qm31_fold_run(p, p->ev.as<uint4>(), p->inv.as<uint4>(), p->out.as<uint4>(), challenge);
     read_back(p->ctx, p->s, {{out, p->out.p, kQ * p->n_out}});
     fill_stats(st, t, 0, gs);
@@ -357,8 +357,8 @@ azk_status azk_fold_chain_plan_execute(azk_fold_chain_plan* p, const uint32_t* e
     std::lock_guard<std::mutex> lk(p->mu);
     AZK_CU(cudaSetDevice(p->ctx->device));
     Timer t;
-    AZK_CU(cudaMemcpyAsync(p->ev.p, evaluations, kQ * p->n_in, cudaMemcpyHostToDevice, p->s));
-    AZK_CU(cudaMemcpyAsync(p->inv.p, inverse_layers, kQ * p->inv_total, cudaMemcpyHostToDevice, p->s));
+    upload(p->ctx, p->s, p->ev.p, evaluations, kQ * p->n_in);
+    upload(p->ctx, p->s, p->inv.p, inverse_layers, kQ * p->inv_total);
     AZK_CU(cudaMemcpyAsync(p->ch.p, challenges, 16ull * p->rounds, cudaMemcpyHostToDevice, p->s));
     GpuTimer g(p->s);
     chain_fold_all(p, p->ev.as<uint4>(), p->inv.as<uint4>(), p->out.as<uint4>());
@@ -397,8 +397,8 @@ azk_status azk_fold_chain_plan_execute_transcript(azk_fold_chain_plan* p, const 
     std::lock_guard<std::mutex> lk(p->mu);
     AZK_CU(cudaSetDevice(p->ctx->device));
     Timer t;
-    AZK_CU(cudaMemcpyAsync(p->ev.p, evaluations, kQ * p->n_in, cudaMemcpyHostToDevice, p->s));
-    AZK_CU(cudaMemcpyAsync(p->inv.p, inverse_layers, kQ * p->inv_total, cudaMemcpyHostToDevice, p->s));
+    upload(p->ctx, p->s, p->ev.p, evaluations, kQ * p->n_in);
+    upload(p->ctx, p->s, p->inv.p, inverse_layers, kQ * p->inv_total);
     AZK_CU(cudaMemcpyAsync(p->cm.p, commitments, 32ull * p->rounds, cudaMemcpyHostToDevice, p->s));
     GpuTimer g(p->s);
     AZK_CU(launch_qm31_transcript_prefix(p->tr.as<Transcript>(), p->n_in, p->rounds, p->s));
@@ -446,8 +446,8 @@ azk_status azk_fold_chain_plan_execute_merkle(azk_fold_chain_plan* p, const uint
     std::lock_guard<std::mutex> lk(p->mu);
     AZK_CU(cudaSetDevice(p->ctx->device));
     Timer t;
-    AZK_CU(cudaMemcpyAsync(p->ev.p, evaluations, kQ * p->n_in, cudaMemcpyHostToDevice, p->s));
-    AZK_CU(cudaMemcpyAsync(p->inv.p, inverse_layers, kQ * p->inv_total, cudaMemcpyHostToDevice, p->s));
+    upload(p->ctx, p->s, p->ev.p, evaluations, kQ * p->n_in);
+    upload(p->ctx, p->s, p->inv.p, inverse_layers, kQ * p->inv_total);
     GpuTimer g(p->s);
     chain_merkle(p, p->ev.as<uint4>(), p->inv.as<uint4>(), p->layers.as<uint4>(), false, p->out.as<uint4>(), nullptr);
     g.stop();
@@ -874,7 +874,7 @@ azk_status azk_circle_fold_plan_execute(azk_circle_fold_plan* p, const uint32_t*
     azk_qm31_fold_plan* f = p->fold;
     AZK_CU(cudaSetDevice(p->ctx->device));
     Timer t;
-    AZK_CU(cudaMemcpyAsync(f->ev.p, evaluations, kQ * n, cudaMemcpyHostToDevice, f->s));
+    upload(f->ctx, f->s, f->ev.p, evaluations, kQ * n);
     azk_stats inner{};
     forward(p->ctx, azk_qm31_fold_plan_execute_resident(f, f->ev.p, 0, p->dom->inv.p, 0, f->out.p, 0, challenge, &inner));
     read_back(f->ctx, f->s, {{out, f->out.p, kQ * (n / 2)}});
@@ -930,7 +930,7 @@ azk_status azk_circle_fold_chain_plan_execute(azk_circle_fold_chain_plan* p, con
     std::lock_guard<std::mutex> lk(p->mu);
     AZK_CU(cudaSetDevice(p->ctx->device));
     Timer t;
-    AZK_CU(cudaMemcpyAsync(c->ev.p, evaluations, kQ * c->n_in, cudaMemcpyHostToDevice, c->s));
+    upload(c->ctx, c->s, c->ev.p, evaluations, kQ * c->n_in);
     azk_stats inner{};
     forward(p->ctx, azk_fold_chain_plan_execute_resident(c, c->ev.p, 0, p->dom->inv.p, 0, c->out.p, 0, challenges, &inner));
     read_back(c->ctx, c->s, {{final_out, c->out.p, kQ * c->n_out}});
@@ -1020,7 +1020,7 @@ azk_status azk_circle_merkle_chain_plan_execute(azk_circle_merkle_chain_plan* p,
     std::lock_guard<std::mutex> lk(p->mu);
     AZK_CU(cudaSetDevice(p->ctx->device));
     Timer t;
-    AZK_CU(cudaMemcpyAsync(c->ev.p, evaluations, kQ * c->n_in, cudaMemcpyHostToDevice, c->s));
+    upload(c->ctx, c->s, c->ev.p, evaluations, kQ * c->n_in);
     azk_stats inner{};
     forward(p->ctx, azk_fold_chain_plan_execute_merkle_readback(c, c->ev.p, 0, p->dom->inv.p, 0, final_out, commitments_out, challenges_out, &inner));
     fill_stats(st, t, 0, inner.gpu_s);

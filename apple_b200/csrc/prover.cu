@@ -720,7 +720,7 @@ azk_status azk_pcs_prover_prove_evaluations(azk_pcs_prover* p, const uint32_t* e
     pcs_ensure_claimed(p, cl);
     Engine& e = p->eng;
     // evaluations go straight into layer 0
-    AZK_CU(cudaMemcpyAsync(e.h_inst[0].layers, ev, 16 * N, cudaMemcpyHostToDevice, e.s));
+    upload(e.ctx, e.s, e.h_inst[0].layers, ev, 16 * N);
     e.check_input_canonical(e.h_inst[0].layers, 4 * N);
     pcs_prove_common(p, false, pub, proof_out, false, proof_len, st, t);
   });
@@ -737,7 +737,7 @@ azk_status azk_pcs_prover_prove_coefficients(azk_pcs_prover* p, const uint32_t* 
     pcs_ensure_claimed(p, {});
     Engine& e = p->eng;
     uint4* in = e.arena.at<uint4>(e.off_input[0]);
-    AZK_CU(cudaMemcpyAsync(in, coeffs, 16 * count, cudaMemcpyHostToDevice, e.s_up));
+    upload(e.ctx, e.s_up, in, coeffs, 16 * count);
     e.scan_inputs({count});
     pcs_prove_common(p, true, pub, proof_out, false, proof_len, st, t);
   });
@@ -805,8 +805,8 @@ azk_status azk_pcs_prover_prove_polynomial(azk_pcs_prover* p, const uint32_t* x,
       p->wy.alloc(16 * std::max<uint64_t>(half, 1), "CirclePCSProver.WitnessY");
     }
     Engine& e = p->eng;
-    if (nx) AZK_CU(cudaMemcpyAsync(p->wx.p, x, 16 * nx, cudaMemcpyHostToDevice, e.s));
-    if (ny) AZK_CU(cudaMemcpyAsync(p->wy.p, y, 16 * ny, cudaMemcpyHostToDevice, e.s));
+    if (nx) upload(e.ctx, e.s, p->wx.p, x, 16 * nx);
+    if (ny) upload(e.ctx, e.s, p->wy.p, y, 16 * ny);
     sync_stream(e.s);
     pcs_witness_input(p, p->wx.p, 0, nx, p->wy.p, 0, ny);
     pcs_prove_common(p, true, pub, proof_out, false, proof_len, st, t);
@@ -849,7 +849,7 @@ azk_status azk_circle_merkle_fold_chain(azk_ctx* ctx, uint32_t logn, const uint3
     Sched sc = resolve_schedule(nullptr, kTuned_pcs_single, kTunedThreads_pcs_single);
     sc.graph = false;
     e.init(ctx, {InstanceCfg{logn, rounds, queries, log_blowup, grinding, {}}}, sc);
-    AZK_CU(cudaMemcpyAsync(e.h_inst[0].layers, ev, 16 * N, cudaMemcpyHostToDevice, e.s));
+    upload(e.ctx, e.s, e.h_inst[0].layers, ev, 16 * N);
     e.check_input_canonical(e.h_inst[0].layers, 4 * N);
     e.set_publics(pub);
     GpuTimer g(e.s);
@@ -907,7 +907,7 @@ azk_status azk_batch_upload(azk_batch* b, const uint32_t* host, const uint64_t* 
       uint64_t N = 1ull << e.cfg[i].logn;
       layout(counts[i] >= 1 && counts[i] <= N);
       uint4* in = e.arena.at<uint4>(e.off_input[i]);
-      AZK_CU(cudaMemcpyAsync(in, host + 4 * offsets[i], 16 * counts[i], cudaMemcpyHostToDevice, e.s_up));
+      upload(e.ctx, e.s_up, in, host + 4 * offsets[i], 16 * counts[i]);
     }
     // every staged word must be canonical (QM31CanonicalityCheck.swift:11-117)
     e.scan_inputs(std::vector<uint64_t>(counts, counts + e.cfg.size()));

@@ -474,7 +474,7 @@ azk_status azk_keccakf_plan_permute(azk_keccakf_plan* p, const void* host_states
     layout(p && host_states && host_out);
     std::lock_guard<std::mutex> lk(p->mu);
     Timer t;
-    AZK_CU(cudaMemcpyAsync(p->in.p, host_states, p->count * p->in_stride, cudaMemcpyHostToDevice, p->s));
+    upload(p->ctx, p->s, p->in.p, host_states, p->count * p->in_stride);
     keccakf_run(p, p->in.as<uint8_t>(), p->out.as<uint8_t>(), nullptr, t);
     read_back(p->ctx, p->s, {{host_out, p->out.p, p->count * p->out_stride}});
     if (st) { st->cpu_wall_s = t.seconds(); st->gpu_s = 0; st->cpu_submit_ns = 0; }
@@ -534,7 +534,7 @@ azk_status azk_hash_plan_hash(azk_hash_plan* p, const void* msgs, void* digests,
     layout(p && digests && (msgs || p->count * p->stride == 0));
     std::lock_guard<std::mutex> lk(p->mu);
     Timer t;
-    if (p->count * p->stride) AZK_CU(cudaMemcpyAsync(p->in.p, msgs, p->count * p->stride, cudaMemcpyHostToDevice, p->s));
+    if (p->count * p->stride) upload(p->ctx, p->s, p->in.p, msgs, p->count * p->stride);
     AZK_CU(launch_hash_batch(p->in.as<uint8_t>(), p->stride, (uint32_t)p->length, p->suffix, p->out.as<uint8_t>(), p->out_stride, p->count,
                              p->threads, p->s));
     uint64_t sub = t.ns();
@@ -641,7 +641,7 @@ azk_status azk_merkle_plan_commit(azk_merkle_plan* p, const void* leaves, uint8_
     layout(p && root && (leaves || p->count * p->stride == 0));
     std::lock_guard<std::mutex> lk(p->mu);
     Timer t;
-    if (p->count * p->stride) AZK_CU(cudaMemcpyAsync(p->leaves.p, leaves, p->count * p->stride, cudaMemcpyHostToDevice, p->s));
+    if (p->count * p->stride) upload(p->ctx, p->s, p->leaves.p, leaves, p->count * p->stride);
     merkle_commit_dev(p, p->leaves.as<uint8_t>(), root, st, t);
   });
 }
@@ -671,7 +671,7 @@ azk_status azk_merkle_plan_open(azk_merkle_plan* p, const void* leaves, uint64_t
     layout(index < p->count);
     std::lock_guard<std::mutex> lk(p->mu);
     Timer t;
-    if (p->count * p->stride) AZK_CU(cudaMemcpyAsync(p->leaves.p, leaves, p->count * p->stride, cudaMemcpyHostToDevice, p->s));
+    if (p->count * p->stride) upload(p->ctx, p->s, p->leaves.p, leaves, p->count * p->stride);
     merkle_commit_dev(p, p->leaves.as<uint8_t>(), root, nullptr, t);
     merkle_gather(p, &index, 1, sib_out);
     if (leaf_out && p->length) std::memcpy(leaf_out, static_cast<const uint8_t*>(leaves) + index * p->stride, p->length);
@@ -740,7 +740,7 @@ azk_status azk_merkle_commit_prehashed(azk_ctx* ctx, const void* digests, uint64
     j.inner = inner.as<uint64_t>();
     j.counters = cnt.as<uint32_t>();
     j.root_out = r.as<uint64_t>();
-    AZK_CU(cudaMemcpyAsync(d.p, digests, bytes, cudaMemcpyHostToDevice, s));
+    upload(ctx, s, d.p, digests, bytes);
     AZK_CU(cudaMemsetAsync(cnt.p, 0, cnt.bytes, s));
     AZK_CU(cudaMemcpyAsync(dw.p, w.data(), tiles * sizeof(uint2), cudaMemcpyHostToDevice, s));
     AZK_CU(cudaMemcpyAsync(jb.p, &j, sizeof(TreeJob), cudaMemcpyHostToDevice, s));
@@ -807,7 +807,7 @@ azk_status azk_merkle_prehashed_plan_commit(azk_merkle_prehashed_plan* p, const 
     std::lock_guard<std::mutex> lk(p->mu);
     AZK_CU(cudaSetDevice(p->ctx->device));
     Timer t;
-    AZK_CU(cudaMemcpyAsync(p->staging.p, host_digests, 32 * p->count, cudaMemcpyHostToDevice, p->s));
+    upload(p->ctx, p->s, p->staging.p, host_digests, 32 * p->count);
     prehashed_commit(p, p->staging.as<uint8_t>(), root_out, st, t);
   });
 }
@@ -905,7 +905,7 @@ azk_status azk_codeword_plan_execute(azk_codeword_plan* p, const uint32_t* coeff
     layout(all_canonical(coeffs, 4 * count));
     std::lock_guard<std::mutex> lk(p->mu);
     Timer t;
-    if (count) AZK_CU(cudaMemcpyAsync(p->coeff.p, coeffs, 16 * count, cudaMemcpyHostToDevice, p->s));
+    if (count) upload(p->ctx, p->s, p->coeff.p, coeffs, 16 * count);
     if (count < n) AZK_CU(cudaMemsetAsync(p->coeff.as<uint4>() + count, 0, 16 * (n - count), p->s));
     codeword_run(p, p->coeff.as<uint4>(), p->out.as<uint4>(), nullptr, t);
     read_back(p->ctx, p->s, {{codeword, p->out.p, 16 * n}});
@@ -1062,8 +1062,8 @@ static void witness_run(azk_witness_plan* p, const uint4* x, uint64_t nx, const 
 static void witness_columns_to_device(azk_witness_plan* w, const uint32_t* x, uint64_t nx, const uint32_t* y, uint64_t ny, void* dout) {
   std::lock_guard<std::mutex> lk(w->mu);
   Timer t;
-  if (nx) AZK_CU(cudaMemcpyAsync(w->host_x(), x, 16 * nx, cudaMemcpyHostToDevice, w->s));
-  if (ny) AZK_CU(cudaMemcpyAsync(w->host_y(), y, 16 * ny, cudaMemcpyHostToDevice, w->s));
+  if (nx) upload(w->ctx, w->s, w->host_x(), x, 16 * nx);
+  if (ny) upload(w->ctx, w->s, w->host_y(), y, 16 * ny);
   witness_run(w, w->host_x(), nx, w->host_y(), ny, static_cast<uint4*>(dout), nullptr, t);
   sync_stream(w->s);
 }
@@ -1120,8 +1120,8 @@ azk_status azk_witness_plan_execute(azk_witness_plan* p, const uint32_t* x, uint
     layout(nx <= p->n && ny <= p->n && nx + ny > 0);
     std::lock_guard<std::mutex> lk(p->mu);
     Timer t;
-    if (nx) AZK_CU(cudaMemcpyAsync(p->host_x(), x, 16 * nx, cudaMemcpyHostToDevice, p->s));
-    if (ny) AZK_CU(cudaMemcpyAsync(p->host_y(), y, 16 * ny, cudaMemcpyHostToDevice, p->s));
+    if (nx) upload(p->ctx, p->s, p->host_x(), x, 16 * nx);
+    if (ny) upload(p->ctx, p->s, p->host_y(), y, 16 * ny);
     witness_run(p, p->host_x(), nx, p->host_y(), ny, p->host_out(), st, t);
     read_back(p->ctx, p->s, {{out, p->host_out(), 32 * p->n}});
   });
@@ -1168,8 +1168,8 @@ azk_status azk_qm31_fold(azk_ctx* ctx, const uint32_t* ev, uint64_t n, const uin
     Timer t;
     cudaStream_t s = ctx->stream;
     DevBuf de(16 * n, "QM31Fold.Input"), di(8 * n, "QM31Fold.Inverse"), dc(16, "QM31Fold.Challenge"), dout(8 * n, "QM31Fold.Output");
-    AZK_CU(cudaMemcpyAsync(de.p, ev, 16 * n, cudaMemcpyHostToDevice, s));
-    AZK_CU(cudaMemcpyAsync(di.p, inv, 8 * n, cudaMemcpyHostToDevice, s));
+    upload(ctx, s, de.p, ev, 16 * n);
+    upload(ctx, s, di.p, inv, 8 * n);
     AZK_CU(cudaMemcpyAsync(dc.p, ch, 16, cudaMemcpyHostToDevice, s));
     GpuTimer g(s);
     AZK_CU(launch_fold_qm31_inv(de.as<uint4>(), di.as<uint4>(), dc.as<uint32_t>(), dout.as<uint4>(), n / 2, s));
@@ -1190,7 +1190,7 @@ azk_status azk_circle_fold_chain(azk_ctx* ctx, uint32_t logn, const uint32_t* ev
     Timer t;
     cudaStream_t s = ctx->stream;
     DevBuf layers(16 * 2 * n, "CircleFold.Layers"), dch(16ull * rounds, "CircleFold.Challenges");
-    AZK_CU(cudaMemcpyAsync(layers.p, ev, 16 * n, cudaMemcpyHostToDevice, s));
+    upload(ctx, s, layers.p, ev, 16 * n);
     AZK_CU(cudaMemcpyAsync(dch.p, ch, 16ull * rounds, cudaMemcpyHostToDevice, s));
     std::vector<FoldJob> jobs;
     std::vector<uint2> work;
@@ -1235,8 +1235,8 @@ azk_status azk_qm31_merkle_fold_chain(azk_ctx* ctx, const uint32_t* ev, uint64_t
     DevBuf layers(16 * 2 * n, "QM31Chain.Layers"), dinv(16 * inv_total + 16, "QM31Chain.Inverse"), dch(16ull * rounds, "QM31Chain.Challenges"),
         dcm(32ull * rounds, "QM31Chain.Commitments"), tr(sizeof(Transcript), "QM31Chain.Transcript"), inner(32 * n, "QM31Chain.Inner"),
         cnt(tree_counter_count(logn, 10) * 4, "QM31Chain.Counters"), jobs(sizeof(TreeJob) * rounds, "QM31Chain.Jobs");
-    AZK_CU(cudaMemcpyAsync(layers.p, ev, 16 * n, cudaMemcpyHostToDevice, s));
-    AZK_CU(cudaMemcpyAsync(dinv.p, inv, 16 * inv_total, cudaMemcpyHostToDevice, s));
+    upload(ctx, s, layers.p, ev, 16 * n);
+    upload(ctx, s, dinv.p, inv, 16 * inv_total);
     AZK_CU(cudaMemsetAsync(cnt.p, 0, cnt.bytes, s));
     std::vector<TreeJob> hj(rounds);
     std::vector<uint2> work;

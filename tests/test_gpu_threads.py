@@ -55,7 +55,7 @@ def _large_codeword(ctx, seed):
     return lambda: p.execute_coefficients(x)[::64].tobytes()
 
 
-@pytest.mark.parametrize("make", [_prove, _prove_evaluations, _hash, _commit, _codeword])
+@pytest.mark.parametrize("make", [_prove, _prove_evaluations, _hash, _commit, _codeword, _large_codeword])
 def test_every_thread_gets_its_calls_through(ctx, make):
     calls = [make(ctx, seed) for seed in range(THREADS)]
     want = [hashlib.sha256(call()).digest() for call in calls]

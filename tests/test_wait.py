@@ -1,5 +1,5 @@
 """The library's waits, compiled for the host: how many threads may spin, and when the
-others sleep."""
+others sleep; and the turns of large uploads."""
 import os
 import subprocess
 

@@ -1,4 +1,4 @@
-// Host-compiled check of the polling waits (azk_wait.h): no more threads spin at a
+// Host-compiled check of the waits and turns (azk_wait.h): no more threads spin at a
 // time than there are places, the others sleep between polls soon after they begin to
 // wait, places are given back, also when a poll throws.  Built and run by
 // tests/test_wait.py.
@@ -77,6 +77,28 @@ int main() {
     go = true;
     for (auto& t : pool) t.join();
     CHECK(places.taken == 0, "places add up");
+  }
+  // turns are taken in the order of arrival, also against a thread that comes back at once
+  {
+    Turns turns;
+    std::vector<int> order;
+    std::vector<std::thread> pool;
+    {
+      Turns::Turn held(turns);
+      for (int i = 0; i < 6; i++) {
+        pool.emplace_back([&, i] {
+          Turns::Turn t(turns);
+          order.push_back(i);
+        });
+        for (;;) {  // the thread has its place in the line
+          std::lock_guard<std::mutex> lk(turns.mu);
+          if (turns.next == (uint64_t)i + 2) break;
+        }
+      }
+    }
+    { Turns::Turn back(turns); order.push_back(6); }
+    for (auto& t : pool) t.join();
+    CHECK((order == std::vector<int>{0, 1, 2, 3, 4, 5, 6}), "turns in the order of arrival");
   }
   CHECK(SpinPlaces::usable_cores() >= 1 && SpinPlaces::process().most == SpinPlaces::usable_cores() / 2, "half of the host's cores");
   std::printf("waits ok\n");
