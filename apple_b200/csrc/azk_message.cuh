@@ -25,6 +25,14 @@ struct ReadOnlyLoads {
   }
 };
 
+// Loads of a message in global or shared memory.
+struct AnyLoads {
+  template <class T>
+  __host__ __device__ __forceinline__ static T load(const uint8_t* p) {
+    return *reinterpret_cast<const T*>(p);
+  }
+};
+
 // Bytes [from, to) of the 4-byte unit at q (4-byte aligned), in their places, zeros
 // around them; no other byte is read.
 template <class L>
@@ -50,13 +58,9 @@ __host__ __device__ __forceinline__ uint64_t aligned_tail(const uint8_t* p, uint
 }
 
 // 64-bit words of a message at any byte address, from aligned 4-byte loads and
-// shifts.  A batch's first and last messages (`edge`) take the units that are not all
-// message by bytes and halves, so nothing before or behind the batch is read; a unit
-// at either end of the others also holds bytes of the gap or the message next to
-// them, which are masked off.  Byte loads throughout were four times as many requests
-// (2^20 messages of 99 bytes at stride 102, 256 threads per CTA: 354 us); 128 threads,
-// host call included: 283 us without an edge, 287 with edge loads for every message,
-// 279 so.
+// shifts.  EDGE: units that are not all message are taken by bytes and halves, so no byte
+// outside the message is read (raw leaves: a select more per word).  Otherwise they are
+// taken whole and masked; hash_batch keeps such units inside its buffers.
 template <bool EDGE, class L = ReadOnlyLoads>
 struct UnalignedWords {
   const uint8_t* q;     // the unit that holds the first byte
@@ -94,32 +98,23 @@ struct UnalignedWords {
   }
 };
 
-// f(reader) with the reader of a message that is not 8-byte aligned: `edge`, the first
-// or the last of its batch.
-template <class L = ReadOnlyLoads, class F>
-__host__ __device__ __forceinline__ void with_unaligned(const uint8_t* p, uint32_t len, bool edge, F f) {
-  if (edge) f(UnalignedWords<true, L>(p, len));
-  else f(UnalignedWords<false, L>(p, len));
-}
-
 // XOR `len` message bytes into lanes 0..16.  aligned8: p is 8-byte aligned, so
-// whole lanes load as u64.  edge: the first or the last message of its batch.
-template <class L = ReadOnlyLoads>
-__host__ __device__ __forceinline__ void xor_message(uint64_t (&a)[25], const uint8_t* p, uint32_t len, bool aligned8, bool edge) {
+// whole lanes load as u64.  EDGE, L: see UnalignedWords; LA: the loads of aligned ones.
+template <bool EDGE, class L = ReadOnlyLoads, class LA = L>
+__host__ __device__ __forceinline__ void xor_message(uint64_t (&a)[25], const uint8_t* p, uint32_t len, bool aligned8) {
   const uint32_t full = len >> 3, rem = len & 7;
   uint64_t v = 0;
   if (aligned8) {
 #pragma unroll
     for (uint32_t i = 0; i < 17; i++)
-      if (i < full) a[i] ^= L::template load<uint64_t>(p + 8 * i);
-    if (rem) v = aligned_tail<L>(p + 8 * full, rem);
+      if (i < full) a[i] ^= LA::template load<uint64_t>(p + 8 * i);
+    if (rem) v = aligned_tail<LA>(p + 8 * full, rem);
   } else {
-    with_unaligned<L>(p, len, edge, [&](const auto& u) {
+    const UnalignedWords<EDGE, L> u(p, len);
 #pragma unroll
-      for (uint32_t i = 0; i < 17; i++)
-        if (i < full) a[i] ^= u.word(i, 8);
-      if (rem) v = u.word(full, rem);
-    });
+    for (uint32_t i = 0; i < 17; i++)
+      if (i < full) a[i] ^= u.word(i, 8);
+    if (rem) v = u.word(full, rem);
   }
   if (rem) {
     // lane index `full` is dynamic here; select it with an unrolled compare
@@ -131,11 +126,12 @@ __host__ __device__ __forceinline__ void xor_message(uint64_t (&a)[25], const ui
 
 #if defined(__CUDACC__)
 // Digest of one message of `len` (<= 136) bytes at p.
-__device__ __forceinline__ void hash_message(const uint8_t* p, uint32_t len, uint32_t suffix, bool aligned8, bool edge, uint64_t (&out)[4]) {
+template <bool EDGE, class L = ReadOnlyLoads, class LA = L>
+__device__ __forceinline__ void hash_message(const uint8_t* p, uint32_t len, uint32_t suffix, bool aligned8, uint64_t (&out)[4]) {
   uint64_t a[25];
 #pragma unroll
   for (int i = 0; i < 25; i++) a[i] = 0;
-  xor_message(a, p, len, aligned8, edge);
+  xor_message<EDGE, L, LA>(a, p, len, aligned8);
   if (len == 136) {
     keccak_f1600(a);
     a[0] ^= suffix;

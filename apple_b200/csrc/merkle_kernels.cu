@@ -38,9 +38,6 @@ __device__ __forceinline__ void ld_dig_cg(const uint64_t* p, uint64_t (&d)[4]) {
 // warp's lanes.
 __device__ __forceinline__ uint32_t warp_index() { return __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0); }
 
-// The first or the last leaf: nothing outside its bytes is read.
-__device__ __forceinline__ bool edge_leaf(const TreeJob& job, uint64_t leaf) { return leaf == 0 || leaf + 1 == 1ull << job.logn; }
-
 template <uint32_t KIND>
 __device__ __forceinline__ void leaf_digest(const TreeJob& job, uint64_t leaf, const uint32_t (&ch)[4], uint64_t (&d)[4]) {
   if constexpr (KIND == kLeafQM31) {
@@ -49,7 +46,7 @@ __device__ __forceinline__ void leaf_digest(const TreeJob& job, uint64_t leaf, c
   } else if constexpr (KIND == kLeafDigest) {
     ld_dig(reinterpret_cast<const uint64_t*>(job.raw) + 4 * leaf, d);
   } else {
-    hash_message(job.raw + leaf * job.stride, job.len, job.suffix, job.aligned8 != 0, edge_leaf(job, leaf), d);
+    hash_message<true>(job.raw + leaf * job.stride, job.len, job.suffix, job.aligned8 != 0, d);
   }
 }
 
@@ -90,8 +87,8 @@ __device__ __forceinline__ void raw_setup(const TreeJob& job, uint64_t leaf, uin
     for (uint32_t i = 0; i < LANES; i++)
       if (i < full) a[i] = __ldg(reinterpret_cast<const uint64_t*>(p) + i);
   } else {
-    // the edge reader for every leaf: both readers in this loop's code cost unaligned
-    // trees 3 % (2^20 leaves of 99 bytes: 606 us, 618 with both, 598 without an edge)
+    // 2^20 leaves of 99 bytes: 606 us, 598 with whole units; 618 with both readers in this
+    // loop's code, one for the first and last leaf
     const UnalignedWords<true> u(p, job.len);
     if (rem) tail |= u.word(full, rem);
 #pragma unroll
@@ -377,7 +374,6 @@ __device__ __forceinline__ uint4 pair_leaf(const TreeJob& job, uint64_t leaf, bo
       if (job.aligned8) {
         words([&](uint32_t i, uint32_t n) { return n == 8 ? __ldg(reinterpret_cast<const uint64_t*>(p) + i) : aligned_tail(p + 8 * i, n); });
       } else {
-        // the exchange between lanes needs the whole warp: one reader for all its leaves
         const UnalignedWords<true> u(p, job.len);
         words([&](uint32_t i, uint32_t n) { return u.word(i, n); });
       }
