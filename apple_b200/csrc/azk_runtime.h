@@ -501,31 +501,38 @@ void read_back(azk_ctx* ctx, cudaStream_t s, const HostResult* results, size_t c
   // first one's way and the last one's copying would otherwise be most of the time.
   const uint64_t most = total >= 4 * kLandingPiece ? kLandingPiece : kLandingPiece / 4;
   cudaEvent_t* const half = lease->halves();
-  struct Piece {
-    uint8_t* dst = nullptr;
-    uint64_t bytes = 0;
-  } piece[2];
+  struct Part {
+    uint8_t* dst;
+    uint64_t at, bytes;
+  };
+  std::vector<Part> part[2];  // what a half holds: the end of one result, small ones whole, the start of another
+  uint64_t used[2] = {0, 0};
   bool checked = false;
-  uint32_t k = 0;
   auto finish = [&](uint32_t h) {
-    if (!piece[h].dst) return;
+    if (!used[h]) return;
     wait_event(half[h]);
     if (!checked) check();
     checked = true;
-    copy_past_caches(piece[h].dst, landing + h * kLandingPiece, piece[h].bytes);
-    piece[h].dst = nullptr;
+    for (const Part& q : part[h]) copy_past_caches(q.dst, landing + h * kLandingPiece + q.at, q.bytes);
+    part[h].clear();
+    used[h] = 0;
   };
+  uint32_t h = 0;
   for (size_t i = 0; i < n; i++) {
-    for (uint64_t at = 0; at < r[i].bytes; at += most, k++) {
-      const uint32_t h = k & 1;
-      finish(h);
-      piece[h] = {static_cast<uint8_t*>(r[i].dst) + at, std::min(r[i].bytes - at, most)};
-      AZK_CU(cudaMemcpyAsync(landing + h * kLandingPiece, static_cast<const uint8_t*>(r[i].src) + at, piece[h].bytes, cudaMemcpyDeviceToHost, s));
+    for (uint64_t at = 0; at < r[i].bytes;) {
+      const uint64_t bytes = std::min(r[i].bytes - at, most - used[h]);
+      AZK_CU(cudaMemcpyAsync(landing + h * kLandingPiece + used[h], static_cast<const uint8_t*>(r[i].src) + at, bytes, cudaMemcpyDeviceToHost, s));
+      part[h].push_back({static_cast<uint8_t*>(r[i].dst) + at, used[h], bytes});
+      used[h] += align_up(bytes, 16);
+      at += bytes;
+      if (used[h] < most && !(i + 1 == n && at == r[i].bytes)) continue;
       AZK_CU(cudaEventRecord(half[h], s));
+      h ^= 1;
+      finish(h);
     }
   }
-  finish(k & 1);
-  finish((k + 1) & 1);
+  finish(h);
+  finish(h ^ 1);
   settle.idle = true;  // every piece was waited for
 }
 inline void read_back(azk_ctx* ctx, cudaStream_t s, std::initializer_list<HostResult> r) { read_back(ctx, s, r.begin(), r.size(), [] {}); }
